@@ -397,9 +397,9 @@ __global__ void __launch_bounds__(128, 4) k_adj_visc(Problem p, int64_t nplain, 
     if (fg) {
 #pragma unroll
       for (int j = 0; j < 12; ++j) gm[j] = fg[(i * QS + q) * 12 + j];
-    } else {  // each cell's gradient is the same at all its face points: slot 0
-      const double* g0 = p.ulv + c * (int64_t)MF * QS * 12;
-      const double* g1 = bnd ? g0 : p.ulv + nb * (int64_t)MF * QS * 12;
+    } else {  // a MUSCL cell's gradient is the same at all its faces
+      const double* g0 = p.ulv + c * (int64_t)QS * 12;
+      const double* g1 = bnd ? g0 : p.ulv + nb * (int64_t)QS * 12;
 #pragma unroll
       for (int j = 0; j < 12; ++j) gm[j] = (g0[j] + g1[j]) / 2.0;
     }
@@ -642,8 +642,7 @@ __device__ void muscl_forward(const Problem& p, const double* __restrict__ U, in
 // Navier-Stokes: the cell's gradient of (T, u, v, w) ([T, u, v, w][x, y,
 // z]) from the viscous least squares on stencil 1 and the frame (AINVJT),
 // in the operations and order of k_muscl's viscous part (gradients.f90:
-// 502-706, SOLUTIONTRIAV2), which writes the same 12 values to every face
-// slot of ulv.
+// 502-706, SOLUTIONTRIAV2): the cell's record of ulv.
 __device__ __forceinline__ void visc_cell_gradient(const Problem& p, const double* __restrict__ U, int64_t c,
                                                    double* gr) {
   const int IM = p.imax, W = IM + 1;
@@ -683,7 +682,7 @@ __device__ __forceinline__ void visc_cell_gradient(const Problem& p, const doubl
 // The reconstruction of every cell with its intermediates kept for the
 // reverse sweep: face values (minus the mean) to dul exactly as k_muscl
 // writes them, the MusclFwd record to fwd[c]; for Navier-Stokes the cell's
-// viscous gradient to face slot 0 of ulv (the slot that k_adj_visc reads).
+// viscous gradient to ulv (read by k_adj_visc).
 // A face neighbour that is also a cell of the stencil shares the stencil
 // cell's slot: the bound slots amin/amax are remapped to it, and fmask keeps
 // the faces whose neighbour has a slot of its own (the reverse map in
@@ -725,7 +724,7 @@ __global__ void __launch_bounds__(128) k_adj_fwd(Problem p, const double* __rest
     double gr[12];
     visc_cell_gradient(p, U, c, gr);
     const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-    double* o = p.ulv + c * (int64_t)MF * QS * 12;
+    double* o = p.ulv + c * (int64_t)QS * 12;
 #pragma unroll
     for (int j = 0; j < 12; ++j) o[j] = gr[j];
   }
@@ -899,7 +898,7 @@ struct Dp5 {
 // (T, u, v, w), [n][12] in the layout of ulv.  With `base` the value parts,
 // which are the reconstruction itself, go out as k_muscl writes it (in place
 // of a k_muscl launch): the face values to dul and, with tgr, the cell's
-// viscous gradient to face slot 0 of ulv (the slot that k_jvp_face reads).
+// viscous gradient to ulv (read by k_jvp_face).
 __global__ void __launch_bounds__(128) k_jvp_muscl(Problem p, const double* __restrict__ U,
                                                    const double* __restrict__ dU, double* __restrict__ tdul,
                                                    double* __restrict__ tgr, bool base) {
@@ -968,7 +967,7 @@ __global__ void __launch_bounds__(128) k_jvp_muscl(Problem p, const double* __re
       for (int kk = 0; kk < 3; ++kk) {
         const D t = Jc[0 * 3 + kk] * gvv[0][a] + Jc[1 * 3 + kk] * gvv[1][a] + Jc[2 * 3 + kk] * gvv[2][a];
         tgr[c * 12 + a * 3 + kk] = t.d[0];
-        if (base) p.ulv[c * (int64_t)MF * QS * 12 + a * 3 + kk] = t.v;
+        if (base) p.ulv[c * (int64_t)QS * 12 + a * 3 + kk] = t.v;
       }
   }
   D mn[NV], mx[NV];
@@ -1075,8 +1074,8 @@ __global__ void __launch_bounds__(128) k_jvp_face(Problem p, const double* __res
 #pragma unroll
     for (int v = 0; v < NV; ++v) tf[v] = tf[v] + fl[v].d[0] * ws;
     if (tgr) {
-      const double* g0 = p.ulv + c * (int64_t)MF * QS * 12;  // slot 0: see k_jvp_muscl
-      const double* g1 = nb >= 0 ? p.ulv + nb * (int64_t)MF * QS * 12 : g0;
+      const double* g0 = p.ulv + c * (int64_t)QS * 12;  // as k_jvp_muscl wrote it
+      const double* g1 = nb >= 0 ? p.ulv + nb * (int64_t)QS * 12 : g0;
       const double* t0 = tgr + c * 12;
       const double* t1 = nb >= 0 ? tgr + nb * 12 : t0;
       D gl[12], gr[12], fv[NV];
@@ -1379,7 +1378,7 @@ __global__ void k_wall_loads(Problem p, const double* __restrict__ U, const doub
       const double w = face_weight(p, ft, q);
       ssp = ssp + (pr[4] * w);
       if (p.governing == 1) {
-        const double* g = p.fgrad ? p.fgrad + (i * QS + q) * 12 : p.ulv + s * 12;  // rows T, u, v, w
+        const double* g = p.fgrad ? p.fgrad + (i * QS + q) * 12 : p.ulv + (c * QS + q) * 12;  // rows T, u, v, w
         const double ux = g[3], uy = g[4], uz = g[5], vx = g[6], vy = g[7], vz = g[8];
         const double wx = g[9], wy = g[10], wz = g[11];
         double mu, lam;

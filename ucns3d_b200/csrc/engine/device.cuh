@@ -78,7 +78,7 @@ struct Problem {
   int8_t* mmus;             // first cascade: msel and reduced, MUSCL recomputed
   int8_t* mord;             // MOOD_O per cell
   void* dul;                // [n][MF][MQ][NV]  face value minus cell mean (T)
-  double* ulv;              // [n][MF][MQ][4][3] face gradients of T,u,v,w (MUSCL IORDER 1)
+  double* ulv;              // [n][QS][4][3] gradients of T,u,v,w, one record a cell (MUSCL IORDER 1: point 0)
   double* fgrad;            // [nown][QS][4][3] face-point average of both sides' gradients of T,u,v,w (WENO)
   void* gv;                 // [n][ideg][4]  viscous LSQ coefficients, in the table precision
   double* prim;             // [n][4] T, u, v, w of each cell (viscous LSQ, formed once per stage)

@@ -166,14 +166,16 @@ template <typename T>
 int launch_recon_t(ucg_engine* e, const Problem& p, const double* U) {
   const ucg_config& c = e->cfg;
   if (c.scheme == 2 && c.iorder == 1) {
-    unsigned blocks = (unsigned)((p.n + 127) / 128);
+    const unsigned blocks = (unsigned)((p.n + 31) / 32);
     const bool vk = c.limiter == 7;
     if (c.governing == 1) {
-      if (vk) k_muscl<T, true, true><<<blocks, 128, 0, e->stream>>>(p, U);
-      else k_muscl<T, true, false><<<blocks, 128, 0, e->stream>>>(p, U);
+      constexpr int TH = 32 * muscl_warps<true>();
+      if (vk) k_muscl<T, true, true><<<blocks, TH, 0, e->stream>>>(p, U);
+      else k_muscl<T, true, false><<<blocks, TH, 0, e->stream>>>(p, U);
     } else {
-      if (vk) k_muscl<T, false, true><<<blocks, 128, 0, e->stream>>>(p, U);
-      else k_muscl<T, false, false><<<blocks, 128, 0, e->stream>>>(p, U);
+      constexpr int TH = 32 * muscl_warps<false>();
+      if (vk) k_muscl<T, false, true><<<blocks, TH, 0, e->stream>>>(p, U);
+      else k_muscl<T, false, false><<<blocks, TH, 0, e->stream>>>(p, U);
     }
     e->launches++;
     CK(cudaGetLastError());
@@ -582,7 +584,7 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
     rc = rc ? rc : alloc(e, e->qbuf, (size_t)ngrp * 32 * c.admis_max * 15 * 8);
   if (c.governing == 1) {
     if (c.scheme == 2 && c.iorder == 1) {
-      rc = rc ? rc : alloc(e, e->ulv, (size_t)n * MF * e->QS * 12 * 8);
+      rc = rc ? rc : alloc(e, e->ulv, (size_t)n * e->QS * 12 * 8);
     } else {
       rc = rc ? rc : alloc(e, e->gv, (size_t)n * c.ideg * 4 * T);
       rc = rc ? rc : alloc(e, e->prim, (size_t)n * 4 * 8);

@@ -11,124 +11,154 @@
 namespace ucg {
 
 // ======================================================================
-// MUSCL, IORDER = 1 (one quadrature point per face), one thread per cell.
-// LEAST_SQUARES (gradients.f90:253-497), MUSCL + Venkatakrishnan
-// (reconstruct_p.f90:2286, 1821, 2044, 3421), CHECKSOLX (3245), and for
-// Navier-Stokes the viscous LSQ (gradients.f90:502-706) + SOLUTIONTRIAV2.
+// MUSCL, IORDER = 1 (one quadrature point per face).  LEAST_SQUARES
+// (gradients.f90:253-497), MUSCL + Venkatakrishnan (reconstruct_p.f90:2286,
+// 1821, 2044, 3421), CHECKSOLX (3245), and for Navier-Stokes the viscous LSQ
+// (gradients.f90:502-706) + SOLUTIONTRIAV2.
 // VK: the limiter is Venkatakrishnan (LIMITER 7) inline; otherwise the
 // SLOPE_LIMITERS code of the configuration, chosen at run time.
+//
+// One block per 32-cell group, one warp per reconstructed variable (lane =
+// cell): the five conserved ones and, for Navier-Stokes, T, u, v, w.  The
+// kernel is bound by the latency of dependent gathers and FP64 divisions (two
+// per limiter value, 30 values a cell), so the work of a cell is spread over
+// five or nine warps instead of one thread: the table rows stay coalesced,
+// and the primitive records of the eight members and the cell are formed once
+// per block, one member per warp, in shared memory.  The limited values go
+// through shared memory for CHECKSOLX (warp = face) and one contiguous store.
+// Same operations in the same order per value as one thread per cell, which
+// took (FP64 Navier-Stokes) 23.4 us at 512 cells and 35.5 us at 32,768, and
+// (mixed, Euler) 51.7 us at 115,260; this form 6.8, 19.2 and
+// 41.2 us.  56 registers (four blocks of nine warps, seven of five per SM): with
+// the compiler's choice the same kernel took 40.5 us at 32,768 cells.
 // ======================================================================
+template <bool NS>
+__host__ __device__ constexpr int muscl_warps() {
+  return NS ? NV + 4 : NV;
+}
 template <typename T, bool NS, bool VK>
-__global__ void __launch_bounds__(128) k_muscl(Problem p, const double* __restrict__ U) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.n) return;
+__global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Problem p, const double* __restrict__ U) {
+  constexpr int NW = muscl_warps<NS>();
+  constexpr int MC = 8;  // members per pass of the primitive records
+  __shared__ double s_d[MF * NV][33];
+  __shared__ double s_p[NS ? MC + 1 : 1][4][32];  // T, u, v, w of the cell and of a pass's members
+  __shared__ int s_first[32], s_nf[32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t grp = blockIdx.x, g0 = grp * 32;
+  const int ncl = p.n - g0 < 32 ? (int)(p.n - g0) : 32;  // cells of this group
+  const int ln = lane < ncl ? lane : ncl - 1;            // spare lanes repeat the last cell
+  const int64_t c = g0 + ln;
   const int IM = p.imax, W = IM + 1, QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + ln;  // row j at st[j * 32]
+  const T* M = (const T*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + ln;
   const int nf = p.nfaces[c];
-  double u0[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) u0[v] = U[c * NV + v];
-  double pm[NV];
-  cons2prim(p.gamma, u0, pm);
-  const double t0 = NS ? pm[4] / (pm[0] * p.r_gas) : 0.0;
-  // least squares on stencil 1
-  const int64_t grp = c >> 5;
-  const int lane = (int)(c & 31);
-  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + lane;  // row j at st[j * 32]
-  const T* M = (const T*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + lane;
-  T g[3][NV];
-  double gvv[3][4];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) g[d][v] = T(0);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) gvv[d][v] = 0.0;
+  if (w == 0) {
+    s_first[lane] = 0;
+    s_nf[lane] = nf;
   }
-  for (int k = 0; k < IM; ++k) {
-    const int64_t y = st[(k + 1) * 32];
-    double uy[NV];
+  if (NS) {
+    double gv[3] = {0.0, 0.0, 0.0};
+    for (int k0 = 0; k0 < IM; k0 += MC) {
+      if (k0) __syncthreads();  // the last pass's records have been read
+      const int j = k0 + w - 1;
+      if (w == 0 ? k0 == 0 : w <= MC && j < IM) {  // warp 0: the cell itself
+        const double* uy = U + (w == 0 ? c : (int64_t)st[(j + 1) * 32]) * NV;
+        double u[NV], py[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) uy[v] = U[y * NV + v];
-    T m0 = M[(k * 3 + 0) * 32], m1 = M[(k * 3 + 1) * 32], m2 = M[(k * 3 + 2) * 32];
+        for (int v = 0; v < NV; ++v) u[v] = uy[v];
+        cons2prim(p.gamma, u, py);
+        s_p[w][0][lane] = py[4] / (py[0] * p.r_gas);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      T du = T(uy[v] - u0[v]);
-      g[0][v] += m0 * du;
-      g[1][v] += m1 * du;
-      g[2][v] += m2 * du;
-    }
-    if (NS) {
-      double py[NV];
-      cons2prim(p.gamma, uy, py);
-      double ds[4] = {py[4] / (py[0] * p.r_gas) - t0, py[1] - pm[1], py[2] - pm[2], py[3] - pm[3]};
+        for (int v = 1; v < 4; ++v) s_p[w][v][lane] = py[v];
+      }
+      __syncthreads();
+      if (w >= NV) {
+        const double t0 = s_p[0][w - NV][lane];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        gvv[0][v] += (double)m0 * ds[v];
-        gvv[1][v] += (double)m1 * ds[v];
-        gvv[2][v] += (double)m2 * ds[v];
+        for (int i = 0; i < MC; ++i)
+          if (k0 + i < IM) {
+            const double ds = s_p[i + 1][w - NV][lane] - t0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) gv[d] += (double)M[((k0 + i) * 3 + d) * 32] * ds;
+          }
       }
     }
-  }
-  // bounds from the cell and its face neighbours (FIND_BOUNDS, strict)
-  double umin[NV], umax[NV];
+    if (w >= NV && lane < ncl) {
+      // the cell's gradient (d/dxi of the linear basis is the unit vector,
+      // then AINVJT = INVCCJAC^T, SOLUTIONTRIAV2), the same at every face
+      const double* J = p.jinv + c * 9;
+      double* o = p.ulv + c * (int64_t)QS * 12 + (w - NV) * 3;
 #pragma unroll
-  for (int v = 0; v < NV; ++v) umin[v] = umax[v] = u0[v];
-  for (int f = 0; f < nf; ++f) {
-    const int64_t nb = p.neigh[c * MF + f];
-    if (nb < 0) continue;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      double un = U[nb * NV + v];
-      umin[v] = fmin(umin[v], un);
-      umax[v] = fmax(umax[v], un);
+      for (int k = 0; k < 3; ++k) o[k] = J[0 * 3 + k] * gv[0] + J[1 * 3 + k] * gv[1] + J[2 * 3 + k] * gv[2];
     }
   }
-  // interleaved over 32-cell groups: element j at [j * 32]
-  const T* qp = (const T*)p.qpts + (c >> 5) * (int64_t)MF * QS * 3 * 32 + (c & 31);
-  const T* bm = (const T*)p.bmean + (c >> 5) * 3 * 32 + (c & 31);
-  const double epsi2 = (p.kappa_ven * p.minedge[c]) * (p.kappa_ven * p.minedge[c]) * (p.kappa_ven * p.minedge[c]);
-  // unlimited face value minus the mean (recomputed rather than stored: three terms)
-  auto face_d = [&](int f, int v) -> double {
-    T b0 = qp[(f * QS * 3 + 0) * 32] - bm[0], b1 = qp[(f * QS * 3 + 1) * 32] - bm[32],
-      b2 = qp[(f * QS * 3 + 2) * 32] - bm[64];
-    T res = b0 * g[0][v] + b1 * g[1][v] + b2 * g[2][v];
-    return (u0[v] + (double)res) - u0[v];
-  };
-  double slope[NV];
+  if (w < NV) {
+    const double u0 = U[c * NV + w];
+    // least squares on stencil 1
+    T g[3] = {T(0), T(0), T(0)};
+#pragma unroll 8
+    for (int k = 0; k < IM; ++k) {
+      const T du = T(U[(int64_t)st[(k + 1) * 32] * NV + w] - u0);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) slope[v] = TOLBIG;
-  for (int f = 0; f < nf; ++f)
+      for (int d = 0; d < 3; ++d) g[d] += M[(k * 3 + d) * 32] * du;
+    }
+    // bounds from the cell and its face neighbours (FIND_BOUNDS, strict)
+    double lo = u0, hi = u0;
+    {
+      const int2* nb2 = (const int2*)(p.neigh + c * MF);  // -1 past the cell's last face
 #pragma unroll
-    for (int v = 0; v < NV; ++v)
-      slope[v] = fmin(slope[v], VK ? venkat(face_d(f, v), umin[v] - u0[v], umax[v] - u0[v], epsi2)
-                                   : slope_limiter(p.limiter, face_d(f, v), umin[v] - u0[v], umax[v] - u0[v], epsi2));
-  // limited face values and CHECKSOLX
-  bool first = false;
-  for (int f = 0; f < nf; ++f) {
-    double uf[NV];
+      for (int f = 0; f < MF; f += 2) {
+        const int2 nb = nb2[f / 2];
+        const double a = nb.x >= 0 ? U[(int64_t)nb.x * NV + w] : u0, b = nb.y >= 0 ? U[(int64_t)nb.y * NV + w] : u0;
+        lo = a < lo ? a : lo;
+        hi = a > hi ? a : hi;
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+      }
+    }
+    lo -= u0;
+    hi -= u0;
+    // unlimited face values minus the mean, limited by the least slope
+    const T* qp = (const T*)p.qpts + grp * (int64_t)MF * QS * 3 * 32 + ln;
+    const T* bm = (const T*)p.bmean + grp * 3 * 32 + ln;
+    const T b0 = bm[0], b1 = bm[32], b2 = bm[64];
+    const double ke = p.kappa_ven * p.minedge[c];
+    const double epsi2 = ke * ke * ke;
+    double dd[MF], slope = TOLBIG;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) uf[v] = u0[v] + face_d(f, v) * slope[v];
-    first = first || jump_bad(p.gamma, pm, uf, 0.95);
+    for (int f = 0; f < MF; ++f) {
+      dd[f] = 0.0;
+      if (f < nf) {
+        const T* x = qp + f * QS * 3 * 32;
+        const T res = (x[0] - b0) * g[0] + (x[32] - b1) * g[1] + (x[64] - b2) * g[2];
+        dd[f] = (u0 + (double)res) - u0;
+        const double phi = VK ? venkat(dd[f], lo, hi, epsi2) : slope_limiter(p.limiter, dd[f], lo, hi, epsi2);
+        slope = phi < slope ? phi : slope;
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < MF; ++f) s_d[f * NV + w][lane] = dd[f] * slope;
   }
-  T* out = (T*)p.dul + c * (int64_t)MF * QS * NV;
-  for (int f = 0; f < nf; ++f)
+  __syncthreads();
+  {  // CHECKSOLX on the limited face values
+    double u0[NV], pm[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) out[f * QS * NV + v] = first ? T(0) : T(face_d(f, v) * slope[v]);
-  if (NS) {
-    // face gradients: d/dxi of the linear basis is the unit vector, then
-    // AINVJT = INVCCJAC^T (SOLUTIONTRIAV2)
-    const double* J = p.jinv + c * 9;
-    double gr[4][3];
+    for (int v = 0; v < NV; ++v) u0[v] = U[c * NV + v];
+    cons2prim(p.gamma, u0, pm);
+    for (int f = w; f < nf; f += NW) {
+      double uf[NV];
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) gr[v][k] = J[0 * 3 + k] * gvv[0][v] + J[1 * 3 + k] * gvv[1][v] + J[2 * 3 + k] * gvv[2][v];
-    double* o = p.ulv + c * (int64_t)MF * QS * 12;
-    for (int f = 0; f < nf; ++f)
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) o[f * QS * 12 + v * 3 + k] = gr[v][k];
+      for (int v = 0; v < NV; ++v) uf[v] = u0[v] + s_d[f * NV + v][lane];
+      if (jump_bad(p.gamma, pm, uf, 0.95)) s_first[lane] = 1;
+    }
+  }
+  __syncthreads();
+  // one run of MF * NV values a cell (QS 1), a cell per warp and turn
+  const int r = lane, f = r / NV;
+  if (r < MF * NV) {
+    T* out = (T*)p.dul + (g0 * MF + f) * QS * NV + (r - f * NV);
+    for (int cl = w; cl < ncl; cl += NW)
+      if (f < s_nf[cl]) out[(int64_t)cl * MF * QS * NV] = s_first[cl] ? T(0) : T(s_d[r][cl]);
   }
 }
 
@@ -219,10 +249,9 @@ __global__ void __launch_bounds__(UCG_FACE_BLOCK, NS ? 6 : 1) k_face(Problem p, 
       // dg_functions.f90:1179-1300) and faces with codes 1-4 drop the jump
       // term (flux_p.f90:1872-1874).
       const double2* gl2 = (const double2*)(p.fgrad ? p.fgrad + (i * QS + q) * 12
-                                                    : p.ulv + ((c * MF + f) * QS + q) * 12);
+                                                    : p.ulv + (c * QS + q) * 12);
       const double2* gr2 = (const double2*)(p.fgrad ? p.fgrad + (i * QS + q) * 12
-                                                    : nb >= 0 ? p.ulv + ((nb * MF + nf) * QS + qq) * 12
-                                                              : p.ulv + ((c * MF + f) * QS + q) * 12);
+                                                    : p.ulv + (nb >= 0 ? nb * QS + qq : c * QS + q) * 12);
       const int code = nb >= 0 ? 0 : p.bc[c * MF + f];
       double gl[12], gr[12];
 #pragma unroll
@@ -467,8 +496,8 @@ __global__ void k_reduce_partial(Problem p, const double* __restrict__ U, int wh
     double x;
     if (what == UCG_REDUCE_ENSTROPHY) {
       // cell-centre velocity gradients g[i][j] = du_i/dx_j: the viscous
-      // least-squares face gradients of a linear polynomial (face 0, point 0)
-      const double* g = p.ulv + c * (int64_t)MF * 12 + 3;
+      // least-squares gradient of a linear polynomial
+      const double* g = p.ulv + c * (int64_t)(p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri) * 12 + 3;
       double on = 0.0;
 #pragma unroll
       for (int i = 0; i < 3; ++i)
