@@ -1,4 +1,5 @@
-"""The MUSCL step: stencils of more members than k_muscl takes per pass."""
+"""The MUSCL step: stencils of more members than k_muscl takes per pass, and
+the time steps that the last stage's update forms."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,25 @@ def test_muscl_more_members_than_a_pass(gov, precision):
         R = e.residual()
         ref = R if ref is None else ref
         assert np.array_equal(R, ref), extra
+
+
+@pytest.mark.parametrize("gov", [EULER, NAVIER_STOKES])
+def test_time_steps_formed_by_the_last_stage(gov):
+    """ucg_step forms each following step's CFL time step in the last stage's
+    update: the same steps as CALCULATE_CFL and RK3 called one by one, also
+    when calls follow one another and other calls use the time step between."""
+    m = Mesh.box_tet(4, 4, 3, seed=2).prepare(SCHEME_MUSCL, 1)
+    cfg = make_config(m, governing=gov, reynolds=200.0, pres=5.0, prandtl=0.71)
+    U = m.initial_condition(IC_TGV, [1.4, 5.0, 1.0])
+    a, b = Engine(m, cfg), Engine(m, cfg)
+    a.set_state(U)
+    b.set_state(U)
+    for nsteps, cfl in ((1, 0.5), (2, 0.4), (5, 0.3), (0, 0.3), (3, 0.5)):
+        a.time_marching(nsteps, cfl)
+        for _ in range(nsteps):
+            dt = b.calculate_cfl(cfl)
+            b.runge_kutta3(dt)
+        assert a.last_dt() == dt
+        assert np.array_equal(a.get_state(), b.get_state())
+        assert a.calculate_cfl(0.2) == b.calculate_cfl(0.2) == a.last_dt()
+        dt = a.last_dt()

@@ -1900,7 +1900,7 @@ int ucg_adjoint_run_obj(ucg_engine* e, int32_t objective, int32_t nsteps, double
   // forward with checkpoints
   for (int s = 0; s < nsteps; ++s) {
     if (s % every == 0) CK(cudaMemcpyAsync(ckpt + (size_t)(s / every) * m, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
-    if ((rc = rk3(e, dt, false))) return rc;
+    if ((rc = rk3(e, dt))) return rc;
   }
   CK(cudaMemcpyAsync(fin, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
   double* sc = bar_scal(e);  // sc[0] J, sc[8..12] pbar accumulator, sc[16..20] partial
@@ -1923,7 +1923,7 @@ int ucg_adjoint_run_obj(ucg_engine* e, int32_t objective, int32_t nsteps, double
     for (int s = s0; s < s1; ++s) {
       double* t = traj + (size_t)3 * (s - s0) * m;
       CK(cudaMemcpyAsync(t, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
-      if ((rc = rk3(e, dt, false))) return rc;
+      if ((rc = rk3(e, dt))) return rc;
       CK(cudaMemcpyAsync(t + m, e->Ua.p, mb, cudaMemcpyDeviceToDevice, e->stream));
       CK(cudaMemcpyAsync(t + 2 * m, e->Ub.p, mb, cudaMemcpyDeviceToDevice, e->stream));
     }

@@ -96,6 +96,8 @@ struct Problem {
   int limiter;   // SLOPE_LIMITERS code (7 Venkatakrishnan)
   int boundtype; // BOUNDTYPE: 0 supersonic inflow/outflow, 1 characteristic treatment
   double* dt_dev;           // device dt (ucg_step)
+  double* dt_next;          // the next step's dt, formed by the last stage's update (nullptr: not formed)
+  double ccfl;              // CFL / 3 of dt_next
 };
 
 // ------------------------------------------------------------- basis

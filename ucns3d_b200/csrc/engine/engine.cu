@@ -150,6 +150,8 @@ Problem make_problem(ucg_engine* e) {
   p.vflux = (double*)e->vflux.p;
   p.health = (unsigned*)e->health.p;
   p.dt_dev = nullptr;
+  p.dt_next = nullptr;
+  p.ccfl = 0.0;
   p.lsq_bulk = e->lsq_bulk ? 1 : 0;
   p.lsq_wait = e->lsq_wait;
   p.wenwrt = c.wenwrt;
@@ -227,12 +229,13 @@ void launch_update_t(ucg_engine* e, const Problem& p0, int mode, const double* U
                      double dt) {
   Problem p = p0;
   p.n = e->n_update;
-  unsigned blocks = (unsigned)((p.n + 255) / 256);
+  const unsigned blocks = (unsigned)((p.n + UPD_CELLS - 1) / UPD_CELLS);
+  constexpr int TH = UPD_CELLS * NV;
   switch (mode) {
-    case 0: k_update<NS, 0, CHK><<<blocks, 256, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    case 1: k_update<NS, 1, CHK><<<blocks, 256, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    case 2: k_update<NS, 2, CHK><<<blocks, 256, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    default: k_update<NS, 3, CHK><<<blocks, 256, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
+    case 0: k_update<NS, 0, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
+    case 1: k_update<NS, 1, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
+    case 2: k_update<NS, 2, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
+    default: k_update<NS, 3, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
   }
   e->launches += 1;
 }
@@ -300,10 +303,13 @@ int mood_stage(ucg_engine* e, const Problem& p, int mode, const double* Uc, cons
   return UCG_OK;
 }
 
-// one RUNGE_KUTTA3 step; dt from the host value or, if dt_dev, from device memory
-int rk3(ucg_engine* e, double dt, bool dt_dev) {
+// one RUNGE_KUTTA3 step; dt from the host value or, if dt_dev, from device
+// memory; dt_next: see k_update
+int rk3(ucg_engine* e, double dt, double* dt_dev, double* dt_next, double ccfl) {
   Problem p = make_problem(e);
-  if (dt_dev) p.dt_dev = (double*)e->dt.p;
+  p.dt_dev = dt_dev;
+  p.dt_next = dt_next;
+  p.ccfl = ccfl;
   double* Un = (double*)e->Un.p;
   double* Ua = (double*)e->Ua.p;
   double* Ub = (double*)e->Ub.p;
@@ -450,6 +456,7 @@ int cells_out(ucg_engine* e, double* host_dst, const double* dev_src) {
 
 int cfl_device(ucg_engine* e, double cfl) {
   Problem p = make_problem(e);
+  e->dt_slot = 0;
   k_dt_init<<<1, 1, 0, e->stream>>>((double*)e->dt.p);
   k_cfl<<<(unsigned)((e->n + 255) / 256), 256, 0, e->stream>>>(p, (const double*)e->Un.p, cfl / 3.0, (double*)e->dt.p);
   e->launches += 2;
@@ -1093,18 +1100,26 @@ int ucg_rk3_step(ucg_engine* e, double dt) {
   if (!e || !(dt > 0)) return fail(e, UCG_EINVAL, "bad argument");
   if (!ready(e) || !e->have_state) return fail(e, UCG_ESTATE, "geometry, tables and state are needed");
   cudaSetDevice(e->device);
-  return rk3(e, dt, false);
+  return rk3(e, dt);
 }
 
 int ucg_step(ucg_engine* e, double cfl, int32_t nsteps) {
   if (!e || !(cfl > 0) || nsteps < 0) return fail(e, UCG_EINVAL, "bad argument");
   if (!ready(e) || !e->have_state) return fail(e, UCG_ESTATE, "geometry, tables and state are needed");
   cudaSetDevice(e->device);
+  // The time step of the first step is CALCULATE_CFL's own kernel; each
+  // step's last update forms the next step's in the other of two slots.  Not
+  // with MOOD, whose last cascade writes the state, nor with partition roles,
+  // whose update covers only part of the cells that CALCULATE_CFL covers.
+  const bool fuse = !e->cfg.mood && e->n_update == e->n;
+  double* dt = (double*)e->dt.p;
   for (int s = 0; s < nsteps; ++s) {
-    int rc = cfl_device(e, cfl);
-    if (rc) return rc;
-    rc = rk3(e, 0.0, true);
-    if (rc) return rc;
+    int rc;
+    if (s == 0 || !fuse)
+      if ((rc = cfl_device(e, cfl))) return rc;
+    double* next = fuse && s + 1 < nsteps ? dt + (e->dt_slot ^ 1) : nullptr;
+    if ((rc = rk3(e, 0.0, dt + e->dt_slot, next, cfl / 3.0))) return rc;
+    if (next) e->dt_slot ^= 1;
   }
   return UCG_OK;
 }
@@ -1112,7 +1127,7 @@ int ucg_step(ucg_engine* e, double cfl, int32_t nsteps) {
 int ucg_last_dt(ucg_engine* e, double* dt) {
   if (!e || !dt) return fail(e, UCG_EINVAL, "null argument");
   cudaSetDevice(e->device);
-  CK(cudaMemcpyAsync(dt, e->dt.p, 8, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaMemcpyAsync(dt, (double*)e->dt.p + e->dt_slot, 8, cudaMemcpyDeviceToHost, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   return UCG_OK;
 }

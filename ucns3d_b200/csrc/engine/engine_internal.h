@@ -44,6 +44,7 @@ struct ucg_engine {
   int QS = 1;
   std::string err;
   int64_t launches = 0;
+  int dt_slot = 0;  // which of the two values in `dt` is the last step's time step
   int64_t bytes = 0;
   bool have_geometry = false, have_state = false;
   int64_t recon_cells = 0;
@@ -115,7 +116,7 @@ int launch_flux(ucg_engine* e, const ucg::Problem& p, int mode, const double* Uc
                 double dt, bool check = true);
 // the face fluxes alone (k_face; with p.msel only the faces of the selected cells)
 int launch_faces(ucg_engine* e, const ucg::Problem& p, const double* Uc);
-int rk3(ucg_engine* e, double dt, bool dt_dev);
+int rk3(ucg_engine* e, double dt, double* dt_dev = nullptr, double* dt_next = nullptr, double ccfl = 0.0);
 // [n][5] FP64 arrays between the caller's cell order on the host and the
 // device order (a plain copy when the engine keeps the caller's order);
 // both leave the copy queued on the handle's stream
