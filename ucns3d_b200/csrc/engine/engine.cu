@@ -589,6 +589,7 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
   }
   if (c.wenwrt == 2)  // characteristic WENO: G^T S G of every stencil (15 values)
     rc = rc ? rc : alloc(e, e->qbuf, (size_t)ngrp * 32 * c.admis_max * 15 * 8);
+  if (c.wenwrt == 2) rc = rc ? rc : alloc(e, e->wflag, (size_t)n);
   if (c.governing == 1) {
     if (c.scheme == 2 && c.iorder == 1) {
       rc = rc ? rc : alloc(e, e->ulv, (size_t)n * e->QS * 12 * 8);

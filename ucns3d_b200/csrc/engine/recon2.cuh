@@ -287,18 +287,11 @@ __global__ void __launch_bounds__(128) k_lsq_tma(Problem p, const double* __rest
 #ifndef UCG_WV_FALL_D
 #define UCG_WV_FALL_D 1
 #endif
-#ifndef UCG_WV_CHAR_F
-#define UCG_WV_CHAR_F 5
-#endif
-#ifndef UCG_WV_CHAR_D
-#define UCG_WV_CHAR_D 3
-#endif
 template <typename T>
 struct WVars {
   static constexpr int is = sizeof(T) == 4 ? UCG_WV_IS_F : UCG_WV_IS_D;
   static constexpr int face = sizeof(T) == 4 ? UCG_WV_FACE_F : UCG_WV_FACE_D;
   static constexpr int fall = sizeof(T) == 4 ? UCG_WV_FALL_F : UCG_WV_FALL_D;
-  static constexpr int chr = sizeof(T) == 4 ? UCG_WV_CHAR_F : UCG_WV_CHAR_D;
 };
 
 // is[k] += sum_d g[d][k] * sum_{e>=d} P_de g[e][k] over d, e < nd <= NMAX.
@@ -330,40 +323,6 @@ __device__ __forceinline__ void quad_form(const T* __restrict__ P, const T (&g)[
       for (int k = 0; k < VG; ++k) is[k] += g[d][k] * t[k];
       // keep the loads of one row together: without this fence the
       // compiler hoists the whole triangle and spills it
-      asm volatile("" ::: "memory");
-    }
-  }
-}
-
-// A[u][w] += sum_d g[d][u] * sum_{e>=d} P_de g[e][w] over d, e < nd (P the
-// packed triangle as in quad_form); sym(A) = g^T S g for every pair of
-// columns, A[u][u] the quadratic form of column u.
-template <int NMAX, int VG, typename T>
-__device__ __forceinline__ void sym_form(const T* __restrict__ P, const T (&g)[NMAX][VG], int nd, T (&A)[VG][VG]) {
-  constexpr int VEC = Vec<T>::N;
-  int rs = 0;
-#pragma unroll
-  for (int d = 0; d < NMAX; ++d) {
-    if (d < nd) {
-      T t[VG];
-#pragma unroll
-      for (int k = 0; k < VG; ++k) t[k] = T(0);
-#pragma unroll
-      for (int q = 0; q < (NMAX - d + VEC - 1) / VEC; ++q)
-        if (d + q * VEC < nd) {
-          T s[VEC];
-          ldv(P + (int64_t)(rs + q) * 32 * VEC, s);
-#pragma unroll
-          for (int i = 0; i < VEC; ++i)
-            if (d + q * VEC + i < NMAX)
-#pragma unroll
-              for (int k = 0; k < VG; ++k) t[k] += s[i] * g[d + q * VEC + i][k];
-        }
-      rs += (nd - d + VEC - 1) / VEC;
-#pragma unroll
-      for (int u = 0; u < VG; ++u)
-#pragma unroll
-        for (int w = 0; w < VG; ++w) A[u][w] += g[d][u] * t[w];
       asm volatile("" ::: "memory");
     }
   }
@@ -628,23 +587,15 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
 // in FP32 (2.1 M-cell CWENO4 Navier-Stokes: 52.7 -> 51.2 ms; in FP64 the
 // bound made the 647 k-cell step 31.8 -> 33.8 ms, so FP64 keeps two; four
 // blocks in FP32 made it 56.0 -> 57.6 ms on another box).
-template <int P, typename T, bool CH = false, bool ISB = false, bool FB = false, bool MU = false>
-__global__ void __launch_bounds__(CH ? 64 : 128, !CH && (P == 2 || (P == 3 && sizeof(T) == 4)) ? 3 : 1)
+template <int P, typename T, bool ISB = false, bool FB = false, bool MU = false>
+__global__ void __launch_bounds__(128, P == 2 || (P == 3 && sizeof(T) == 4) ? 3 : 1)
     k_wpost(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int VEC = Vec<T>::N;
   constexpr int L2 = ID < 9 ? ID : 9;  // CWENO lower order: IDEGFREE2 3 or 9 (grid_p.f90:6145-6160)
   constexpr int VI = WVars<T>::is, VH = WVars<T>::face, VF = WVars<T>::fall;
-  // variables per pass of the characteristic face polynomial (its 5x5 FP64
-  // combination matrices beside the polynomial).  Every pass reads all the
-  // stencil polynomials again for each face, so fewer variables per pass
-  // remove the spills (FP32: 978 bytes at 5, 16 at 2, none at 1) but cost
-  // more: 64^3 WENO5 reconstruction 17.2 ms at 5, 21.1 at 3, 25.3 at 2,
-  // 36.8 at 1 (FP32); FP64 52.6 ms at 3, 61.6 at 2, 78.5 at 1.
-  constexpr int VC = WVars<T>::chr;
-  constexpr int BT = CH ? 64 : 128;    // threads per block
+  constexpr int BT = 128;              // threads per block
   __shared__ double s_w[7 * NV * BT];  // per thread, [ll][v]: indicators, then weights
-  __shared__ double s_e[CH ? 50 * BT : 1];  // per thread: left then right eigenvectors (characteristic form)
   const int tid = threadIdx.x;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + tid;
   if (c >= p.n) return;
@@ -754,13 +705,13 @@ __global__ void __launch_bounds__(CH ? 64 : 128, !CH && (P == 2 || (P == 3 && si
   const bool md = p.mprev != nullptr;
   if (FB && !(MU ? p.mmus[c] : p.wflag[c])) return;
   bool fall = FB || !weno || (!md && !p.full[c]);  // CHECKSOL: FULL = 0 -> REDUCE
-  if (!CH && !fall && ISB) {
+  if (!fall && ISB) {
     // ---- smoothness indicators from k_wis
     const double* is = p.isb + grp * (int64_t)A * NV * 32 + lane;
     for (int ll = 0; ll < adm; ++ll)
 #pragma unroll
       for (int v = 0; v < NV; ++v) sw[(ll * NV + v) * BT] = is[(int64_t)(ll * NV + v) * 32];
-  } else if (!CH && !ISB && !fall) {
+  } else if (!ISB && !fall) {
     // ---- smoothness indicators g^T S g per stencil and variable
     const T* Pc = (const T*)p.ind + grp * p.istride * 32 + lane * VEC;
     for (int ll = 0; ll < adm; ++ll) {
@@ -785,7 +736,7 @@ __global__ void __launch_bounds__(CH ? 64 : 128, !CH && (P == 2 || (P == 3 && si
       }
     }
   }
-  if (!CH && !fall) {
+  if (!fall) {
     weights();
     // ---- combined polynomial, face values, CHECKSOL (threshold 0.85)
     bool flag = false;
@@ -853,215 +804,6 @@ __global__ void __launch_bounds__(CH ? 64 : 128, !CH && (P == 2 || (P == 3 && si
         }
       }
     }
-    fall = flag;
-  }
-  if (CH && !fall) {
-    // ---- CHARACTERISTIC_RECONSTRUCTION (src/reconstruct_p.f90:497-758), per
-    // face: eigenvectors at the average of the cell mean and the face
-    // neighbour's mean (or the boundary ghost of the cell mean), both in the
-    // face frame; stencil polynomials projected on the left eigenvectors
-    // (global-frame conserved variables, as the reference projects them);
-    // indicators and weights per characteristic variable; the face's
-    // polynomial back-projected.  The indicator of the projection W = G EL^T
-    // is EL_k^T (G^T S G) EL_k, so G^T S G is formed once per stencil and
-    // each face only applies its eigenvectors.  With M_ll = ER diag(w_ll) EL the combined
-    // conserved polynomial is sum_ll M_ll G_ll (rows d >= 1) and its mean
-    // sum_ll M_ll u0, formed in FP64.
-    const T* Pc = (const T*)p.ind + grp * p.istride * 32 + lane * VEC;
-    double* EL = s_e + tid;            // EL[(k * NV + v) * BT]
-    double* ER = s_e + 25 * BT + tid;  // ER[(v * NV + k) * BT]
-    // stencil polynomial row d of variable u (CWENO: the central one with the
-    // lower-order stencils removed, reconstruct_p.f90:1723-1737; g3 holds
-    // sum_l2 lk * G(l2) for the rows d < IDEGFREE2)
-    auto Gp = [&](int ll, int d, int u, const T (&g3)[L2][NV]) -> T {
-      if (!(cw && ll == 0)) return G(ll, d, u);
-      return T(1.0 / lc1) * (G(0, d, u) - (d < L2 ? g3[d][u] : T(0)));
-    };
-    auto lower_sum = [&](T (&g3)[L2][NV]) {
-#pragma unroll
-      for (int d = 0; d < L2; ++d)
-#pragma unroll
-        for (int u = 0; u < NV; ++u) g3[d][u] = T(0);
-      if (!cw) return;
-      for (int l2 = 1; l2 < adm; ++l2)
-#pragma unroll
-        for (int d = 0; d < L2; ++d)
-          if (d < ID2)
-#pragma unroll
-            for (int u = 0; u < NV; ++u) g3[d][u] = g3[d][u] + T(lk) * G(l2, d, u);
-    };
-    // Q_l = G_l^T S G_l (symmetric 5x5, upper triangle row by row) once per
-    // cell: the face-independent part of the characteristic indicators
-    double* Qc = p.qbuf + grp * (int64_t)(A * 15) * 32 + lane;
-#pragma unroll 1
-    for (int ll = 0; ll < adm; ++ll) {
-      const bool low = cw && ll > 0;
-      T g3[L2][NV];
-      lower_sum(g3);
-      auto store = [&](int u, int w, double x) {
-        Qc[(int64_t)(ll * 15 + (u * (2 * NV - u + 1)) / 2 + (w - u)) * 32] = x;
-      };
-      auto forms = [&](auto& g, const T* Pl, int nd) {
-        constexpr int ND = sizeof(g) / sizeof(g[0]);
-        constexpr int VG = sizeof(g[0]) / sizeof(T);
-        if constexpr (VG == NV) {  // all five variables at once
-#pragma unroll
-          for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int u = 0; u < NV; ++u) g[d][u] = d < nd ? Gp(ll, d, u, g3) : T(0);
-          T a[NV][NV];
-#pragma unroll
-          for (int u = 0; u < NV; ++u)
-#pragma unroll
-            for (int w = 0; w < NV; ++w) a[u][w] = T(0);
-          sym_form<ND, NV>(Pl, g, nd, a);
-#pragma unroll
-          for (int u = 0; u < NV; ++u)
-#pragma unroll
-            for (int w = u; w < NV; ++w) store(u, w, u == w ? (double)a[u][u] : 0.5 * ((double)a[u][w] + (double)a[w][u]));
-        } else {  // pairs of variables
-#pragma unroll 1
-          for (int u = 0; u < NV; ++u)
-#pragma unroll 1
-            for (int w = u; w < NV; ++w) {
-#pragma unroll
-              for (int d = 0; d < ND; ++d) {
-                g[d][0] = d < nd ? Gp(ll, d, u, g3) : T(0);
-                g[d][1] = d < nd ? Gp(ll, d, w, g3) : T(0);
-              }
-              T a[2][2] = {{T(0), T(0)}, {T(0), T(0)}};
-              sym_form<ND, 2>(Pl, g, nd, a);
-              store(u, w, u == w ? (double)a[0][0] : 0.5 * ((double)a[0][1] + (double)a[1][0]));
-            }
-        }
-      };
-      constexpr int QV = sizeof(T) == 4 ? NV : 2;
-      if (low) {
-        T g[L2][QV];
-        forms(g, Pc + (int64_t)(p.i2off / VEC) * 32 * VEC, ID2);
-      } else {
-        T g[ID][QV];
-        forms(g, Pc, ID);
-      }
-    }
-    bool flag = false;
-    for (int f = 0; f < nf; ++f) {
-      double r[4], ur[NV];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) r[k] = p.rot[(c * MF + f) * 4 + k];
-      const int64_t nb = p.neigh[c * MF + f];
-      if (nb >= 0) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) ur[v] = U[nb * NV + v];
-      } else {
-        boundary_ghost(p, p.bc[c * MF + f], r, u0, ur);
-      }
-      {
-        double rl[NV], rr[NV];
-        rot_f(r, u0, rl);
-        rot_f(r, ur, rr);
-        char_eigenvectors(p.gamma, rl, rr, EL, ER, BT);
-      }
-      // indicators of the projected polynomials: IS_l[k] = EL_k^T Q_l EL_k
-#pragma unroll 1
-      for (int ll = 0; ll < adm; ++ll) {
-        double q[15];
-#pragma unroll
-        for (int j = 0; j < 15; ++j) q[j] = Qc[(int64_t)(ll * 15 + j) * 32];
-#pragma unroll 1
-        for (int k = 0; k < NV; ++k) {
-          double l[NV];
-#pragma unroll
-          for (int u = 0; u < NV; ++u) l[u] = EL[(k * NV + u) * BT];
-          double is = 0.0;
-          int j = 0;
-#pragma unroll
-          for (int u = 0; u < NV; ++u)
-#pragma unroll
-            for (int w = u; w < NV; ++w, ++j) is += (u == w ? 1.0 : 2.0) * l[u] * l[w] * q[j];
-          sw[(ll * NV + k) * BT] = is;
-        }
-      }
-      weights();
-      // the face's polynomial in conserved variables, VC at a time
-      const int nq = face_nq(p, p.ftype[c * MF + f]);
-#pragma unroll 1
-      for (int v0 = 0; v0 < NV; v0 += VC) {
-        T gh[ID][VC];
-        double f0[VC];
-#pragma unroll
-        for (int k = 0; k < VC; ++k) {
-          f0[k] = 0.0;
-#pragma unroll
-          for (int d = 0; d < ID; ++d) gh[d][k] = T(0);
-        }
-#pragma unroll 1
-        for (int ll = 0; ll < adm; ++ll) {
-          const int nd = cw && ll > 0 ? ID2 : ID;
-          T g3[L2][NV];
-          if (ll == 0) lower_sum(g3);
-          double M[VC][NV];
-#pragma unroll
-          for (int k = 0; k < VC; ++k)
-#pragma unroll
-            for (int u = 0; u < NV; ++u) {
-              double a = 0.0;
-              if (v0 + k < NV)
-#pragma unroll
-                for (int j = 0; j < NV; ++j)
-                  a += ER[((v0 + k) * NV + j) * BT] * sw[(ll * NV + j) * BT] * EL[(j * NV + u) * BT];
-              M[k][u] = a;
-            }
-#pragma unroll
-          for (int k = 0; k < VC; ++k)
-#pragma unroll
-            for (int u = 0; u < NV; ++u) f0[k] += M[k][u] * u0[u];
-#pragma unroll
-          for (int d = 0; d < ID; ++d)
-            if (d < nd) {
-              T gu[NV];
-#pragma unroll
-              for (int u = 0; u < NV; ++u) gu[u] = Gp(ll, d, u, g3);
-#pragma unroll
-              for (int k = 0; k < VC; ++k)
-#pragma unroll
-                for (int u = 0; u < NV; ++u) gh[d][k] += T(M[k][u]) * gu[u];
-            }
-        }
-        T cb[VC];
-        mean_term(gh, cb);
-        for (int q = 0; q < QS; ++q) {
-          T* o = out + (f * QS + q) * NV;
-          if (q >= nq) {
-#pragma unroll
-            for (int k = 0; k < VC; ++k)
-              if (v0 + k < NV) o[v0 + k] = T(0);
-            continue;
-          }
-          T m[ID];
-          mono(f, q, m);
-#pragma unroll
-          for (int k = 0; k < VC; ++k) {
-            T rsum = T(0);
-#pragma unroll
-            for (int d = 0; d < ID; ++d) rsum += m[d] * gh[d][k];
-            if (v0 + k < NV) o[v0 + k] = T((f0[k] - u0[v0 + k]) + (double)(rsum - cb[k]));
-          }
-        }
-      }
-      // CHECKSOL on this face's stored values
-      for (int q = 0; q < nq; ++q) {
-        const T* o = out + (f * QS + q) * NV;
-        double uf[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) uf[v] = u0[v] + (double)o[v];
-        flag = flag || jump_bad(p.gamma, pm, uf, 0.85);
-      }
-    }
-    for (int f = nf; f < MF; ++f)
-      for (int q = 0; q < QS; ++q)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) out[(f * QS + q) * NV + v] = T(0);
     fall = flag;
   }
   // CHECKSOLX (threshold 0.95) cannot fire where the 0.85 test passed on the
@@ -1318,13 +1060,324 @@ __global__ void k_visc_facegrad(Problem p) {
     o[k] = make_double2((double)((gl[2 * k] + gr[2 * k]) / T(2)), (double)((gl[2 * k + 1] + gr[2 * k + 1]) / T(2)));
 }
 
-// Characteristic-variable post-processing (k_wpost<P, T, true>), 64 threads
-// per block for its shared eigenvectors.  Instantiated only in
-// recon_char_*.cu (explicit instantiations), which nvcc compiles in parallel
-// with the other reconstruction units.
+// CHARACTERISTIC_RECONSTRUCTION (src/reconstruct_p.f90:497-758): per face, the
+// eigenvectors at the average of the cell mean and the face neighbour's mean
+// (or the boundary ghost of the cell mean), both in the face frame; stencil
+// polynomials projected on the left eigenvectors (global-frame conserved
+// variables, as the reference projects them); indicators and weights per
+// characteristic variable; the face's polynomial back-projected.  The
+// indicator of the projection W = G EL^T is EL_k^T (G^T S G) EL_k, so G^T S G
+// is formed once per cell and stencil (k_char_forms) and each face only
+// applies its eigenvectors (k_char_face).  With M_ll = ER diag(w_ll) EL the
+// combined conserved polynomial is sum_ll M_ll G_ll (rows d >= 1) and its
+// mean sum_ll M_ll u0, formed in FP64.
+//
+// Both run one block per 32-cell group (and stencil, or faces) with one warp
+// per variable, lane = cell, as k_wis and k_wface do: the polynomials of one
+// variable fit in registers, and the five warps read the same triangles and
+// stencil polynomials at about the same time (from L1).  One lane per cell
+// with all five variables (four 64-thread blocks per SM, 1-1.4 KB of spills)
+// was latency-bound: 27,000 cells, WENO5 FP64: 5.92 ms -> 0.52 + 1.28 ms.
+//
+// Rows d < IDEGFREE2 of sum_l2 lk G_l2, what CWENO takes off its central
+// stencil (reconstruct_p.f90:1723-1737), of variable v into s[d][v][lane].
+template <int P, typename T>
+__device__ __forceinline__ void char_lower_sum(const Problem& p, const T* Gc, int adm, int v, int lane, T* s) {
+  constexpr int ID = Deg<P>::ideg;
+  const double lc1 = 1.0 - 1.0 / p.lwci;
+  const double lk = adm > 1 ? (1.0 - lc1) / (adm - 1) : 0.0;
+  for (int d = 0; d < p.ideg2; ++d) {
+    T g3 = T(0);
+    for (int l2 = 1; l2 < adm; ++l2) g3 = g3 + T(lk) * Gc[(int64_t)((l2 * ID + d) * NV + v) * 32];
+    s[(d * NV + v) * 32 + lane] = g3;
+  }
+}
+
+// G_l^T S G_l (symmetric 5x5, upper triangle row by row) of every stencil:
+// block (group, stencil), warp w forms the column products with variable w.
+template <int P, typename T>
+__global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
+  constexpr int ID = Deg<P>::ideg;
+  constexpr int VEC = Vec<T>::N;
+  constexpr int L2 = ID < 9 ? ID : 9;
+  __shared__ T s_a[NV * NV][32];
+  __shared__ T s_g[L2 * NV * 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ll = blockIdx.y;
+  const int64_t grp = blockIdx.x, c = grp * 32 + lane;
+  const bool cell = c < p.n, full = cell && p.full[c];
+  if (ll == 0 && w == 0 && cell) p.wflag[c] = full ? 0 : 1;  // CHECKSOL: FULL = 0 -> REDUCE
+  const int adm = full || (cell && p.mprev) ? p.admis[c] : 0;
+  const int A = p.admis_max, ID2 = p.ideg2;
+  const bool cw = p.ees == 5, low = cw && ll > 0, rem = cw && ll == 0;
+  const T* Gc = (const T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
+  if (rem) {
+    char_lower_sum<P, T>(p, Gc, adm, w, lane, s_g);
+    __syncthreads();
+  }
+  const T ilc = T(1.0 / (1.0 - 1.0 / p.lwci));
+  auto Gp = [&](int d, int u) -> T {
+    const T g = Gc[(int64_t)((ll * ID + d) * NV + u) * 32];
+    return rem ? ilc * (g - (d < L2 && d < ID2 ? s_g[(d * NV + u) * 32 + lane] : T(0))) : g;
+  };
+  const T* Pc = (const T*)p.ind + grp * p.istride * 32 + lane * VEC;
+  T a[NV];
+#pragma unroll
+  for (int u = 0; u < NV; ++u) a[u] = T(0);
+  // a[u] += g[d][u] * sum_{e>=d} P_de g[e][w], the packed triangle as in quad_form
+  auto form = [&](auto& g, const T* Pl, int nd) {
+    constexpr int ND = sizeof(g) / sizeof(T);
+#pragma unroll
+    for (int d = 0; d < ND; ++d) g[d] = d < nd ? Gp(d, w) : T(0);
+    int rs = 0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if (d < nd) {
+        T t = T(0);
+#pragma unroll
+        for (int q = 0; q < (ND - d + VEC - 1) / VEC; ++q)
+          if (d + q * VEC < nd) {
+            T x[VEC];
+            ldv(Pl + (int64_t)(rs + q) * 32 * VEC, x);
+#pragma unroll
+            for (int i = 0; i < VEC; ++i)
+              if (d + q * VEC + i < ND) t += x[i] * g[d + q * VEC + i];
+          }
+        rs += (nd - d + VEC - 1) / VEC;
+#pragma unroll
+        for (int u = 0; u < NV; ++u) a[u] += Gp(d, u) * t;
+        asm volatile("" ::: "memory");  // as in quad_form
+      }
+  };
+  if (ll < adm) {
+    if (low) {
+      T g[L2];
+      form(g, Pc + (int64_t)(p.i2off / VEC) * 32 * VEC, ID2);
+    } else {
+      T g[ID];
+      form(g, Pc, ID);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NV; ++u) s_a[u * NV + w][lane] = a[u];
+  __syncthreads();
+  if (ll >= adm) return;
+  double* Qc = p.qbuf + grp * (int64_t)(A * 15) * 32 + lane;
+  int j = 0;
+#pragma unroll
+  for (int u = 0; u < NV; ++u)
+#pragma unroll
+    for (int k = u; k < NV; ++k, ++j)
+      if (j % NV == w)
+        Qc[(int64_t)(ll * 15 + j) * 32] = u == k ? (double)s_a[u * NV + u][lane]
+                                                 : 0.5 * ((double)s_a[u * NV + k][lane] + (double)s_a[k * NV + u][lane]);
+}
+
+// Faces of a block, whose polynomials of one variable stay in registers
+// together, so that each stencil polynomial is read once for all of them.
+template <int P, typename T>
+struct CharFaces {
+  static constexpr int value = P < 4 || sizeof(T) == 4 ? 3 : 2;
+};
+template <int P, typename T>
+__host__ __device__ constexpr size_t char_face_smem(int QS) {
+  constexpr int NF = CharFaces<P, T>::value, ID = Deg<P>::ideg, L2 = ID < 9 ? ID : 9;
+  return (size_t)NF * (50 + 7 * NV) * 32 * 8 + ((size_t)((QS * NV) | 1) + L2 * NV) * 32 * sizeof(T);
+}
+template <int P, typename T>
+__global__ void __launch_bounds__(32 * NV) k_char_face(Problem p, const double* __restrict__ U) {
+  constexpr int ID = Deg<P>::ideg;
+  constexpr int L2 = ID < 9 ? ID : 9;
+  constexpr int NF = CharFaces<P, T>::value;
+  constexpr int MA = 7;  // stencils per cell at most
+  extern __shared__ __align__(16) unsigned char cf_smem[];
+  const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  const int FQ = MF * QS, RS = (QS * NV) | 1;
+  double* s_e = (double*)cf_smem;          // [NF][50][32]: left, then right eigenvectors
+  double* s_w = s_e + NF * 50 * 32;        // [NF][MA][NV][32]: weights
+  T* s_g = (T*)(s_w + NF * MA * NV * 32);  // [L2][NV][32]: char_lower_sum
+  T* s_o = s_g + L2 * NV * 32;             // [32][RS]: the values of one face
+  const int lane = threadIdx.x & 31, v = threadIdx.x >> 5;
+  const int64_t grp = blockIdx.x, c = grp * 32 + lane;
+  const int f0 = blockIdx.y * NF;
+  const bool cell = c < p.n;
+  const bool live = cell && (p.full[c] || p.mprev);
+  const int adm = live ? p.admis[c] : 0, nf = live ? p.nfaces[c] : 0;
+  const int A = p.admis_max, ID2 = p.ideg2;
+  const bool cw = p.ees == 5;
+  const double lc1 = 1.0 - 1.0 / p.lwci;
+  const double lk = adm > 1 ? (1.0 - lc1) / (adm - 1) : 0.0;
+  const T* Gc = (const T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
+  double u0[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) u0[k] = cell ? U[c * NV + k] : 1.0;
+  for (int f = v; f < NF; f += NV)
+    if (f0 + f < nf) {
+      const int64_t cf = c * MF + f0 + f;
+      double r[4], ur[NV], rl[NV], rr[NV];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r[k] = p.rot[cf * 4 + k];
+      const int64_t nb = p.neigh[cf];
+      if (nb >= 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) ur[k] = U[nb * NV + k];
+      } else {
+        boundary_ghost(p, p.bc[cf], r, u0, ur);
+      }
+      rot_f(r, u0, rl);
+      rot_f(r, ur, rr);
+      char_eigenvectors(p.gamma, rl, rr, s_e + f * 50 * 32 + lane, s_e + (f * 50 + 25) * 32 + lane, 32);
+    }
+  if (cw) char_lower_sum<P, T>(p, Gc, adm, v, lane, s_g);
+  __syncthreads();
+  // indicators and weights (WENOWEIGHTS, FP64) of characteristic variable v
+  const double* Qc = p.qbuf + grp * (int64_t)(A * 15) * 32 + lane;
+  for (int f = 0; f < NF; ++f) {
+    if (f0 + f >= nf) break;
+    double l[NV], w[MA];
+#pragma unroll
+    for (int u = 0; u < NV; ++u) l[u] = s_e[(f * 50 + v * NV + u) * 32 + lane];
+    double tau = 0.0, sum = 0.0;
+#pragma unroll
+    for (int ll = 0; ll < MA; ++ll) {
+      w[ll] = 0.0;
+      if (ll < adm) {
+        double is = 0.0;
+        int j = 0;
+#pragma unroll
+        for (int u = 0; u < NV; ++u)
+#pragma unroll
+          for (int k = u; k < NV; ++k, ++j)
+            is += (u == k ? 1.0 : 2.0) * l[u] * l[k] * Qc[(int64_t)(ll * 15 + j) * 32];
+        w[ll] = is;
+      }
+    }
+    if (cw && p.wenoz) {
+#pragma unroll
+      for (int ll = 0; ll < MA; ++ll)
+        if (ll < adm) tau += fabs(w[0] - w[ll]);
+      tau = tau / (adm - 1);
+    }
+#pragma unroll
+    for (int ll = 0; ll < MA; ++ll)
+      if (ll < adm) {
+        const double e = p.weno_eps + w[ll];
+        const double lam = ll == 0 ? (cw ? lc1 : p.lwci) : (cw ? lk : 1.0);
+        if (cw && p.wenoz) {
+          double q = tau / e;
+          q = q * q;
+          w[ll] = lam * (1.0 + q * q);
+        } else {
+          const double e2 = e * e;
+          w[ll] = lam / (e2 * e2);
+        }
+        sum += w[ll];
+      }
+#pragma unroll
+    for (int ll = 0; ll < MA; ++ll)
+      if (ll < adm) s_w[((f * MA + ll) * NV + v) * 32 + lane] = w[ll] / sum;
+  }
+  __syncthreads();
+  // the faces' polynomials of variable v
+  T gh[NF][ID];
+  double fm[NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    fm[f] = 0.0;
+#pragma unroll
+    for (int d = 0; d < ID; ++d) gh[f][d] = T(0);
+  }
+#pragma unroll 1
+  for (int ll = 0; ll < adm; ++ll) {
+    const int nd = cw && ll > 0 ? ID2 : ID;
+    const bool rem = cw && ll == 0;
+    T M[NF][NV];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+#pragma unroll
+      for (int u = 0; u < NV; ++u) M[f][u] = T(0);
+      if (f0 + f < nf) {
+        const double *EL = s_e + f * 50 * 32 + lane, *ER = EL + 25 * 32, *wf = s_w + (f * MA + ll) * NV * 32 + lane;
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+          double a = 0.0;
+#pragma unroll
+          for (int j = 0; j < NV; ++j) a += ER[(v * NV + j) * 32] * wf[j * 32] * EL[(j * NV + u) * 32];
+          fm[f] += a * u0[u];
+          M[f][u] = T(a);
+        }
+      }
+    }
+    const T* Gl = Gc + (int64_t)(ll * ID) * NV * 32;
+#pragma unroll
+    for (int d = 0; d < ID; ++d)
+      if (d < nd) {
+        T gu[NV];
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+          gu[u] = Gl[(int64_t)(d * NV + u) * 32];
+          if (rem) gu[u] = T(1.0 / lc1) * (gu[u] - (d < L2 && d < ID2 ? s_g[(d * NV + u) * 32 + lane] : T(0)));
+        }
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+          for (int u = 0; u < NV; ++u) gh[f][d] += M[f][u] * gu[u];
+      }
+  }
+  // face values, CHECKSOL and the stores, face by face
+  const T* bmv = (const T*)p.bmean + grp * (int64_t)ID * 32 + lane;
+  const T* xq = (const T*)p.qpts + grp * (int64_t)FQ * 3 * 32 + lane;
+  double pm[NV];
+  cons2prim(p.gamma, u0, pm);
+  bool flag = false;
+  T* out = (T*)p.dul + grp * 32 * (int64_t)FQ * NV;
+  const int ncl = p.n - grp * 32 < 32 ? (int)(p.n - grp * 32) : 32;
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    const int fc = f0 + f;
+    if (fc >= MF) break;
+    if (f) __syncthreads();  // the stores of the last face have read s_o
+    const int nq = fc < nf ? face_nq(p, p.ftype[c * MF + fc]) : 0;
+    T cb = T(0);
+#pragma unroll
+    for (int d = 0; d < ID; ++d) cb += bmv[d * 32] * gh[f][d];
+    for (int q = 0; q < QS; ++q) {
+      T r = T(0);
+      if (q < nq) {
+        const T* xi = xq + (int64_t)(fc * QS + q) * 3 * 32;
+        T m[ID], t = T(0);
+        monomials<P, T>(xi[0], xi[32], xi[64], m);
+#pragma unroll
+        for (int d = 0; d < ID; ++d) t += m[d] * gh[f][d];
+        r = T((fm[f] - u0[v]) + (double)(t - cb));
+      }
+      s_o[lane * RS + q * NV + v] = r;
+    }
+    __syncthreads();
+    for (int q = v; q < nq; q += NV) {  // CHECKSOL (0.85): warp v takes the points v, v + NV, ...
+      double uf[NV];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) uf[k] = u0[k] + (double)s_o[lane * RS + q * NV + k];
+      flag = flag || jump_bad(p.gamma, pm, uf, 0.85);
+    }
+    for (int cl = v; cl < ncl; cl += NV)
+      for (int r = lane; r < QS * NV; r += 32) out[(int64_t)cl * FQ * NV + fc * QS * NV + r] = s_o[cl * RS + r];
+  }
+  if (flag) p.wflag[c] = 1;  // to the MUSCL fall-back (k_wpost<..., FB>)
+}
+
+// Characteristic-variable post-processing: compiled only in recon_char*.cu
+// (explicit instantiations), in parallel with the other reconstruction units.
 template <int P, typename T>
 cudaError_t launch_wpost_char(const Problem& p, const double* U, cudaStream_t st) {
-  k_wpost<P, T, true><<<(unsigned)((p.n + 63) / 64), 64, 0, st>>>(p, U);
+  const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  constexpr int NF = CharFaces<P, T>::value;
+  const unsigned ng = (unsigned)((p.n + 31) / 32);
+  const size_t smem = char_face_smem<P, T>(QS);
+  const cudaError_t e = cudaFuncSetAttribute(k_char_face<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_char_forms<P, T><<<dim3(ng, (unsigned)p.admis_max), 32 * NV, 0, st>>>(p);
+  k_char_face<P, T><<<dim3(ng, (MF + NF - 1) / NF), 32 * NV, smem, st>>>(p, U);
+  k_wpost<P, T, false, true><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
   return cudaGetLastError();
 }
 #ifndef UCG_RECON_CHAR_TU
@@ -1351,7 +1404,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
   Problem pa = p;
   pa.n = p.nall > p.n ? p.nall : p.n;
   if (p.mmus) {  // the first MOOD cascade: MUSCL of the selected cells from this stage's G
-    k_wpost<P, T, false, false, true, true><<<b, 128, 0, st>>>(p, U);
+    k_wpost<P, T, false, true, true><<<b, 128, 0, st>>>(p, U);
     ++*launches;
     return cudaGetLastError();
   }
@@ -1375,6 +1428,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
   if (p.wenwrt == 2) {
     const cudaError_t e = launch_wpost_char<P, T>(p, U, st);
     if (e != cudaSuccess) return e;
+    *launches += 2;
   } else {
     // indicators in their own kernel at IORDER 4, where the cell's packed
     // triangle (595 entries) no longer stays in L1 between the stencils of
@@ -1389,7 +1443,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
         cudaFuncSetAttribute(k_wface<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_wis<P, T><<<(unsigned)((p.n + 31) / 32), 32 * p.admis_max, 0, st>>>(p);
         k_wface<P, T><<<(unsigned)((p.n + 31) / 32), 32 * NV, smem, st>>>(p, U);
-        k_wpost<P, T, false, false, true><<<b, 128, 0, st>>>(p, U);
+        k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
         *launches += 2;
         done = true;
       }
@@ -1397,7 +1451,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     if constexpr (P == 4) {
       if (!done && p.isb && p.scheme == 3) {
         k_wis<P, T><<<(unsigned)((p.n + 31) / 32), 32 * p.admis_max, 0, st>>>(p);
-        k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
+        k_wpost<P, T, true><<<b, 128, 0, st>>>(p, U);
         ++*launches;
         done = true;
       }
