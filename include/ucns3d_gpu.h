@@ -269,19 +269,21 @@ int ucg_synchronize(ucg_engine* e);
 /* Average device time of the stage kernels over `reps` residual
  * evaluations of the current state, measured with CUDA events on the
  * handle's stream, into ms[4]: ms[0] reconstruction, ms[1] face fluxes,
- * ms[2] time step (CALCULATE_CFL), ms[3] the stencil least-squares kernel
+ * ms[2] time step (CALCULATE_CFL), ms[3] the stencil least squares
  * alone (part of ms[0]; all of it for MUSCL IORDER 1), after one untimed
  * evaluation.  For profiling; it leaves the state unchanged.               */
 int ucg_time_kernels(ucg_engine* e, int32_t reps, double* ms);
 
-/* Bounded device waits.  The opt-in least squares through the shared-memory
- * bulk-copy ring (UCG_LSQ_BULK=1 in the environment at ucg_create) waits on
- * each copy for at most `polls` polls (about 300 ns each; the default, about
- * 20 ms, is restored by polls < 0).  A wait that gives up makes its warp
- * finish the copies it has in flight (each with the default bound) and
- * return, and the next ucg_check_health reports UCG_ETIMEOUT; the handle
- * stays usable.  polls = 0 makes every such wait give up at once, which
- * exercises that path without a fault.  No counterpart in the reference. */
+/* Bounded device waits.  The stencil least squares passes its tables and
+ * gathered states through rings in shared memory, whose waits give up after
+ * 65,536 polls (about 300 ns each, about 20 ms in all).  An engine created
+ * with UCG_LSQ_BULK=1 in the environment takes `polls` as its bound instead
+ * (the default is
+ * restored by polls < 0).  A wait that gives up makes its block finish the
+ * copies it has in flight (each with the default bound) and return, and the
+ * next ucg_check_health reports UCG_ETIMEOUT; the handle stays usable.
+ * polls = 0 makes every such wait give up at once, which exercises that path
+ * without a fault.  No counterpart in the reference. */
 int ucg_set_wait_limit(ucg_engine* e, int64_t polls);
 
 /* The cell numbering chosen at ucg_upload_geometry.  With cfg.reorder 1 the

@@ -1415,8 +1415,7 @@ int force_device(ucg_engine* e, const Problem& p, const double* U, const double*
   if (dU && weno) {  // the tangent face values: dG = least squares of dU, then the WENO tangent
     Problem pt = p;
     pt.gbuf = e->adjw_gbar.p;
-    CK(launch_lsq_f64(e->cfg.iorder, pt, dU, e->stream));
-    e->launches++;
+    CK(launch_lsq_f64(e->cfg.iorder, pt, dU, e->stream, &e->launches));
     if ((rc = launch_weno_tangent(e, p, U, dU, (const double*)e->adjw_gbar.p, tdul))) return rc;
   } else if (dU) {
     k_jvp_muscl<<<blocks_for(e->n, 128), 128, 0, e->stream>>>(p, U, dU, tdul, nullptr, false);
@@ -1587,8 +1586,7 @@ int weno_jvp_device(ucg_engine* e, const Problem& p, const double* U, const doub
   if (rc) return rc;
   Problem pt = p;
   pt.gbuf = e->adjw_gbar.p;  // dG = least squares of dU
-  CK(launch_lsq_f64(e->cfg.iorder, pt, dU, e->stream));
-  e->launches++;
+  CK(launch_lsq_f64(e->cfg.iorder, pt, dU, e->stream, &e->launches));
   double* tdul = (double*)e->adjw_face.p;
   double* tflux = (double*)e->adjw_contrib.p;
   if ((rc = launch_weno_tangent(e, p, U, dU, (const double*)e->adjw_gbar.p, tdul))) return rc;

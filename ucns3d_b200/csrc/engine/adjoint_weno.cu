@@ -3,7 +3,7 @@
 // and smoothness indicators (src/reconstruct_p.f90:920-1250) and of the
 // stencil least squares (LEAST_SQUARES, src/gradients.f90:253-497).
 //
-// Forward, per cell c and variable v (k_lsq, k_wpost):
+// Forward, per cell c and variable v (the least squares, k_wpost):
 //   G_l  = M_l (U_st(l,k) - U_c)                         l < ADMIS
 // (The tangent, k_jvp_wpost, pushes dG = M_l (dU_st - dU_c) forward instead.)
 //   IS_l = G_l^T S G_l,  wt_l = lam_l / (eps + IS_l)^4,  om_l = wt_l / sum wt
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_adj_wpost(Problem 
 }
 
 // k_adj_lsq: one lane per cell, the transpose of the stencil least squares,
-// shaped like k_lsq: DH rows of Gb in registers per pass, the members of
+// DH rows of Gb in registers per pass, the members of
 // the stencil streamed; a member's contribution is the sum of its row
 // passes (the first writes, the next add).  Contributions go to slot-major
 // buffers: slot 0 the cell, 1 + l*IMAX + k member k of stencil l (CWENO:

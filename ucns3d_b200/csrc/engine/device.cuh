@@ -82,15 +82,15 @@ struct Problem {
   double* fgrad;            // [nown][QS][4][3] face-point average of both sides' gradients of T,u,v,w (WENO)
   void* gv;                 // [n][ideg][4]  viscous LSQ coefficients, in the table precision
   double* prim;             // [n][4] T, u, v, w of each cell (viscous LSQ, formed once per stage)
-  double* upad;             // [n][6] conserved state in 48-byte records (k_lsq gathers, formed once per stage)
   double* rhs;              // [n][NV] residual output (residual-only mode)
   const int32_t* own;       // owned faces, code cell*8 + face
   int64_t nown;
   double* fflux;            // [n][MF][NV] convective face sums (owner and negated copy)
   double* vflux;            // [n][MF][NV] viscous face sums
   unsigned* health;
-  int lsq_bulk;  // stencil least squares through the shared-memory bulk-copy ring (k_lsq_tma)
-  long lsq_wait; // polls of a k_lsq_tma stage wait before it gives up (< 0: the default)
+  bool lsq_bulk; // lsq_wait is the bound of the least squares' waits
+  long lsq_wait; // polls of a stage wait before it gives up (< 0: the default)
+  int nsm;       // SMs of the device
   int wenwrt;    // 1 conserved-variable WENO, 2 characteristic-variable WENO
   int riemann;   // 1 HLLC, 2 Rusanov, 3 Roe, 4 rotated Roe-HLL, 5 t-Roe, 9 HLL
   int limiter;   // SLOPE_LIMITERS code (7 Venkatakrishnan)
@@ -676,6 +676,9 @@ __device__ __forceinline__ void fence_proxy_async() {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile(

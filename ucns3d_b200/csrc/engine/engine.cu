@@ -142,7 +142,6 @@ Problem make_problem(ucg_engine* e) {
   p.fgrad = (double*)e->fgrad.p;
   p.gv = e->gv.p;
   p.prim = (double*)e->prim.p;
-  p.upad = (double*)e->upad.p;
   p.rhs = (double*)e->rhs.p;
   p.own = (const int32_t*)e->own.p;
   p.nown = e->nown;
@@ -152,7 +151,8 @@ Problem make_problem(ucg_engine* e) {
   p.dt_dev = nullptr;
   p.dt_next = nullptr;
   p.ccfl = 0.0;
-  p.lsq_bulk = e->lsq_bulk ? 1 : 0;
+  p.lsq_bulk = e->lsq_bulk;
+  p.nsm = e->nsm;
   p.lsq_wait = e->lsq_wait;
   p.wenwrt = c.wenwrt;
   p.riemann = c.riemann;
@@ -192,7 +192,7 @@ int launch_recon_t(ucg_engine* e, const Problem& p, const double* U) {
 
 // the reconstruction covers cells [0, n_recon) (all of them unless a
 // partition's roles leave its outer halo out); the per-cell records that
-// stencils gather (k_pad_state, k_visc_prim) still cover every cell
+// the viscous stencils gather (k_visc_prim) still cover every cell
 int launch_recon(ucg_engine* e, const Problem& p, const double* U) {
   Problem pr = p;
   pr.n = e->n_recon;
@@ -522,6 +522,7 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
   {
     const char* bulk = std::getenv("UCG_LSQ_BULK");
     e->lsq_bulk = bulk && bulk[0] == '1';
+    e->nsm = prop.multiProcessorCount;
   }
   {
     // slices and smoothness blocks padded to 16 bytes (bulk-copy granularity)
@@ -564,10 +565,8 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
   if (c.governing == 1) rc = rc ? rc : alloc(e, e->vflux, (size_t)n * MF * NV * 8);
   rc = rc ? rc : alloc(e, e->dul, (size_t)n * MF * e->QS * NV * T);
   const int64_t ngrp = (n + 31) / 32;
-  if (!(c.scheme == 2 && c.iorder == 1)) {
+  if (!(c.scheme == 2 && c.iorder == 1))
     rc = rc ? rc : alloc(e, e->gbuf, (size_t)ngrp * 32 * c.admis_max * c.ideg * NV * T);
-    if (c.iorder == 3) rc = rc ? rc : alloc(e, e->upad, (size_t)n * 6 * 8);  // k_lsq<3, T, true>
-  }
   if (c.scheme == 3 && c.wenwrt == 1 && c.iorder == 4) {  // smoothness indicators of every stencil (k_wis)
     const char* wis = std::getenv("UCG_WENO_IS");
     if (!(wis && wis[0] == '0')) rc = rc ? rc : alloc(e, e->isb, (size_t)ngrp * 32 * c.admis_max * NV * 8);
@@ -621,7 +620,7 @@ void ucg_destroy(ucg_engine* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   DevBuf* all[] = {&e->nfaces, &e->ftype, &e->neigh, &e->nface, &e->bc, &e->qperm, &e->rot, &e->area, &e->dih,
                    &e->vol, &e->minedge, &e->jinv, &e->admis, &e->full, &e->qpts, &e->bmean, &e->sten, &e->invmat,
-                   &e->ind, &e->dul, &e->ulv, &e->gv, &e->prim, &e->upad, &e->rhs, &e->Un, &e->Ua, &e->Ub,
+                   &e->ind, &e->dul, &e->ulv, &e->gv, &e->prim, &e->rhs, &e->Un, &e->Ua, &e->Ub,
                    &e->health, &e->dt, &e->partial, &e->red, &e->staging, &e->own, &e->fflux, &e->vflux, &e->gbuf,
                    &e->qbuf, &e->d_n2o, &e->permbuf, &e->fgrad, &e->isb, &e->wflag, &e->mprev, &e->mflag,
                    &e->msel, &e->mmus, &e->mord, &e->Um, &e->imp_dtl, &e->imp_dinv, &e->imp_off, &e->imp_du,
@@ -1183,7 +1182,7 @@ int ucg_time_kernels(ucg_engine* e, int32_t reps, double* ms) {
   for (auto& x : ev) CK(cudaEventCreate(&x));
   double acc[4] = {0, 0, 0, 0};
   int rc = UCG_OK;
-  const bool split = !(e->cfg.scheme == 2 && e->cfg.iorder == 1);  // k_lsq + k_wpost
+  const bool split = !(e->cfg.scheme == 2 && e->cfg.iorder == 1);  // least squares, then the rest
   // r = -1: one untimed pass (first launches load the kernels' modules)
   for (int r = -1; r < reps && !rc; ++r) {
     cudaEventRecord(ev[0], e->stream);

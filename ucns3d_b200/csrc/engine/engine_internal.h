@@ -15,7 +15,7 @@
 
 namespace ucg {
 // the stencil least squares alone, FP64 tables (recon_f64.cu)
-cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st);
+cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st, int64_t* launches);
 }  // namespace ucg
 
 namespace ucg_host {
@@ -54,7 +54,7 @@ struct ucg_engine {
   // tables
   DevBuf sten, invmat, ind;
   // scratch and state
-  DevBuf gbuf, isb, wflag, dul, ulv, fgrad, gv, prim, upad, rhs, Un, Ua, Ub, health, dt, partial, red, staging, own, fflux, vflux, qbuf;
+  DevBuf gbuf, isb, wflag, dul, ulv, fgrad, gv, prim, rhs, Un, Ua, Ub, health, dt, partial, red, staging, own, fflux, vflux, qbuf;
   // MOOD (cfg.mood): RECALC, the cascade's flags and selections, MOOD_O, the candidate state
   DevBuf mprev, mflag, msel, mmus, mord, Um;
   // implicit steps (ucg_implicit_step): local time steps, inverse diagonals, face blocks, corrections
@@ -65,10 +65,11 @@ struct ucg_engine {
   double totvol = 0.0;      // TOTALVOLUME
   int64_t nown = 0;
   int64_t nown_plain = 0;  // owned faces [0, nown_plain): interior and mirror; the rest other boundaries
-  cudaEvent_t mark = nullptr;  // recorded after k_lsq while ucg_time_kernels runs
-  bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: k_lsq_tma instead of k_lsq
+  cudaEvent_t mark = nullptr;  // recorded after the least squares while ucg_time_kernels runs
+  bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: ucg_set_wait_limit sets the least squares' bound
+  int nsm = 148;
   bool wface = false;          // IORDER 4 conserved WENO: face values one warp per variable (k_wface)
-  long lsq_wait = -1;          // polls of a k_lsq_tma stage wait (ucg_set_wait_limit; < 0 the default)
+  long lsq_wait = -1;          // polls of a k_lsq_ring stage wait (ucg_set_wait_limit; < 0 the default)
   std::vector<uint8_t> recon_done;  // per cell, for ucg_upload_recon chunks
   std::vector<int8_t> admis_h;      // ADMIS per cell, for the stencil checks of ucg_upload_recon
   std::vector<int32_t> neigh_h;     // [n][6] face neighbours (host copy, adjoint set-up)

@@ -1,256 +1,251 @@
-// Reconstruction for WENO / CWENO / high-order MUSCL in two kernels.
+// Reconstruction for WENO / CWENO / high-order MUSCL.
 //
-// k_lsq      LEAST_SQUARES (src/gradients.f90:253-497): one lane per cell.
-//            Tables are interleaved over groups of 32 cells, so every table
-//            load of a warp is one contiguous 128/256-byte row; each gathered
-//            difference U_k - U_i is reused across DH rows held in registers.
-//            Output: the stencil polynomials G[ll][d][v], interleaved.
-// k_wpost    CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL,
-//            MUSCL fall-back, CHECKSOLX (3126-3406): one lane per cell, no
-//            block barriers; smoothness indicators as packed quadratic forms.
+// LEAST_SQUARES (src/gradients.f90:253-497), stencil polynomials G[ll][d][v]:
+//   k_lsq_ring  the cells' tables, streamed from DRAM through shared memory
+//               (interleaved over groups of 32 cells)
+// CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL, MUSCL
+// fall-back, CHECKSOLX (3126-3406): k_wpost, one lane per cell, no block
+// barriers, smoothness indicators as packed quadratic forms; at IORDER 4
+// k_wis and k_wface; characteristic variables k_char_forms and
+// k_char_face.
 #pragma once
 
 #include "device.cuh"
 
+
 namespace ucg {
 
-// rows of G held in registers per pass (accumulators: DH x 5 values of T)
+// rows of G that one warp holds in registers per pass (DH x 5 values of T)
 template <int P, typename T>
 struct LsqRows {
   static constexpr int ID = Deg<P>::ideg;
   static constexpr int value = P == 4 ? (sizeof(T) == 4 ? 34 : 17) : P == 3 ? (sizeof(T) == 4 ? 19 : 10) : ID;
 };
 
-// The conserved state in 48-byte records (five values and a zero), formed
-// once per stage: k_lsq<P, T, true> gathers each stencil member with three
-// aligned 16-byte loads instead of five 8-byte loads.
-template <int P, typename T>
-__global__ void k_pad_state(Problem p, const double* __restrict__ U) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.n) return;
-  const double* u = U + c * NV;
-  double2* o = (double2*)(p.upad + c * 6);
-  o[0] = make_double2(u[0], u[1]);
-  o[1] = make_double2(u[2], u[3]);
-  o[2] = make_double2(u[4], 0.0);
-}
-
-// PAD: stencil members gathered from p.upad (the engine's stage), else from U
-// (also used on tangent states by the discrete adjoint).
-// FP32 at IORDER 3: four blocks per SM (128 registers instead of 160), at
-// IORDER 2 five (instead of four at 126): the gather of the stencil members
-// is latency-bound, and more warps in flight made the 2.1 M-cell CWENO4
-// step 6 % faster (61.1 -> 57.3 ms on one box) and the 82,944-tet WENO3
-// step 3 % (1.094 -> 1.063 ms); the same values bit for bit.  Five blocks
-// at IORDER 3 (102 registers) made the CWENO4 step slower (56.0 -> 58.0 ms).
-template <int P, typename T, bool PAD = false>
-__global__ void __launch_bounds__(128, sizeof(T) != 4 ? 1 : P == 3 ? 4 : P == 2 ? 5 : 1)
-    k_lsq(Problem p, const double* __restrict__ U) {
-  constexpr int ID = Deg<P>::ideg;
-  constexpr int DH = LsqRows<P, T>::value;
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int A = p.admis_max, W = p.imax + 1;
-  const bool cw = p.ees == 5;
-  const int64_t grp = c >> 5;
-  const int lane = (int)(c & 31);
-  const bool live = c < p.n;
-  const int adm = live ? p.admis[c] : 0;
-  double u0[NV];
+// Gathers of a producer warp for the 32 cells of its consumer.  The lanes
+// share a member's 32 records of 40 bytes element by element, lane l taking
+// the elements l, l + 32, ... of the 160, so that a load touches the lines of
+// six or seven records instead of 32 (a lane per record reads five values of
+// 32 distant records, five times over: with scattered members the L1 tag
+// lookups alone bound the kernel).  The differences go to shared memory as
+// they come, [cell][variable], which the consumer reads without bank
+// conflicts (row stride 5).
+struct GatherShare {
+  int r[NV], v[NV];
+  __device__ __forceinline__ explicit GatherShare(int lane) {
 #pragma unroll
-  for (int v = 0; v < NV; ++v) u0[v] = live ? U[c * NV + v] : 0.0;
-  const T* Mi = (const T*)p.invmat + grp * p.tstride * 32 + lane;
-  const int32_t* Si = p.sten + grp * (int64_t)(A * W) * 32 + lane;
-  T* Gi = (T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
-  for (int ll = 0; ll < A; ++ll) {
-    const bool low = cw && ll > 0;
-    const int nk = low ? p.imax2 : p.imax, nd = low ? p.ideg2 : ID;
-    const bool act = ll < adm;
-    for (int d0 = 0; d0 < nd; d0 += DH) {
-      T acc[DH][NV];
-#pragma unroll
-      for (int j = 0; j < DH; ++j)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[j][v] = T(0);
-      if (act) {
-        const T* M = Mi + (int64_t)(p.soff[ll] + d0) * 32;
-        const int32_t* S = Si + (ll * W + 1) * 32;
-#pragma unroll 2
-        for (int k = 0; k < nk; ++k) {
-          T du[NV];
-          if (PAD) {
-            const double2* q = (const double2*)(p.upad + (int64_t)S[k * 32] * 6);
-            const double2 a = q[0], b = q[1], e = q[2];
-            const double uy[NV] = {a.x, a.y, b.x, b.y, e.x};
-#pragma unroll
-            for (int v = 0; v < NV; ++v) du[v] = T(uy[v] - u0[v]);
-          } else {
-            const double* uy = U + (int64_t)S[k * 32] * NV;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) du[v] = T(uy[v] - u0[v]);
-          }
-          const T* Mk = M + (int64_t)k * nd * 32;
-#pragma unroll
-          for (int j = 0; j < DH; ++j)
-            if (d0 + j < nd) {
-              T m = Mk[j * 32];
-#pragma unroll
-              for (int v = 0; v < NV; ++v) acc[j][v] += m * du[v];
-            }
-        }
-      }
-      if (live)
-#pragma unroll
-        for (int j = 0; j < DH; ++j)
-          if (d0 + j < nd)
-#pragma unroll
-            for (int v = 0; v < NV; ++v) Gi[(int64_t)((ll * ID + d0 + j) * NV + v) * 32] = acc[j][v];
+    for (int i = 0; i < NV; ++i) {
+      r[i] = (lane + 32 * i) / NV;
+      v[i] = lane + 32 * i - r[i] * NV;
     }
   }
-}
-
-// k_lsq with the pseudo-inverse rows streamed through shared memory by bulk
-// copies.  Each warp owns one 32-cell group and a ring of NSTG stages; a
-// stage holds the rows [d0, d0 + DH) of one stencil member for the 32 cells
-// (DH * 32 table elements, contiguous in the interleaved layout), copied by
-// cp.async.bulk and completed on the stage's mbarrier.  Lane 0 refills a
-// stage as soon as the warp has consumed it, so NSTG - 1 members are in
-// flight while the warp multiplies the current one; the gathered neighbour
-// state of the next member is loaded one member ahead.  Same products and
-// accumulation order as k_lsq, so G is the same bit for bit.  A wait that
-// gives up (after Problem::lsq_wait polls) sets HEALTH_TIMEOUT, drains the
-// copies in flight (each wait bounded by LSQ_WAIT, whatever lsq_wait is) and
-// leaves the group.  Opt-in (Problem::lsq_bulk): on B200 it takes 7.2 ms
-// against k_lsq's 5.8 ms for the mixed WENO5 64^3 stage, at 3, 4 or 6
-// stages alike, because k_lsq is bound by the per-member gather of the
-// neighbour states and the issue rate of 8 warps per SM, not by the latency
-// of its coalesced table loads.
-template <int P, typename T>
-__host__ __device__ constexpr int lsq_stage_elems() {
-  return LsqRows<P, T>::value * 32;
-}
-template <int P, typename T, int NSTG>
-__host__ __device__ constexpr size_t lsq_tma_smem() {
-  return (size_t)4 * NSTG * lsq_stage_elems<P, T>() * sizeof(T) + (size_t)4 * NSTG * sizeof(uint64_t);
-}
+  // the lane's elements of the records of cells y (lane = cell)
+  __device__ __forceinline__ void load(const double* __restrict__ U, int y, double (&u)[NV]) const {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) u[i] = U[(int64_t)__shfl_sync(0xffffffffu, y, r[i]) * NV + v[i]];
+  }
+};
 
 // polls of one stage wait (about 20 ms; a stage normally lands in microseconds)
 constexpr long LSQ_WAIT = 1L << 16;
 
-template <int P, typename T, int NSTG>
-__global__ void __launch_bounds__(128) k_lsq_tma(Problem p, const double* __restrict__ U) {
-  constexpr int ID = Deg<P>::ideg;
-  constexpr int DH = LsqRows<P, T>::value;
-  constexpr int CH = lsq_stage_elems<P, T>();
-  extern __shared__ __align__(128) unsigned char lsq_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T* ring = (T*)lsq_smem + warp * NSTG * CH;
-  uint64_t* bar = (uint64_t*)((T*)lsq_smem + 4 * NSTG * CH) + warp * NSTG;
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t grp = c >> 5;
-  if (grp * 32 >= p.n) return;  // the whole warp: no cell of this group exists
-  const bool live = c < p.n;
-  const int A = p.admis_max, W = p.imax + 1;
-  const bool cw = p.ees == 5;
-  const int adm = live ? p.admis[c] : 0;
-  const int admw = __reduce_max_sync(0xffffffffu, adm);
-  double u0[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) u0[v] = live ? U[c * NV + v] : 0.0;
-  const T* Mg = (const T*)p.invmat + grp * p.tstride * 32;  // the group's tables
-  const int32_t* Si = p.sten + grp * (int64_t)(A * W) * 32 + lane;
-  T* Gi = (T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
-  if (lane == 0) {
-    for (int s = 0; s < NSTG; ++s) mbar_init(&bar[s], 1);
+// mbar_wait of a warp that also gives up when another warp of the block has
+__device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity, long limit, const volatile int* stop) {
+  bool ok = false;
+  for (long it = 0; it < limit; ++it) {
+    ok = mbar_try_wait(bar, parity);
+    if (ok || *stop) break;
+    if (it > 64) __nanosleep(256);
+  }
+  return __all_sync(0xffffffffu, ok);
+}
+
+// LEAST_SQUARES of the cells that read their own tables: the pseudo-inverse
+// rows and the gathered differences come through shared memory.  One or two
+// blocks per SM, four pairs of warps: a producer gathers the members'
+// differences into a stage of its pair's ring and issues the
+// bulk copies (cp.async.bulk) of the members' rows [d0, d0 + DH) of the 32
+// cells, which are contiguous in the interleaved layout; the consumer
+// multiplies.  The full barrier of a stage completes on the producer's arrival
+// and the copied bytes, the empty barrier on the consumer's arrival.  The
+// kernel is bound by the table bytes from DRAM.  One lane per cell holding the
+// accumulators and the loads in flight was bound by the bytes that its
+// registers left room for and by the chain index -> state -> product of each
+// member; here the copies run NSTG stages ahead.  The work is the list of
+// (group, stencil) items, an equal share of consecutive items per pair, so
+// that a mesh of any size fills the SMs (one lane per cell: 16,464 cells were
+// 129 blocks).  Against one lane per cell: 16,464 tetrahedra, WENO5
+// mixed, 0.500 -> 0.257 ms (1.63 GB, 6.3 TB/s); 82,944, WENO3, FP64 0.312 ->
+// 0.201 (6.4 TB/s), mixed 0.205 -> 0.190; 24,576, CWENO4, FP64 0.160 -> 0.107,
+// mixed 0.237 -> 0.067; two blocks per SM at IORDER 2 and 3 against one: 0.267
+// -> 0.201 (WENO3 FP64), 0.121 -> 0.067 (CWENO4 mixed).
+//
+// Every wait is bounded (`wait` polls).  A wait that gives up sets
+// HEALTH_TIMEOUT and s_stop; the other warps see it in their own waits, and a
+// producer leaves only after its copies in flight have landed (each wait
+// bounded by LSQ_WAIT, whatever `wait` is).
+template <int P, typename T>
+struct Ring {
+  static constexpr int DH = LsqRows<P, T>::value;
+  static constexpr int TAB = DH * 32 * sizeof(T), DU = NV * 32 * sizeof(T);  // of a member
+  static constexpr int MS = 2;                                               // members of a stage
+  static constexpr int STAGE = MS * (TAB + DU);
+  // blocks per SM: two where the accumulators leave room (128 registers)
+  static constexpr int BPS = DH * NV * sizeof(T) <= 400 ? 2 : 1;
+  static constexpr int NSTG = 56000 / BPS / STAGE < 8 ? 56000 / BPS / STAGE : 8;
+  static constexpr int GRP = 4;  // members that a producer gathers together
+  static constexpr size_t smem = (size_t)4 * NSTG * STAGE;
+};
+template <int P, typename T>
+__global__ void __launch_bounds__(256, Ring<P, T>::BPS) k_lsq_ring(Problem p, const double* __restrict__ U, int64_t items, long wait) {
+  using R = Ring<P, T>;
+  constexpr int ID = Deg<P>::ideg, DH = R::DH, NSTG = R::NSTG, GRP = R::GRP, MS = R::MS;
+  extern __shared__ __align__(128) unsigned char rg_smem[];
+  __shared__ __align__(8) uint64_t s_full[4][NSTG], s_empty[4][NSTG];
+  __shared__ int s_stop;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pair = warp & 3;
+  const bool producer = warp >= 4;
+  unsigned char* ring = rg_smem + (size_t)pair * NSTG * R::STAGE;
+  uint64_t *full = s_full[pair], *empty = s_empty[pair];
+  if (threadIdx.x == 0) {
+    s_stop = 0;
+    for (int w = 0; w < 4; ++w)
+      for (int s = 0; s < NSTG; ++s) {
+        mbar_init(&s_full[w][s], 1);
+        mbar_init(&s_empty[w][s], 1);
+      }
     mbar_fence_init();
   }
-  __syncwarp();
-  // copy cursor: the next (stencil, row pass, member) to copy, tracked by
-  // every lane (warp-uniform); lane 0 issues the copies
-  int ill = 0, id0 = 0, ik = 0;
-  auto n_k = [&](int ll) { return cw && ll > 0 ? p.imax2 : p.imax; };
-  auto n_d = [&](int ll) { return cw && ll > 0 ? p.ideg2 : ID; };
-  auto copy_next = [&](int slot) {
-    const int nd = n_d(ill);
-    if (lane == 0) {
-      const int rows = nd - id0 < DH ? nd - id0 : DH;
-      const unsigned bytes = (unsigned)(rows * 32 * sizeof(T));
-      fence_proxy_async();
-      mbar_expect_tx(&bar[slot], bytes);
-      bulk_g2s(ring + slot * CH, Mg + (int64_t)(p.soff[ill] + id0 + ik * nd) * 32, bytes, &bar[slot]);
-    }
-    if (++ik == n_k(ill)) {
-      ik = 0;
-      id0 += DH;
-      if (id0 >= nd) {
-        id0 = 0;
-        ++ill;
-      }
-    }
-  };
-  int issued = 0;
-  for (; issued < NSTG && ill < admw; ++issued) copy_next(issued);
-  int t = 0;  // members consumed
+  __syncthreads();
+  const int A = p.admis_max, W = p.imax + 1;
+  const bool cw = p.ees == 5;
+  const int64_t pairs = (int64_t)gridDim.x * 4, me = (int64_t)blockIdx.x * 4 + pair;
+  const int64_t i0 = items * me / pairs, i1 = items * (me + 1) / pairs;
+  const GatherShare sh(lane);
+  int slot = 0;
+  unsigned ph = 0;  // phase of the ring's current round
+  int issued = 0;   // producer: stages filled, for the drain
   bool ok = true;
-  const long wait = p.lsq_wait < 0 ? LSQ_WAIT : p.lsq_wait;
-  for (int ll = 0; ll < admw && ok; ++ll) {
-    const int nk = n_k(ll), nd = n_d(ll);
-    const bool act = ll < adm;
-    const int32_t* S = Si + (ll * W + 1) * 32;
-    for (int d0 = 0; d0 < nd && ok; d0 += DH) {
-      T acc[DH][NV];
+  for (int64_t it = i0; it < i1 && ok; ++it) {
+    const int64_t g = it / A;
+    const int ll = (int)(it - g * A);
+    const int64_t grp = g, c = grp * 32 + lane;
+    const bool low = cw && ll > 0, live = c < p.n;
+    const int nk = low ? p.imax2 : p.imax, nd = low ? p.ideg2 : ID;
+    const bool act = live && ll < p.admis[c];
+    const bool any = __any_sync(0xffffffffu, act);
+    if (producer) {
+      if (!any) continue;
+      const int32_t* S = p.sten + (grp * (int64_t)(A * W) + ll * W + 1) * 32 + lane;
+      const int own = (int)(c < p.n ? c : grp * 32);
+      auto member = [&](int k) -> int { return act ? S[(k < nk ? k : nk - 1) * 32] : own; };
+      double u0[NV];
+      sh.load(U, own, u0);
+      const T* M = (const T*)p.invmat + (grp * p.tstride + p.soff[ll]) * 32;
+      for (int d0 = 0; d0 < nd && ok; d0 += DH) {
+        const unsigned bytes = (unsigned)((nd - d0 < DH ? nd - d0 : DH) * 32 * sizeof(T));
+        int y[GRP];
 #pragma unroll
-      for (int j = 0; j < DH; ++j)
+        for (int j = 0; j < GRP; ++j) y[j] = member(j);
+        for (int k = 0; k < nk && ok; k += GRP) {
+          double u[GRP][NV];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) acc[j][v] = T(0);
-      double un[NV] = {0, 0, 0, 0, 0};  // state of member k, loaded one member ahead
-      if (act) {
-        const double* uy = U + (int64_t)S[0] * NV;
+          for (int j = 0; j < GRP; ++j) sh.load(U, y[j], u[j]);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) un[v] = uy[v];
-      }
-      for (int k = 0; k < nk; ++k) {
-        T du[NV];
+          for (int j = 0; j < GRP; ++j) y[j] = member(k + GRP + j);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) du[v] = T(un[v] - u0[v]);
-        if (act && k + 1 < nk) {
-          const double* uy = U + (int64_t)S[(k + 1) * 32] * NV;
+          for (int j0 = 0; j0 < GRP; j0 += MS) {
+            if (k + j0 >= nk) break;
+            if (!(ok = ring_wait(&empty[slot], ph ^ 1u, wait, &s_stop))) break;  // the first round finds them empty
+            unsigned char* st = ring + slot * R::STAGE;
+            T* du = (T*)(st + MS * R::TAB) + lane;
 #pragma unroll
-          for (int v = 0; v < NV; ++v) un[v] = uy[v];
-        }
-        const int slot = t % NSTG;
-        if (!__all_sync(0xffffffffu, mbar_wait(&bar[slot], (unsigned)(t / NSTG) & 1u, wait))) {
-          ok = false;
-          break;
-        }
-        if (act) {
-          const T* Mk = ring + slot * CH + lane;
+            for (int j = 0; j < MS; ++j)
 #pragma unroll
-          for (int j = 0; j < DH; ++j)
-            if (d0 + j < nd) {
-              const T m = Mk[j * 32];
-#pragma unroll
-              for (int v = 0; v < NV; ++v) acc[j][v] += m * du[v];
+              for (int i = 0; i < NV; ++i) du[(j * NV + i) * 32] = T(u[j0 + j][i] - u0[i]);
+            __syncwarp();
+            if (lane == 0) {
+              const int km = nk - k - j0 < MS ? nk - k - j0 : MS;
+              fence_proxy_async();
+              mbar_expect_tx(&full[slot], bytes * km);
+              for (int j = 0; j < km; ++j)
+                bulk_g2s(st + j * R::TAB, M + ((int64_t)(k + j0 + j) * nd + d0) * 32, bytes, &full[slot]);
             }
-        }
-        __syncwarp();
-        ++t;
-        if (ill < admw) {  // refill the stage just consumed
-          copy_next(slot);
-          ++issued;
+            ++issued;
+            if (++slot == NSTG) slot = 0, ph ^= 1u;
+          }
         }
       }
-      if (ok && live)
+    } else {
+      T* Gi = (T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + (int64_t)(ll * ID) * NV * 32 + lane;
+      for (int d0 = 0; d0 < nd && ok; d0 += DH) {
+        T acc[DH][NV];
 #pragma unroll
         for (int j = 0; j < DH; ++j)
-          if (d0 + j < nd)
 #pragma unroll
-            for (int v = 0; v < NV; ++v) Gi[(int64_t)((ll * ID + d0 + j) * NV + v) * 32] = acc[j][v];
+          for (int v = 0; v < NV; ++v) acc[j][v] = T(0);
+        if (any)
+          for (int k = 0; k < nk; k += MS) {
+            if (!(ok = ring_wait(&full[slot], ph, wait, &s_stop))) break;
+            const unsigned char* st = ring + slot * R::STAGE;
+            const T* m = (const T*)st + lane;
+            const T* d = (const T*)(st + MS * R::TAB) + lane * NV;
+            const int km = nk - k < MS ? nk - k : MS;
+#pragma unroll 1
+            for (int q = 0; q < km; ++q, m += R::TAB / sizeof(T), d += 32 * NV) {
+              T du[NV];
+#pragma unroll
+              for (int v = 0; v < NV; ++v) du[v] = d[v];
+#pragma unroll
+              for (int j = 0; j < DH; ++j)
+                if (d0 + j < nd) {
+                  const T r = m[j * 32];
+#pragma unroll
+                  for (int v = 0; v < NV; ++v) acc[j][v] += r * du[v];
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[slot]);
+            if (++slot == NSTG) slot = 0, ph ^= 1u;
+          }
+        if (ok && live)
+#pragma unroll
+          for (int j = 0; j < DH; ++j)
+            if (d0 + j < nd)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) Gi[(int64_t)((d0 + j) * NV + v) * 32] = act ? acc[j][v] : T(0);
+      }
     }
   }
-  if (!ok) {
-    if (lane == 0) atomicOr(p.health, HEALTH_TIMEOUT);
-    for (; t < issued; ++t) mbar_wait(&bar[t % NSTG], (unsigned)(t / NSTG) & 1u, LSQ_WAIT);
+  if (!ok && lane == 0) {
+    atomicOr(p.health, HEALTH_TIMEOUT);
+    *(volatile int*)&s_stop = 1;
   }
+  if (producer) {  // no copy may be in flight into a block that has ended
+    const int nout = issued < NSTG ? issued : NSTG;
+    for (int j = 0; j < nout; ++j) {
+      if (--slot < 0) slot = NSTG - 1, ph ^= 1u;
+      mbar_wait(&full[slot], ph, LSQ_WAIT);
+    }
+  }
+}
+
+template <int P, typename T>
+cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) {
+  using R = Ring<P, T>;
+  const cudaError_t e = cudaFuncSetAttribute(k_lsq_ring<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem);
+  if (e != cudaSuccess) return e;
+  const int64_t items = ((p.n + 31) / 32) * p.admis_max, nb = (items + 3) / 4;
+  const long wait = p.lsq_bulk && p.lsq_wait >= 0 ? p.lsq_wait : LSQ_WAIT;
+  k_lsq_ring<P, T><<<(unsigned)(nb < p.nsm * R::BPS ? nb : p.nsm * R::BPS), 256, R::smem, st>>>(p, U, items, wait);
+  return cudaGetLastError();
+}
+
+// the stencil polynomials of every cell into p.gbuf, from the state U
+template <int P, typename T>
+cudaError_t launch_lsq(const Problem& p, const double* U, cudaStream_t st, int64_t* launches) {
+  ++*launches;
+  return launch_lsq_ring<P, T>(p, U, st);
 }
 
 // ------------------------------------------------------------- k_wpost
@@ -1394,7 +1389,7 @@ extern template cudaError_t launch_wpost_char<4, double>(const Problem&, const d
 // One reconstruction: stencil polynomials, WENO post-processing and, for
 // Navier-Stokes, the viscous LSQ and face gradients.  Instantiated per
 // precision and order in recon_*.cu, which nvcc compiles in parallel.
-// `mark`, if not null, is recorded between k_lsq and k_wpost (kernel timing).
+// `mark`, if not null, is recorded after the least squares (kernel timing).
 template <int P, typename T>
 cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cudaStream_t st, int64_t* launches,
                           cudaEvent_t mark) {
@@ -1408,22 +1403,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     ++*launches;
     return cudaGetLastError();
   }
-  if (p.lsq_bulk) {  // opt-in: tables staged through shared memory (UCG_LSQ_BULK=1)
-    constexpr int NSTG = 4;
-    constexpr size_t smem = lsq_tma_smem<P, T, NSTG>();
-    cudaFuncSetAttribute(k_lsq_tma<P, T, NSTG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_lsq_tma<P, T, NSTG><<<b, 128, smem, st>>>(p, U);
-  } else if (P == 3) {
-    // padded records: 6.9 -> 4.7 ms per stage for CWENO4 at 2.1 M cells; on
-    // B200 the vector gather doubled k_lsq's time at IORDER 4 (255
-    // registers: it breaks the load schedule) and made IORDER 2 slower by a
-    // third, so those keep five 8-byte loads
-    k_pad_state<P, T><<<(unsigned)((pa.n + 255) / 256), 256, 0, st>>>(pa, U);
-    k_lsq<P, T, (P == 3)><<<b, 128, 0, st>>>(p, U);
-    ++*launches;
-  } else {
-    k_lsq<P, T><<<b, 128, 0, st>>>(p, U);
-  }
+  const cudaError_t el = launch_lsq<P, T>(p, U, st, launches);
+  if (el != cudaSuccess) return el;
   if (mark) cudaEventRecord(mark, st);
   if (p.wenwrt == 2) {
     const cudaError_t e = launch_wpost_char<P, T>(p, U, st);
@@ -1458,7 +1439,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     }
     if (!done) k_wpost<P, T><<<b, 128, 0, st>>>(p, U);
   }
-  *launches += 2;
+  ++*launches;
   if (ns) {
     k_visc_prim<P, T><<<(unsigned)((pa.n + 255) / 256), 256, 0, st>>>(pa, U);
     k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
@@ -1483,7 +1464,7 @@ cudaError_t launch_weno_f64_p4(const Problem& p, const double* U, bool ns, int Q
                                int64_t* launches, cudaEvent_t mark);
 // the stencil least squares alone (FP64 tables) into p.gbuf: G is linear in
 // U, so applied to a tangent dU it gives the tangent dG (adjoint.cu)
-cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st);
-cudaError_t launch_lsq_f64_p4(const Problem& p, const double* U, cudaStream_t st);
+cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st, int64_t* launches);
+cudaError_t launch_lsq_f64_p4(const Problem& p, const double* U, cudaStream_t st, int64_t* launches);
 
 }  // namespace ucg

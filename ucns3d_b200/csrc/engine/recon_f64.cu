@@ -15,16 +15,14 @@ cudaError_t launch_weno_f64(int iorder, const Problem& p, const double* U, bool 
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st) {
-  const unsigned b = (unsigned)((p.n + 127) / 128);
+cudaError_t launch_lsq_f64(int iorder, const Problem& p, const double* U, cudaStream_t st, int64_t* launches) {
   switch (iorder) {
-    case 1: k_lsq<1, double><<<b, 128, 0, st>>>(p, U); break;
-    case 2: k_lsq<2, double><<<b, 128, 0, st>>>(p, U); break;
-    case 3: k_lsq<3, double><<<b, 128, 0, st>>>(p, U); break;
-    case 4: return launch_lsq_f64_p4(p, U, st);
-    default: return cudaErrorInvalidValue;
+    case 1: return launch_lsq<1, double>(p, U, st, launches);
+    case 2: return launch_lsq<2, double>(p, U, st, launches);
+    case 3: return launch_lsq<3, double>(p, U, st, launches);
+    case 4: return launch_lsq_f64_p4(p, U, st, launches);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace ucg
