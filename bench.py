@@ -172,42 +172,69 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-# DRAM traffic of one k_lsq launch per cell, dram__bytes_read.sum +
-# dram__bytes_write.sum of a one-kernel ncu capture divided by the cells of
-# the captured mesh, keyed by (workload, precision).  Only measured entries
-# are listed; other workloads report traffic null.  The k_lsq traffic grows
-# in proportion to the cells (no re-reads between cells), so a launch on a
-# larger mesh of the same workload moves this times its cells.
-#   vortex_hex_weno5, mixed: 32^3 capture, 1.00x the algorithmic bytes
-LSQ_DRAM_BYTES_PER_CELL = {("vortex_hex_weno5", 1): 106_700}
+# DRAM traffic of one launch of the stencil least squares per cell,
+# dram__bytes_read.sum + dram__bytes_write.sum of a one-kernel ncu capture
+# divided by the cells of the captured mesh, keyed by (workload, precision).
+# Only measured entries are listed; other workloads report traffic null.  The
+# traffic grows in proportion to the cells, so a launch on a larger mesh of the
+# same workload moves this times its cells.
+#   vortex_hex_weno5, mixed: 32^3 capture of k_lsq_set (97.6 + 113.9 MB)
+LSQ_DRAM_BYTES_PER_CELL = {("vortex_hex_weno5", 1): 6_456}
 
 
-def lsq_bytes_per_cell(cfg):
-    """Algorithmic bytes of k_lsq per cell: the pseudo-inverse slices and
-    stencil indices of every stencil, the cell's own state, and the stencil
-    polynomials G written (neighbour states come through L2; they are
-    counted once, in the flux kernel)."""
+def lsq_bytes_per_cell(cfg, sets_per_cell=1.0):
+    """Algorithmic bytes of the stencil least squares per cell: the
+    pseudo-inverse slices (times the distinct matrix sets per cell) and stencil
+    indices of every stencil, the cell's own state, and the stencil polynomials
+    G written (neighbour states come through L2; they are counted once, in the
+    flux kernel)."""
     from ucns3d_b200 import _native as N
     s = 4 if cfg.precision == N.UCG_MIXED else 8
     b = 5 * 8
     for ll in range(cfg.admis_max):
         low = cfg.ees == 5 and ll > 0
         nk, nd = (cfg.imax2, cfg.ideg2) if low else (cfg.imax, cfg.ideg)
-        b += s * nk * nd + 4 * nk + s * nd * 5
+        b += s * nk * nd * sets_per_cell + 4 * nk + s * nd * 5
     return b
 
 
-def recon_bytes_per_cell(cfg):
+def lsq_flops_per_cell(cfg):
+    """Multiply-adds of the stencil least squares per cell, times two."""
+    return sum(10 * ((cfg.imax2 * cfg.ideg2) if cfg.ees == 5 and ll > 0 else cfg.imax * cfg.ideg)
+               for ll in range(cfg.admis_max))
+
+
+def lsq_roofline(cfg, mesh, ncells, ms, peak, peak_kind, sm_mhz):
+    """The least squares against what bounds it: DRAM where the cells have
+    their own matrices, the FP32 (FP64) multiply-adds where they share sets
+    (nominal peak: 148 SMs x 128 (64) lanes at the SM clock)."""
+    from ucns3d_b200 import _native as N
+    share = mesh.ntables / ncells
+    bpc = lsq_bytes_per_cell(cfg, share)
+    hbm = bpc * ncells / (ms / 1000.0) / 1e9
+    if share > 0.5 or cfg.scheme == 2 and cfg.iorder == 1:
+        return {"bound": "hbm", "achieved": hbm, "peak": peak, "unit": "GB/s", "frac": hbm / peak,
+                "peak_kind": peak_kind, "nominal_peak": NOMINAL_HBM_GBS, "frac_nominal": hbm / NOMINAL_HBM_GBS,
+                "bytes_per_cell": bpc}
+    lanes = 128 if cfg.precision == N.UCG_MIXED else 64
+    top = 148 * lanes * 2 * sm_mhz * 1e6 / 1e12
+    tf = lsq_flops_per_cell(cfg) * ncells / (ms / 1000.0) / 1e12
+    return {"bound": "fma", "achieved": tf, "peak": top, "unit": "TFLOP/s", "frac": tf / top, "peak_kind": "nominal",
+            "hbm_gbs": hbm, "bytes_per_cell": bpc, "distinct_matrix_sets": mesh.ntables}
+
+
+def recon_bytes_per_cell(cfg, sets_per_cell=1.0):
     """Algorithmic bytes the reconstruction kernel must move per cell: the
-    pseudo-inverses, stencil indices, smoothness matrix, face quadrature
-    points and basis means of the cell, its own state and its face values
-    written (neighbour state counted once, in the flux kernel)."""
+    pseudo-inverses and smoothness matrices (times the distinct matrix sets per
+    cell), stencil indices, face quadrature points and basis means of the cell,
+    its own state and its face values written (neighbour state counted once,
+    in the flux kernel)."""
     from ucns3d_b200 import _native as N
     s = 4 if cfg.precision == N.UCG_MIXED else 8
     nq = max(cfg.nq_quad, cfg.nq_tri)
-    b = s * cfg.ideg * cfg.imax * cfg.admis_max + 4 * (cfg.imax + 1) * cfg.admis_max
+    b = s * cfg.ideg * cfg.imax * cfg.admis_max * sets_per_cell + 4 * (cfg.imax + 1) * cfg.admis_max
     if cfg.scheme == 3:  # packed upper triangle of the smoothness matrix
-        b += s * cfg.ideg * (cfg.ideg + 1) // 2
+        b += s * cfg.ideg * (cfg.ideg + 1) // 2 * sets_per_cell
     b += s * 6 * nq * 3 + s * cfg.ideg + 5 * 8
     b += s * 6 * nq * 5  # face values written
     return b
@@ -218,8 +245,8 @@ def recon_kernels(cfg, wenwrt):
     if cfg.scheme == 2 and cfg.iorder == 1:
         return "k_muscl"
     if cfg.scheme == 3 and cfg.iorder == 4 and wenwrt == 1:
-        return "k_lsq + k_wis + k_wface + k_wpost fall-back"
-    return "k_lsq + k_wpost"
+        return "least squares + indicators + k_wface + k_wpost fall-back"
+    return "least squares + k_wpost"
 
 
 L2_BYTES = 126 * 2 ** 20
@@ -764,13 +791,14 @@ def main():
     value = ws * ncells * 3 * args.steps / (ms / 1000.0)
     e2e_s = max_over_ranks(r32["e2e"]["seconds"], ws, local)
     e2e_value = ws * ncells * 3 * args.steps / e2e_s
-    # roofline of the dominant kernel (k_lsq), achieved from its CUDA-event
+    # roofline of the stencil least squares, achieved from its CUDA-event
     # duration on the engine stream; the whole reconstruction beside it
-    bpc = lsq_bytes_per_cell(cfg32)
-    table_bytes = bpc * ncells
+    share = c32.mesh.ntables / ncells
+    table_bytes = lsq_bytes_per_cell(cfg32, share) * ncells  # tables, indices, polynomials: what a stage touches
     lsq_ms = r32["kern"]["lsq"]
-    achieved = bpc * ncells / (lsq_ms / 1000.0) / 1e9
-    rbpc = recon_bytes_per_cell(cfg32)
+    sm_mhz = (r32["clocks"] or {}).get("sm_mhz") or 1965.0
+    roof = lsq_roofline(cfg32, c32.mesh, ncells, lsq_ms, peak, peak_kind, sm_mhz)
+    rbpc = recon_bytes_per_cell(cfg32, share)
     per_cell = LSQ_DRAM_BYTES_PER_CELL.get((args.case, int(cfg32.precision)))
     traffic = per_cell * ncells if per_cell is not None and args.wenwrt == 1 else None
     out = {
@@ -781,13 +809,10 @@ def main():
         "config": {"workload": args.case, "cells": ncells, "n": args.n,
                    "scheme": scheme_label(c32, args.wenwrt),
                    "parallelism": f"replicas x{ws}",
-                   "l2": ("inputs larger than L2 (tables)" if table_bytes > L2_BYTES
-                          else "tables smaller than L2: not an HBM-roofline case")},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "nominal_peak": NOMINAL_HBM_GBS, "frac_nominal": achieved / NOMINAL_HBM_GBS,
-                     "traffic": traffic, "traffic_unit": "bytes per launch",
-                     "kernel": "k_lsq (stencil least squares)",
-                     "bytes_per_cell": bpc, "kernel_ms": lsq_ms,
+                   "l2": ("inputs larger than L2 (stencils, tables, polynomials)" if table_bytes > L2_BYTES
+                          else "inputs smaller than L2: not an HBM-roofline case")},
+        "roofline": {**roof, "traffic": traffic, "traffic_unit": "bytes per launch",
+                     "kernel": "stencil least squares", "kernel_ms": lsq_ms,
                      "reconstruction": {"kernels": recon_kernels(cfg32, args.wenwrt), "bytes_per_cell": rbpc,
                                         "ms": r32["kern"]["recon"],
                                         "frac": rbpc * ncells / (r32["kern"]["recon"] / 1000.0) / 1e9 / peak}},
@@ -809,9 +834,9 @@ def main():
         ra, rb = r64["state"][:, 0], r32["state"][:, 0]
         l2 = float(np.sqrt(np.mean((ra - rb) ** 2)) / np.sqrt(np.mean(ra ** 2)))
         linf = float(np.abs(ra - rb).max() / np.abs(ra).max())
-        bpc64 = lsq_bytes_per_cell(cfg64)
+        roof64 = lsq_roofline(cfg64, c32.mesh, ncells, r64["kern"]["lsq"], peak, peak_kind, sm_mhz)
         out["fp64"] = {"value": v64, "ms_per_step": ms64 / args.steps, "kernel_ms": r64["kern"],
-                       "roofline_frac": bpc64 * ncells / (r64["kern"]["lsq"] / 1000.0) / 1e9 / peak,
+                       "roofline_frac": roof64["frac"], "roofline_bound": roof64["bound"],
                        "mixed_speedup": value / v64,
                        "density_rel_l2_mixed_vs_fp64": l2, "density_rel_linf_mixed_vs_fp64": linf,
                        "after_steps": args.warmup + args.steps}

@@ -277,8 +277,8 @@ int ucg_time_kernels(ucg_engine* e, int32_t reps, double* ms);
 /* Bounded device waits.  The stencil least squares passes its tables and
  * gathered states through rings in shared memory, whose waits give up after
  * 65,536 polls (about 300 ns each, about 20 ms in all).  An engine created
- * with UCG_LSQ_BULK=1 in the environment takes `polls` as its bound instead
- * (the default is
+ * with UCG_LSQ_BULK=1 in the environment reads every cell's own tables (no
+ * shared matrix sets) and takes `polls` as its bound instead (the default is
  * restored by polls < 0).  A wait that gives up makes its block finish the
  * copies it has in flight (each with the default bound) and return, and the
  * next ucg_check_health reports UCG_ETIMEOUT; the handle stays usable.

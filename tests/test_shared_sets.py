@@ -1,0 +1,75 @@
+"""Matrix sets shared by many cells (k_lsq_set, k_lsq_low, k_wis_set):
+the same engine once with the tables of one upload, whose shared sets are
+tiled, and once with the same tables uploaded in two halves, where every cell
+reads its own copy.  The forward kernels take the same operations in the same
+order, so residuals and states are equal bit for bit.
+
+Meshes: whole tiles and remainders (1 to 127 cells in a set's last tile), sets
+above and below the 32 cells from which they are tiled, all cells tiled and
+some left over (a box without periodicity), CWENO with both stencil sizes,
+renumbered cells, Navier-Stokes."""
+import numpy as np
+import pytest
+
+from ucns3d_b200 import _native as N
+from ucns3d_b200.config import EULER, NAVIER_STOKES, make_config
+from ucns3d_b200.engine import Engine
+from ucns3d_b200.mesh import IC_TGV, SCHEME_MUSCL, SCHEME_WENO, Mesh, RenumberedMesh
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "weno5_hex12": (lambda: Mesh.box_hex(12, 12, 12), SCHEME_WENO, 4, 0, EULER, 1),
+    "weno5_hex_open": (lambda: Mesh.box_hex(10, 10, 24, periodic=(1, 1, 0), bc=(0, 0, 0, 0, 6, 6)), SCHEME_WENO, 4, 0,
+                       EULER, 1),
+    "weno5_hex_char": (lambda: Mesh.box_hex(11, 10, 10), SCHEME_WENO, 4, 0, EULER, 2),
+    "weno3_ns_hex9": (lambda: Mesh.box_hex(9, 9, 9), SCHEME_WENO, 2, 0, NAVIER_STOKES, 1),
+    "weno3_tet": (lambda: Mesh.box_tet(10, 10, 10, jitter=0.0), SCHEME_WENO, 2, 0, EULER, 1),
+    "cweno4_ns_mixed10": (lambda: Mesh.mixed_box(10, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES, 1),
+    "cweno4_mixed16": (lambda: Mesh.mixed_box(16, seed=4), SCHEME_WENO, 3, 5, EULER, 1),
+    "muscl_p2_hex8": (lambda: Mesh.box_hex(8, 8, 8), SCHEME_MUSCL, 2, 0, EULER, 1),
+}
+
+
+def _engines(name, precision, shuffle=False):
+    mk, scheme, iorder, ees, gov, wenwrt = CASES[name]
+    m = mk().prepare(scheme, iorder, ees)
+    if shuffle:
+        m = RenumberedMesh(m, np.random.default_rng(5).permutation(m.ncells))
+    cfg = make_config(m, governing=gov, precision=precision, reynolds=200.0, pres=5.0, prandtl=0.71, wenwrt=wenwrt)
+    shared = Engine(m, cfg)
+    own = Engine(m, cfg, upload=False)
+    own.upload_geometry(m.geometry_struct())
+    r, s, n = m.recon_struct(), m.sizes, m.ncells
+    row = s["admis_max"] * (s["imax"] + 1)
+    st = np.ctypeslib.as_array(r.stencil, shape=(n * row,))
+    tid = np.ctypeslib.as_array(r.table_id, shape=(n,))
+    half = n // 2
+    for a, b in ((0, half), (half, n)):
+        part = N.UcgRecon.from_buffer_copy(r)
+        part.first, part.count = a, b - a
+        part.stencil = N.ptr(st[a * row:b * row], N.C.c_int32)
+        part.table_id = N.ptr(tid[a:b], N.C.c_int32)
+        own.upload_recon(part)
+    x = m.centres()
+    U = m.initial_condition(IC_TGV, [1.4, 5.0, 1.0])
+    U = U * (1.0 + 0.02 * np.sin(1.3 * x[:, :1] + 0.7 * x[:, 1:2] + 2.1 * x[:, 2:3] + np.arange(5.0)))
+    return m, shared, own, U
+
+
+@pytest.mark.parametrize("precision", [N.UCG_FP64, N.UCG_MIXED])
+@pytest.mark.parametrize("name", list(CASES))
+def test_shared_sets_equal_own_tables(name, precision):
+    m, shared, own, U = _engines(name, precision, shuffle=name in ("weno5_hex12", "cweno4_ns_mixed10"))
+    assert shared.device_bytes != own.device_bytes  # the shared engine holds its tiles
+    out = []
+    for e in (shared, own):
+        e.set_state(U)
+        R = e.residual()
+        e.time_marching(2, 0.4)
+        out.append((R, e.get_state(), e.last_dt()))
+        e.check_health()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
+    assert out[0][2] == out[1][2]
+    assert np.abs(out[0][0]).max() > 0

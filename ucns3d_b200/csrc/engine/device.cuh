@@ -63,6 +63,18 @@ struct Problem {
   const void* ind;
   int64_t istride;
   int i2off;
+  // matrix sets shared by many cells (see k_lsq_set): the tiled cells in tiles
+  // of SET_TILE that share a set, and each set's pseudo-inverses once
+  const int32_t* tcell;     // [ntile][SET_TILE] cells, -1 = none (never the first of a tile)
+  const int32_t* tset;      // [ntile] set
+  int64_t ntile;            // 0: every cell reads its own tables
+  const int8_t* tiled;      // [n] the cell is in a tile; nullptr: every cell is (or none)
+  const void* setmat;       // [nset][sstride], stencil ll at sso[ll]: rows [nk][set_stride(nd)]
+  int64_t sstride;
+  int sso[8];
+  const void* setind;       // [nset][istride] the sets' packed smoothness triangles (WENO)
+  const int32_t* ugrp;      // [nugrp] 32-cell groups with cells that are not tiled (k_lsq_ring)
+  int64_t nugrp;
   // scratch
   void* gbuf;               // stencil polynomials G[ll][d][v], interleaved like the stencils
   double* qbuf;             // characteristic WENO: G_l^T S G_l per stencil, 15 values, interleaved
@@ -88,8 +100,8 @@ struct Problem {
   double* fflux;            // [n][MF][NV] convective face sums (owner and negated copy)
   double* vflux;            // [n][MF][NV] viscous face sums
   unsigned* health;
-  bool lsq_bulk; // lsq_wait is the bound of the least squares' waits
-  long lsq_wait; // polls of a stage wait before it gives up (< 0: the default)
+  bool lsq_bulk; // every cell's least squares through k_lsq_ring
+  long lsq_wait; // with it: polls of a stage wait before it gives up (< 0: the default)
   int nsm;       // SMs of the device
   int wenwrt;    // 1 conserved-variable WENO, 2 characteristic-variable WENO
   int riemann;   // 1 HLLC, 2 Rusanov, 3 Roe, 4 rotated Roe-HLL, 5 t-Roe, 9 HLL
@@ -129,6 +141,14 @@ __device__ __forceinline__ void ldv(const double* p, double (&o)[2]) {
   const double2 x = *(const double2*)p;
   o[0] = x.x;
   o[1] = x.y;
+}
+
+// cells of a tile of k_lsq_set, and the row stride of a shared matrix (whole
+// 16-byte vectors)
+constexpr int SET_TILE = 128;
+template <typename T>
+__host__ __device__ constexpr int set_stride(int nd) {
+  return (nd + Vec<T>::N - 1) / Vec<T>::N * Vec<T>::N;
 }
 
 template <int P>

@@ -127,6 +127,16 @@ Problem make_problem(ucg_engine* e) {
   for (int k = 0; k < 8; ++k) {
     p.soff[k] = e->layout.soff[k];
   }
+  p.ntile = e->ntile;
+  p.tcell = (const int32_t*)e->tcell.p;
+  p.tset = (const int32_t*)e->tset.p;
+  p.tiled = e->all_tiled ? nullptr : (const int8_t*)e->tiled.p;
+  p.setmat = e->setmat.p;
+  p.sstride = e->sstride;
+  for (int k = 0; k < 8; ++k) p.sso[k] = e->sso[k];
+  p.setind = e->setind.p;
+  p.ugrp = (const int32_t*)e->ugrp.p;
+  p.nugrp = e->nugrp;
   p.gbuf = e->gbuf.p;
   p.qbuf = (double*)e->qbuf.p;
   p.isb = (double*)e->isb.p;
@@ -624,6 +634,8 @@ void ucg_destroy(ucg_engine* e) {
                    &e->health, &e->dt, &e->partial, &e->red, &e->staging, &e->own, &e->fflux, &e->vflux, &e->gbuf,
                    &e->qbuf, &e->d_n2o, &e->permbuf, &e->fgrad, &e->isb, &e->wflag, &e->mprev, &e->mflag,
                    &e->msel, &e->mmus, &e->mord, &e->Um, &e->imp_dtl, &e->imp_dinv, &e->imp_off, &e->imp_du,
+                   &e->tcell, &e->tset, &e->tiled, &e->setmat, &e->setind,
+                   &e->ugrp,
                    &e->dual_hist, &e->dual_part, &e->halo_send, &e->halo_recv, &e->wl_buf};
   for (DevBuf* b : all) release(*b);
   adjoint_release(e);
@@ -787,6 +799,7 @@ int ucg_upload_geometry(ucg_engine* e, const ucg_geometry* g) {
     rc = rc ? rc : alloc(e, e->permbuf, (size_t)n * NV * 8);
   }
   if (rc) return rc;
+  e->ntile = 0;  // the tiles follow the cell order; ucg_upload_recon makes them
   // reference-frame quadrature points and basis means, in table precision
   // interleaved over 32-cell groups: element j of cell c at ((c/32)*len + j)*32 + c%32
   const int64_t ngrp = (n + 31) / 32, lq = (int64_t)MF * QS * 3;
@@ -897,6 +910,85 @@ int ucg_host::upload_stencils(ucg_engine* e, int64_t first, int64_t count, const
   return UCG_OK;
 }
 
+namespace {
+
+// Which cells k_lsq_set reconstructs: the cells of a matrix set that at least
+// SET_MIN cells share (a quarter of a tile: below that a tile costs more than
+// the group of 32 that k_lsq_ring would read), cut into tiles of SET_TILE in
+// device order.  set_of gets each table's set, -1 where its cells read their
+// own tables.  Kept only where it pays: a tile is taken to cost three fifths of
+// what its 128 cells cost k_lsq_ring, which costs the same for a group of 32
+// cells whether one or all of them are left to it.  Measured, all cells tiled
+// against all through the ring: WENO5 64^3 mixed 2.13 / 4.81 ms, 40^3 FP64
+// 1.21 / 2.11, 12^3 FP64 0.058 / 0.090; WENO3 48^3 0.193 / 0.298 (mixed), 0.290
+// / 0.340 (FP64); CWENO4 271,872 cells mixed 0.438 / 0.482, 75,776 FP64 0.236 /
+// 0.234.
+constexpr int64_t SET_MIN = 32;
+int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<int32_t>& set_of, int64_t* tiles) {
+  const ucg_config& c = e->cfg;
+  const int64_t n = e->n_recon;
+  const bool perm = !e->n2o.empty();
+  auto table = [&](int64_t cell) { return table_id[perm ? e->n2o[cell] : cell]; };
+  std::vector<int64_t> cells(ntab, 0);
+  for (int64_t i = 0; i < n; ++i) cells[table(i)]++;
+  set_of.assign(ntab, -1);
+  std::vector<int64_t> at;  // first tile slot of each set
+  int64_t nset = 0, ntile = 0;
+  for (int64_t t = 0; t < ntab; ++t)
+    if (cells[t] >= SET_MIN) {
+      set_of[t] = (int32_t)nset++;
+      at.push_back(ntile * SET_TILE);
+      ntile += (cells[t] + SET_TILE - 1) / SET_TILE;
+    }
+  std::vector<int32_t> ugrp;  // groups with cells of their own tables
+  for (int64_t g = 0; g < n; g += 32)
+    for (int64_t i = g; i < n && i < g + 32; ++i)
+      if (set_of[table(i)] < 0) {
+        ugrp.push_back((int32_t)(g >> 5));
+        break;
+      }
+  if (!ntile || ntile >= (1 << 30) || 5 * (int64_t)ugrp.size() * 32 + 3 * ntile * SET_TILE > 5 * n) {
+    set_of.clear();
+    return UCG_OK;
+  }
+  std::vector<int32_t> tcell((size_t)ntile * SET_TILE, -1), tset((size_t)ntile);
+  std::vector<int8_t> tiled((size_t)e->n, 0);
+  e->all_tiled = true;
+  for (int64_t i = 0; i < n; ++i) {
+    const int32_t s = set_of[table(i)];
+    if (s < 0) {
+      e->all_tiled = false;
+      continue;
+    }
+    tset[(size_t)(at[s] / SET_TILE)] = s;
+    tcell[(size_t)at[s]++] = (int32_t)i;
+    tiled[(size_t)i] = 1;
+  }
+  const int64_t vec = e->mixed ? 4 : 2;
+  int64_t off = 0;
+  for (int ll = 0; ll < c.admis_max; ++ll) {
+    const bool low = c.ees == 5 && ll > 0;
+    e->sso[ll] = (int)off;
+    off += (int64_t)(low ? c.imax2 : c.imax) * (((low ? c.ideg2 : c.ideg) + vec - 1) / vec * vec);
+  }
+  e->sstride = off;
+  e->nset = nset;
+  int rc = UCG_OK;
+  rc = rc ? rc : upload(e, e->tcell, tcell);
+  rc = rc ? rc : upload(e, e->tset, tset);
+  rc = rc ? rc : upload(e, e->tiled, tiled);
+  rc = rc ? rc : alloc(e, e->setmat, (size_t)nset * e->sstride * tsize(e));
+  if (c.scheme == 3) rc = rc ? rc : alloc(e, e->setind, (size_t)nset * e->layout.istride * tsize(e));
+  rc = rc ? rc : upload(e, e->ugrp, ugrp);
+  e->nugrp = (int64_t)ugrp.size();
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(e->stream));
+  *tiles = ntile;
+  return UCG_OK;
+}
+
+}  // namespace
+
 // The matrix sets of tables [0, ntab) into the engine's interleaved tables
 // for cells [first, first + count): `fill(which, t0, t1, staging)` writes
 // the FP64 blocks of tables [t0, t1) into the device staging buffer, the
@@ -905,11 +997,45 @@ int ucg_host::upload_stencils(ucg_engine* e, int64_t first, int64_t count, const
 // each); they are expanded per cell (d_tid: cell -> table, NULL = the
 // cell's own row), pseudo-inverses element by element, smoothness matrices
 // by 16-byte vectors, in 512 MiB chunks.
-int ucg_host::expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t ntab, const int32_t* d_tid,
-                            const int32_t* d_rowmap, const std::function<int(int, int64_t, int64_t, double*)>& fill) {
+int ucg_host::expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t ntab, const int32_t* table_id,
+                            const int32_t* d_tid, const int32_t* d_rowmap, const std::function<int(int, int64_t, int64_t, double*)>& fill) {
   const Layout& Ly = e->layout;
   const int64_t n = e->n;
   const bool perm = !e->o2n.empty();
+  // shared sets, where one call gives every cell's (with chunked uploads the
+  // table numbers of one call say nothing about another's)
+  e->ntile = 0;
+  std::vector<int32_t> set_of;
+  int64_t ntile = 0;
+  struct Tmp {
+    ucg_engine* e;
+    DevBuf b;
+    ~Tmp() {
+      e->bytes -= (int64_t)b.bytes;
+      release(b);
+    }
+  } d_set{e, {}};
+  SetLayout SL{};
+  if (table_id && first == 0 && count == n && !(e->cfg.scheme == 2 && e->cfg.iorder == 1) && !e->lsq_bulk) {
+    int rc = plan_sets(e, table_id, ntab, set_of, &ntile);
+    if (rc) return rc;
+    if (ntile) {
+      const ucg_config& c = e->cfg;
+      const int vec = e->mixed ? 4 : 2;
+      SL.tstride = Ly.tstride;
+      SL.sstride = e->sstride;
+      SL.nst = c.admis_max;
+      for (int ll = 0; ll < c.admis_max; ++ll) {
+        const bool low = c.ees == 5 && ll > 0;
+        SL.soff[ll] = Ly.soff[ll];
+        SL.sso[ll] = e->sso[ll];
+        SL.nk[ll] = low ? c.imax2 : c.imax;
+        SL.nd[ll] = low ? c.ideg2 : c.ideg;
+        SL.stride[ll] = (SL.nd[ll] + vec - 1) / vec * vec;
+      }
+      if ((rc = upload(e, d_set.b, set_of))) return rc;
+    }
+  }
   struct Part {
     int64_t len;
     DevBuf* dst;
@@ -930,6 +1056,23 @@ int ucg_host::expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t
       int64_t total = (perm ? n : count) * pt.len;
       unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 64);
       const double* sp = (const double*)e->staging.p;
+      if (pt.which == 0 && ntile) {
+        const int32_t* so = (const int32_t*)d_set.b.p;
+        if (e->mixed) k_pack_sets<float><<<(unsigned)(t1 - t0), 256, 0, e->stream>>>((float*)e->setmat.p, sp, so, t0, SL);
+        else k_pack_sets<double><<<(unsigned)(t1 - t0), 256, 0, e->stream>>>((double*)e->setmat.p, sp, so, t0, SL);
+        e->launches++;
+      }
+      if (pt.which == 1 && ntile) {  // the packed triangles as they are
+        SetLayout I{};
+        I.tstride = I.sstride = pt.len;
+        I.nst = 1;
+        I.nk[0] = 1;
+        I.nd[0] = I.stride[0] = (int)pt.len;
+        const int32_t* so = (const int32_t*)d_set.b.p;
+        if (e->mixed) k_pack_sets<float><<<(unsigned)(t1 - t0), 256, 0, e->stream>>>((float*)e->setind.p, sp, so, t0, I);
+        else k_pack_sets<double><<<(unsigned)(t1 - t0), 256, 0, e->stream>>>((double*)e->setind.p, sp, so, t0, I);
+        e->launches++;
+      }
       if (e->mixed) {
         if (pt.which == 0)
           k_expand_il<float, double, 1><<<blocks, 256, 0, e->stream>>>((float*)pt.dst->p, sp, d_tid, first, count, pt.len, t0, t1, d_rowmap, n);
@@ -949,6 +1092,7 @@ int ucg_host::expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t
   e->bytes -= (int64_t)e->staging.bytes;
   release(e->staging);
   CK(cudaStreamSynchronize(e->stream));
+  e->ntile = ntile;
   return UCG_OK;
 }
 
@@ -1028,7 +1172,7 @@ int ucg_upload_recon(ucg_engine* e, const ucg_recon* r) {
     if (cw) pack_tri(r->indicator2 + t * ideg2 * ideg2, ideg2, dst + Ly.i2off);
   };
   std::vector<double> host;
-  rc = expand_tables(e, first, count, ntab, d_tid, d_rowmap, [&](int which, int64_t t0, int64_t t1, double* dev) {
+  rc = expand_tables(e, first, count, ntab, r->table_id, d_tid, d_rowmap, [&](int which, int64_t t0, int64_t t1, double* dev) {
     const int64_t len = which == 0 ? Ly.tstride : Ly.istride;
     host.resize((size_t)(t1 - t0) * len);
     for (int64_t t = t0; t < t1; ++t) {

@@ -53,6 +53,12 @@ struct ucg_engine {
   DevBuf nfaces, ftype, neigh, nface, bc, qperm, rot, area, dih, vol, minedge, jinv, admis, full, qpts, bmean;
   // tables
   DevBuf sten, invmat, ind;
+  // matrix sets shared by many cells (plan_sets): tiles of cells, each set's
+  // matrices once, the groups with cells that are not tiled
+  DevBuf tcell, tset, tiled, setmat, setind, ugrp;
+  int64_t ntile = 0, nset = 0, sstride = 0, nugrp = 0;
+  int sso[8] = {0};
+  bool all_tiled = false;
   // scratch and state
   DevBuf gbuf, isb, wflag, dul, ulv, fgrad, gv, prim, rhs, Un, Ua, Ub, health, dt, partial, red, staging, own, fflux, vflux, qbuf;
   // MOOD (cfg.mood): RECALC, the cascade's flags and selections, MOOD_O, the candidate state
@@ -66,7 +72,7 @@ struct ucg_engine {
   int64_t nown = 0;
   int64_t nown_plain = 0;  // owned faces [0, nown_plain): interior and mirror; the rest other boundaries
   cudaEvent_t mark = nullptr;  // recorded after the least squares while ucg_time_kernels runs
-  bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: ucg_set_wait_limit sets the least squares' bound
+  bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: no shared sets, every cell through k_lsq_ring
   int nsm = 148;
   bool wface = false;          // IORDER 4 conserved WENO: face values one warp per variable (k_wface)
   long lsq_wait = -1;          // polls of a k_lsq_ring stage wait (ucg_set_wait_limit; < 0 the default)
@@ -128,8 +134,8 @@ int cells_out(ucg_engine* e, double* host_dst, const double* dev_src);
 // the staging buffer itself
 int upload_stencils(ucg_engine* e, int64_t first, int64_t count, const int32_t* stencil, DevBuf& rowbuf,
                     const int32_t** d_rowmap);
-int expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t ntab, const int32_t* d_tid,
-                  const int32_t* d_rowmap, const std::function<int(int, int64_t, int64_t, double*)>& fill);
+int expand_tables(ucg_engine* e, int64_t first, int64_t count, int64_t ntab, const int32_t* table_id,
+                  const int32_t* d_tid, const int32_t* d_rowmap, const std::function<int(int, int64_t, int64_t, double*)>& fill);
 void mark_recon(ucg_engine* e, int64_t first, int64_t count);
 // frees the adjoint buffers (adjoint.cu)
 void adjoint_release(ucg_engine* e);

@@ -54,4 +54,25 @@ __global__ void __launch_bounds__(256) k_expand_il(D* __restrict__ dst, const S*
   }
 }
 
+// The pseudo-inverses of the shared sets, each once: table tlo + blockIdx.x
+// of the staging buffer into set set_of[table] (-1: none) of k_lsq_set's
+// layout, rows padded with zeros to `stride` elements.
+struct SetLayout {
+  int64_t tstride, sstride;
+  int nst, soff[8], sso[8], nk[8], nd[8], stride[8];
+};
+template <typename D>
+__global__ void __launch_bounds__(256) k_pack_sets(D* __restrict__ dst, const double* __restrict__ src,
+                                                   const int32_t* __restrict__ set_of, int64_t tlo, SetLayout L) {
+  const int32_t set = set_of[tlo + blockIdx.x];
+  if (set < 0) return;
+  src += blockIdx.x * L.tstride;
+  dst += set * L.sstride;
+  for (int ll = 0; ll < L.nst; ++ll)
+    for (int i = threadIdx.x; i < L.nk[ll] * L.stride[ll]; i += blockDim.x) {
+      const int k = i / L.stride[ll], d = i - k * L.stride[ll];
+      dst[L.sso[ll] + i] = d < L.nd[ll] ? D(src[L.soff[ll] + k * L.nd[ll] + d]) : D(0);
+    }
+}
+
 }  // namespace ucg

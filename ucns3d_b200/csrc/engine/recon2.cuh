@@ -1,12 +1,14 @@
 // Reconstruction for WENO / CWENO / high-order MUSCL.
 //
 // LEAST_SQUARES (src/gradients.f90:253-497), stencil polynomials G[ll][d][v]:
-//   k_lsq_ring  the cells' tables, streamed from DRAM through shared memory
-//               (interleaved over groups of 32 cells)
+//   k_lsq_ring  cells that read their own tables, streamed from DRAM through
+//               shared memory (interleaved over groups of 32 cells)
+//   k_lsq_set   cells that share a matrix set, tiled (and k_lsq_low, the
+//               CWENO directional stencils of those cells)
 // CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL, MUSCL
 // fall-back, CHECKSOLX (3126-3406): k_wpost, one lane per cell, no block
 // barriers, smoothness indicators as packed quadratic forms; at IORDER 4
-// k_wis and k_wface; characteristic variables k_char_forms and
+// k_wis / k_wis_set and k_wface; characteristic variables k_char_forms and
 // k_char_face.
 #pragma once
 
@@ -60,10 +62,338 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity, long l
   return __all_sync(0xffffffffu, ok);
 }
 
+template <int N>
+struct IntC {
+  static constexpr int value = N;
+};
+
+// acc[row] += r[row] du of one 16-byte vector of rows.  FP32 in packed pairs
+// of rows (FFMA2: two IEEE multiply-adds, the same values): one scalar FFMA a
+// cycle is half of the FP32 rate.
+template <typename T>
+struct RowAcc;
+template <>
+struct RowAcc<float> {
+  float2 a[2][NV];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) a[h][v] = make_float2(0.0f, 0.0f);
+  }
+  __device__ __forceinline__ void add(const float* m, const float (&du)[NV]) {
+    const float4 r = *(const float4*)m;
+    const float2 r0 = make_float2(r.x, r.y), r1 = make_float2(r.z, r.w);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a[0][v] = __ffma2_rn(r0, make_float2(du[v], du[v]), a[0][v]);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a[1][v] = __ffma2_rn(r1, make_float2(du[v], du[v]), a[1][v]);
+  }
+  __device__ __forceinline__ float get(int i, int v) const { return i & 1 ? a[i >> 1][v].y : a[i >> 1][v].x; }
+};
+template <>
+struct RowAcc<double> {
+  double a[2][NV];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) a[h][v] = 0.0;
+  }
+  __device__ __forceinline__ void add(const double* m, const double (&du)[NV]) {
+    const double2 r = *(const double2*)m;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a[0][v] += r.x * du[v];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a[1][v] += r.y * du[v];
+  }
+  __device__ __forceinline__ double get(int i, int v) const { return a[i][v]; }
+};
+
+// LEAST_SQUARES of the cells that share a matrix set (table_id of ucg_recon:
+// cells of the same local geometry).  Streaming every cell's own copy of the
+// pseudo-inverses from DRAM (100 KB a cell for WENO5 in FP32) bounds
+// k_lsq_ring; here a block takes 64 cells of one set and one stencil, keeps
+// the stencil's rows in shared memory and reads them as 16-byte broadcasts,
+// each row feeding five multiply-adds of a cell, so the kernel is bound by the
+// multiply-adds.  Per 32 cells NPR producer warps take turns to gather the
+// differences of MS members (all in flight, their indices loaded a turn ahead)
+// into a ring of NSTG stages, and NSL consumer warps multiply, each a slice of
+// the rows: with all 34 rows in one warp (170 accumulators) a scheduler has
+// one warp to run, whose shared-memory latencies nothing hides (64^3 WENO5,
+// mixed: 3.95 ms; and 4.36 ms with the gathers in the same warp).  The members
+// are added in their order per row and variable, so that G does not depend on
+// the kernel that forms it, bit for bit.
+// One lane per cell reading its own tables took 5.48 ms (64^3 WENO5, mixed),
+// 1.43 ms (27,000 cells, FP64) and 0.97 ms (271,872-cell CWENO4, mixed); this
+// kernel 2.13, 0.51 and, with k_lsq_low and the 48 groups left to k_lsq_ring,
+// 0.43.  Its shared-memory loads (34 words a row of five multiply-adds, 70
+// cycles a member and 32 cells in FP32) stand before the multiply-adds (43).
+template <typename T, int ND>
+struct SetRing {
+  static constexpr int VEC = Vec<T>::N, NVEC = (ND + VEC - 1) / VEC;  // vectors of rows
+  static constexpr int NSL = (NVEC + (VEC == 4 ? 2 : 4)) / (VEC == 4 ? 3 : 5);
+  static constexpr int MAXV = (NVEC + NSL - 1) / NSL;  // of a slice
+  // producers of 32 cells: two keep up with three or more slices (64,000 cells,
+  // WENO5 mixed: 0.711 ms with one, 0.534 with two; 27,000, FP64: 0.533, 0.506)
+  // and with two in FP32 (271,872 cells, CWENO4: 0.494, 0.436); elsewhere the
+  // second only takes registers (32,768-cell CWENO4 FP64: 0.236, 0.253)
+  static constexpr int NPR = NSL > (VEC == 4 ? 1 : 2) ? 2 : 1;
+  static constexpr int WARPS = 2 * (NSL + NPR);
+  static constexpr int MS = 4, NSTG = 4;  // members of a stage, stages (a multiple of NPR)
+  static constexpr int elems = MS * 32 * NV;  // of a stage
+};
+template <int P, typename T, int ND>
+__global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS) k_lsq_set(Problem p, const double* __restrict__ U) {
+  constexpr int ID = Deg<P>::ideg;
+  constexpr int RS = set_stride<T>(ND);
+  using R = SetRing<T, ND>;
+  constexpr int VEC = R::VEC, MS = R::MS, NSTG = R::NSTG;
+  constexpr int TH = 32 * R::WARPS;
+  extern __shared__ __align__(16) unsigned char ls_smem[];
+  __shared__ __align__(8) uint64_t s_full[2][NSTG], s_empty[2][NSTG];
+  __shared__ int s_stop;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = warp & 1, role = warp >> 1;
+  const int64_t tile = blockIdx.x >> 1;
+  const int ll = blockIdx.y;
+  const int nk = p.imax, A = p.admis_max, W = p.imax + 1;
+  const int32_t* tc = p.tcell + tile * SET_TILE + (blockIdx.x & 1) * 64;
+  if (tc[0] < 0) return;  // the tile's second half may hold no cell
+  T* s = (T*)ls_smem;
+  T* ring = s + nk * RS + half * NSTG * R::elems;
+  uint64_t *full = s_full[half], *empty = s_empty[half];
+  if (threadIdx.x == 0) {
+    s_stop = 0;
+    for (int w = 0; w < 2; ++w)
+      for (int i = 0; i < NSTG; ++i) {
+        mbar_init(&s_full[w][i], 1);
+        mbar_init(&s_empty[w][i], R::NSL);
+      }
+    mbar_fence_init();
+  }
+  {
+    const float4* src = (const float4*)((const T*)p.setmat + p.tset[tile] * p.sstride + p.sso[ll]);
+    for (int i = threadIdx.x; i < nk * RS / VEC; i += TH) ((float4*)s)[i] = src[i];
+  }
+  const int mine = tc[half * 32 + lane];
+  const bool live = mine >= 0;
+  const int c = live ? mine : tc[0];
+  const bool act = live && ll < p.admis[c];
+  const bool any = __any_sync(0xffffffffu, act);
+  __syncthreads();
+  int slot = 0;
+  unsigned ph = 0;  // phase of the ring's current round
+  bool ok = true;
+  if (role >= R::NSL) {
+    slot = role - R::NSL;  // this producer's first stage
+    if (any) {
+      const GatherShare sh(lane);
+      const int32_t* S = p.sten + (int64_t)(c >> 5) * (A * W) * 32 + (c & 31) + (ll * W + 1) * 32;
+      auto member = [&](int k) -> int { return act ? S[(k < nk ? k : nk - 1) * 32] : c; };
+      double u0[NV];
+      sh.load(U, c, u0);
+      int y[MS];
+#pragma unroll
+      for (int j = 0; j < MS; ++j) y[j] = member(slot * MS + j);
+      for (int k = slot * MS; k < nk; k += R::NPR * MS) {
+        double u[MS][NV];
+#pragma unroll
+        for (int j = 0; j < MS; ++j) sh.load(U, y[j], u[j]);
+#pragma unroll
+        for (int j = 0; j < MS; ++j) y[j] = member(k + R::NPR * MS + j);
+        if (!(ok = ring_wait(&empty[slot], ph ^ 1u, LSQ_WAIT, &s_stop))) break;  // the first round finds them empty
+        T* du = ring + slot * R::elems + lane;
+#pragma unroll
+        for (int j = 0; j < MS; ++j)
+#pragma unroll
+          for (int i = 0; i < NV; ++i) du[(j * NV + i) * 32] = T(u[j][i] - u0[i]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[slot]);
+        if ((slot += R::NPR) >= NSTG) slot -= NSTG, ph ^= 1u;
+      }
+    }
+  } else {
+    // this warp's vectors of rows [q0, q0 + NQ), NQ = MAXV or one less
+    const int q0 = role * R::NVEC / R::NSL, nq = (role + 1) * R::NVEC / R::NSL - q0;
+    auto multiply = [&](auto nqc) {
+      constexpr int NQ = decltype(nqc)::value;
+      RowAcc<T> acc[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) acc[q].zero();
+      auto add = [&](const T* m, const T* d) {
+        T du[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) du[v] = d[v];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) acc[q].add(m + q * VEC, du);
+      };
+      if (any)
+        for (int k = 0; k < nk; k += MS) {
+          if (!(ok = ring_wait(&full[slot], ph, LSQ_WAIT, &s_stop))) break;
+          const T* d = ring + slot * R::elems + lane * NV;
+          const T* m = s + k * RS + q0 * VEC;
+          if (k + MS <= nk) {
+#pragma unroll
+            for (int j = 0; j < MS; ++j) add(m + j * RS, d + j * 32 * NV);
+          } else {
+            for (int j = 0; j < nk - k; ++j) add(m + j * RS, d + j * 32 * NV);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[slot]);
+          if (++slot == NSTG) slot = 0, ph ^= 1u;
+        }
+      T* Gi = (T*)p.gbuf + (int64_t)(c >> 5) * (A * ID * NV) * 32 + (int64_t)(ll * ID + q0 * VEC) * NV * 32 + (c & 31);
+      if (ok && live)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+          for (int i = 0; i < VEC; ++i)
+            if ((q0 + q) * VEC + i < ND)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) Gi[(int64_t)((q * VEC + i) * NV + v) * 32] = act ? acc[q].get(i, v) : T(0);
+    };
+    if (R::NVEC % R::NSL == 0 || nq == R::MAXV) multiply(IntC<R::MAXV>());
+    else multiply(IntC<(R::MAXV > 1 ? R::MAXV - 1 : 1)>());
+  }
+  if (!ok && lane == 0) {
+    atomicOr(p.health, HEALTH_TIMEOUT);
+    *(volatile int*)&s_stop = 1;
+  }
+}
+
+// The CWENO directional stencils (ND = IDEGFREE2 rows of a few members) of the
+// tiled cells: a tile and a stencil per block, one lane per cell; a warp
+// gathers four members at a time through its own shared-memory buffer.
+template <int P, typename T, int ND>
+__global__ void __launch_bounds__(SET_TILE) k_lsq_low(Problem p, const double* __restrict__ U) {
+  constexpr int ID = Deg<P>::ideg;
+  constexpr int RS = set_stride<T>(ND);
+  constexpr int VEC = Vec<T>::N;
+  constexpr int GRP = 4;
+  extern __shared__ __align__(16) unsigned char lw_smem[];
+  __shared__ T s_du[SET_TILE / 32][GRP][32 * NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tile = blockIdx.x;
+  const int ll = blockIdx.y + 1;
+  const int nk = p.imax2, A = p.admis_max, W = p.imax + 1;
+  T* s = (T*)lw_smem;
+  {
+    const float4* src = (const float4*)((const T*)p.setmat + p.tset[tile] * p.sstride + p.sso[ll]);
+    for (int i = threadIdx.x; i < nk * RS / VEC; i += SET_TILE) ((float4*)s)[i] = src[i];
+  }
+  const int mine = p.tcell[tile * SET_TILE + threadIdx.x];
+  const bool live = mine >= 0;
+  const int c = live ? mine : p.tcell[tile * SET_TILE];
+  const bool act = live && ll < p.admis[c];
+  const int32_t* S = p.sten + (int64_t)(c >> 5) * (A * W) * 32 + (c & 31) + (ll * W + 1) * 32;
+  const GatherShare sh(lane);
+  double u0[NV];
+  sh.load(U, c, u0);
+  T acc[ND][NV];
+#pragma unroll
+  for (int j = 0; j < ND; ++j)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[j][v] = T(0);
+  __syncthreads();
+  for (int k = 0; k < nk; k += GRP) {
+    double u[GRP][NV];
+#pragma unroll
+    for (int j = 0; j < GRP; ++j) sh.load(U, act ? S[(k + j < nk ? k + j : nk - 1) * 32] : c, u[j]);
+    __syncwarp();  // the last group's differences have been read
+#pragma unroll
+    for (int j = 0; j < GRP; ++j)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) s_du[warp][j][lane + 32 * i] = T(u[j][i] - u0[i]);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < GRP; ++j)
+      if (k + j < nk) {
+        T du[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) du[v] = s_du[warp][j][lane * NV + v];
+#pragma unroll
+        for (int q = 0; q < RS / VEC; ++q) {
+          T r[VEC];
+          ldv(s + (k + j) * RS + q * VEC, r);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i)
+            if (q * VEC + i < ND)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) acc[q * VEC + i][v] += r[i] * du[v];
+        }
+      }
+  }
+  if (!live) return;
+  T* Gi = (T*)p.gbuf + (int64_t)(c >> 5) * (A * ID * NV) * 32 + (int64_t)(ll * ID) * NV * 32 + (c & 31);
+#pragma unroll
+  for (int j = 0; j < ND; ++j)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) Gi[(int64_t)(j * NV + v) * 32] = act ? acc[j][v] : T(0);
+}
+
+// Smoothness indicators of the tiled cells: a tile and a stencil per block,
+// the set's triangle in shared memory as 16-byte broadcasts, two variables of
+// the cell's polynomial in registers per pass (one would leave the kernel
+// bound by the shared-memory loads).  k_wis, whose warps read each cell's own
+// copy of the triangle, takes the other cells.
+template <int P, typename T>
+__global__ void __launch_bounds__(SET_TILE) k_wis_set(Problem p) {
+  constexpr int ID = Deg<P>::ideg;
+  constexpr int VEC = Vec<T>::N;
+  constexpr int VI = 2;
+  extern __shared__ __align__(16) unsigned char wi_smem[];
+  T* s = (T*)wi_smem;
+  const int64_t tile = blockIdx.x;
+  const int ll = blockIdx.y, A = p.admis_max;
+  {
+    const float4* tri = (const float4*)((const T*)p.setind + p.tset[tile] * p.istride);
+    for (int i = threadIdx.x; i < p.i2off / VEC; i += SET_TILE) ((float4*)s)[i] = tri[i];
+  }
+  __syncthreads();
+  const int64_t c = p.tcell[tile * SET_TILE + threadIdx.x];
+  if (c < 0 || (!p.mprev && !p.full[c]) || ll >= p.admis[c]) return;
+  const T* Gc = (const T*)p.gbuf + (c >> 5) * (int64_t)(A * ID * NV) * 32 + (int64_t)(ll * ID) * NV * 32 + (c & 31);
+  double* o = p.isb + (((c >> 5) * A + ll) * (int64_t)NV) * 32 + (c & 31);
+#pragma unroll 1
+  for (int v0 = 0; v0 < NV; v0 += VI) {
+    T g[ID][VI], is[VI];
+#pragma unroll
+    for (int d = 0; d < ID; ++d)
+#pragma unroll
+      for (int k = 0; k < VI; ++k) g[d][k] = v0 + k < NV ? Gc[(int64_t)(d * NV + v0 + k) * 32] : T(0);
+#pragma unroll
+    for (int k = 0; k < VI; ++k) is[k] = T(0);
+    int rs = 0;
+#pragma unroll
+    for (int d = 0; d < ID; ++d) {
+      T t[VI];
+#pragma unroll
+      for (int k = 0; k < VI; ++k) t[k] = T(0);
+#pragma unroll
+      for (int q = 0; q < (ID - d + VEC - 1) / VEC; ++q) {
+        T x[VEC];
+        ldv(s + (rs + q) * VEC, x);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i)
+          if (d + q * VEC + i < ID)
+#pragma unroll
+            for (int k = 0; k < VI; ++k) t[k] += x[i] * g[d + q * VEC + i][k];
+      }
+      rs += (ID - d + VEC - 1) / VEC;
+#pragma unroll
+      for (int k = 0; k < VI; ++k) is[k] += g[d][k] * t[k];
+      asm volatile("" ::: "memory");  // as in quad_form
+    }
+#pragma unroll
+    for (int k = 0; k < VI; ++k)
+      if (v0 + k < NV) o[(v0 + k) * 32] = (double)is[k];
+  }
+}
+
 // LEAST_SQUARES of the cells that read their own tables: the pseudo-inverse
 // rows and the gathered differences come through shared memory.  One or two
 // blocks per SM, four pairs of warps: a producer gathers the members'
-// differences into a stage of its pair's ring and issues the
+// differences (as in k_lsq_set) into a stage of its pair's ring and issues the
 // bulk copies (cp.async.bulk) of the members' rows [d0, d0 + DH) of the 32
 // cells, which are contiguous in the interleaved layout; the consumer
 // multiplies.  The full barrier of a stage completes on the producer's arrival
@@ -74,7 +404,8 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity, long l
 // member; here the copies run NSTG stages ahead.  The work is the list of
 // (group, stencil) items, an equal share of consecutive items per pair, so
 // that a mesh of any size fills the SMs (one lane per cell: 16,464 cells were
-// 129 blocks).  Against one lane per cell: 16,464 tetrahedra, WENO5
+// 129 blocks).  With tiles (p.ntile) the groups are those with cells that are
+// not tiled (p.ugrp).  Against one lane per cell: 16,464 tetrahedra, WENO5
 // mixed, 0.500 -> 0.257 ms (1.63 GB, 6.3 TB/s); 82,944, WENO3, FP64 0.312 ->
 // 0.201 (6.4 TB/s), mixed 0.205 -> 0.190; 24,576, CWENO4, FP64 0.160 -> 0.107,
 // mixed 0.237 -> 0.067; two blocks per SM at IORDER 2 and 3 against one: 0.267
@@ -129,8 +460,8 @@ __global__ void __launch_bounds__(256, Ring<P, T>::BPS) k_lsq_ring(Problem p, co
   for (int64_t it = i0; it < i1 && ok; ++it) {
     const int64_t g = it / A;
     const int ll = (int)(it - g * A);
-    const int64_t grp = g, c = grp * 32 + lane;
-    const bool low = cw && ll > 0, live = c < p.n;
+    const int64_t grp = p.ntile ? p.ugrp[g] : g, c = grp * 32 + lane;
+    const bool low = cw && ll > 0, live = c < p.n && !(p.ntile && p.tiled[c]);
     const int nk = low ? p.imax2 : p.imax, nd = low ? p.ideg2 : ID;
     const bool act = live && ll < p.admis[c];
     const bool any = __any_sync(0xffffffffu, act);
@@ -230,22 +561,67 @@ __global__ void __launch_bounds__(256, Ring<P, T>::BPS) k_lsq_ring(Problem p, co
   }
 }
 
+// the cells' own tables: all groups, or those with cells that are not tiled
 template <int P, typename T>
 cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) {
   using R = Ring<P, T>;
   const cudaError_t e = cudaFuncSetAttribute(k_lsq_ring<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem);
   if (e != cudaSuccess) return e;
-  const int64_t items = ((p.n + 31) / 32) * p.admis_max, nb = (items + 3) / 4;
+  const int64_t items = (p.ntile ? p.nugrp : (p.n + 31) / 32) * p.admis_max, nb = (items + 3) / 4;
   const long wait = p.lsq_bulk && p.lsq_wait >= 0 ? p.lsq_wait : LSQ_WAIT;
   k_lsq_ring<P, T><<<(unsigned)(nb < p.nsm * R::BPS ? nb : p.nsm * R::BPS), 256, R::smem, st>>>(p, U, items, wait);
   return cudaGetLastError();
+}
+
+// the least squares of the tiled cells, and of the others through k_lsq_ring
+template <int P, typename T, int ND>
+cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cudaStream_t st) {
+  using R = SetRing<T, ND>;
+  const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + 2 * R::NSTG * R::elems) * sizeof(T);
+  const cudaError_t e = cudaFuncSetAttribute(k_lsq_set<P, T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U);
+  return cudaGetLastError();
+}
+template <int P, typename T, int ND>
+cudaError_t launch_lsq_low(const Problem& p, const double* U, cudaStream_t st) {
+  const size_t smem = (size_t)p.imax2 * set_stride<T>(ND) * sizeof(T);
+  const cudaError_t e = cudaFuncSetAttribute(k_lsq_low<P, T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_lsq_low<P, T, ND><<<dim3((unsigned)p.ntile, (unsigned)p.admis_max - 1), SET_TILE, smem, st>>>(p, U);
+  return cudaGetLastError();
+}
+// The tiled cells' indicators come from k_wis_set: IORDER 4 (the only order
+// with indicators of their own kernel), WENO (CWENO's central polynomial needs
+// the other stencils first).
+template <int P>
+bool sets_give_is(const Problem& p) {
+  return P == 4 && p.ntile && p.isb && p.scheme == 3 && p.ees != 5;
+}
+template <int P, typename T>
+cudaError_t launch_lsq_set(const Problem& p, const double* U, cudaStream_t st, int64_t* launches) {
+  constexpr int ID = Deg<P>::ideg;
+  const bool cw = p.ees == 5 && p.admis_max > 1;
+  cudaError_t e = launch_lsq_set_t<P, T, ID>(p, U, cw ? 1 : (unsigned)p.admis_max, st);
+  if (e == cudaSuccess && cw) {
+    if constexpr (P > 1) {
+      if (p.ideg2 == 9) e = launch_lsq_low<P, T, 9>(p, U, st);
+    }
+    if (p.ideg2 == 3) e = launch_lsq_low<P, T, 3>(p, U, st);
+    ++*launches;
+  }
+  if (e == cudaSuccess && p.nugrp) {
+    e = launch_lsq_ring<P, T>(p, U, st);
+    ++*launches;
+  }
+  return e;
 }
 
 // the stencil polynomials of every cell into p.gbuf, from the state U
 template <int P, typename T>
 cudaError_t launch_lsq(const Problem& p, const double* U, cudaStream_t st, int64_t* launches) {
   ++*launches;
-  return launch_lsq_ring<P, T>(p, U, st);
+  return p.ntile ? launch_lsq_set<P, T>(p, U, st, launches) : launch_lsq_ring<P, T>(p, U, st);
 }
 
 // ------------------------------------------------------------- k_wpost
@@ -332,8 +708,8 @@ __device__ __forceinline__ void quad_form(const T* __restrict__ P, const T (&g)[
 // lane runs all the stencils of its cell.  Output: p.isb, FP64, interleaved
 // over 32-cell groups ((group * A + ll) * NV + v) * 32 + lane; cells that
 // take the MUSCL fall-back outright (not FULL) are skipped, except under
-// MOOD, where every cell is reconstructed.
-template <int P, typename T>
+// MOOD, where every cell is reconstructed.  MASK: not the cells of p.tiled.
+template <int P, typename T, bool MASK = false>
 __global__ void __launch_bounds__(224) k_wis(Problem p) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int VEC = Vec<T>::N;
@@ -342,6 +718,7 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
   const int lane = threadIdx.x & 31, ll = threadIdx.x >> 5;
   const int64_t grp = blockIdx.x, c = grp * 32 + lane;
   if (c >= p.n || (!p.mprev && !p.full[c])) return;
+  if (MASK && p.tiled[c]) return;
   const int adm = p.admis[c];
   if (ll >= adm) return;
   const int A = p.admis_max, ID2 = p.ideg2;
@@ -1386,6 +1763,20 @@ extern template cudaError_t launch_wpost_char<3, double>(const Problem&, const d
 extern template cudaError_t launch_wpost_char<4, double>(const Problem&, const double*, cudaStream_t);
 #endif
 
+// the indicators of every cell into p.isb
+template <int P, typename T>
+cudaError_t launch_wis(const Problem& p, cudaStream_t st) {
+  const unsigned ng = (unsigned)((p.n + 31) / 32), th = 32 * p.admis_max;
+  if (!sets_give_is<P>(p)) {
+    k_wis<P, T><<<ng, th, 0, st>>>(p);
+    return cudaGetLastError();
+  }
+  const size_t smem = (size_t)p.i2off * sizeof(T);
+  k_wis_set<P, T><<<dim3((unsigned)p.ntile, (unsigned)p.admis_max), SET_TILE, smem, st>>>(p);
+  if (p.tiled) k_wis<P, T, true><<<ng, th, 0, st>>>(p);
+  return cudaGetLastError();
+}
+
 // One reconstruction: stencil polynomials, WENO post-processing and, for
 // Navier-Stokes, the viscous LSQ and face gradients.  Instantiated per
 // precision and order in recon_*.cu, which nvcc compiles in parallel.
@@ -1422,7 +1813,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
         const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
         const size_t smem = ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
         cudaFuncSetAttribute(k_wface<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_wis<P, T><<<(unsigned)((p.n + 31) / 32), 32 * p.admis_max, 0, st>>>(p);
+        const cudaError_t e = launch_wis<P, T>(p, st);
+        if (e != cudaSuccess) return e;
         k_wface<P, T><<<(unsigned)((p.n + 31) / 32), 32 * NV, smem, st>>>(p, U);
         k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
         *launches += 2;
@@ -1431,7 +1823,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     }
     if constexpr (P == 4) {
       if (!done && p.isb && p.scheme == 3) {
-        k_wis<P, T><<<(unsigned)((p.n + 31) / 32), 32 * p.admis_max, 0, st>>>(p);
+        const cudaError_t e = launch_wis<P, T>(p, st);
+        if (e != cudaSuccess) return e;
         k_wpost<P, T, true><<<b, 128, 0, st>>>(p, U);
         ++*launches;
         done = true;

@@ -466,7 +466,7 @@ int ucg_build_recon(ucg_engine* e, const ucg_shapes* s, const ucg_recon* r) {
     if ((rc = upload_vec(e, tidbuf, r->table_id, n))) return bail(rc);
     tmp.push_back(&tidbuf);
   }
-  rc = expand_tables(e, 0, n, ntab, (const int32_t*)tidbuf.p, d_rowmap,
+  rc = expand_tables(e, 0, n, ntab, r->table_id, (const int32_t*)tidbuf.p, d_rowmap,
                      [&](int which, int64_t t0, int64_t t1, double* dev) {
                        const int64_t len = which == 0 ? a.tstride : a.istride;
                        CK(cudaMemsetAsync(dev, 0, (size_t)(t1 - t0) * len * 8, e->stream));
