@@ -1,8 +1,10 @@
-"""Matrix sets shared by many cells (k_lsq_set, k_lsq_low, k_wis_set):
+"""Matrix sets shared by many cells (k_lsq_set, k_wis_set, k_adj_lsq_set):
 the same engine once with the tables of one upload, whose shared sets are
 tiled, and once with the same tables uploaded in two halves, where every cell
 reads its own copy.  The forward kernels take the same operations in the same
-order, so residuals and states are equal bit for bit.
+order, so residuals and states are equal bit for bit; the reverse adds a
+member's rows and a cell's stencils in another order (FP64 rounding of sums of
+at most a few thousand terms of one size: 1e-12 of the result's largest value).
 
 Meshes: whole tiles and remainders (1 to 127 cells in a set's last tile), sets
 above and below the 32 cells from which they are tiled, all cells tiled and
@@ -73,3 +75,19 @@ def test_shared_sets_equal_own_tables(name, precision):
     assert np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2]
     assert np.abs(out[0][0]).max() > 0
+
+
+@pytest.mark.parametrize("name", ["weno5_hex12", "weno5_hex_open", "weno3_ns_hex9", "weno3_tet", "cweno4_ns_mixed10",
+                                  "cweno4_mixed16"])
+def test_shared_sets_reverse(name):
+    m, shared, own, U = _engines(name, N.UCG_FP64, shuffle=name == "weno3_tet")
+    rng = np.random.default_rng(3)
+    lam, du = rng.standard_normal(U.shape), rng.standard_normal(U.shape) * 1e-2
+    out = []
+    for e in (shared, own):
+        e.set_state(U)
+        mu, pbar = e.residual_vjp(lam)
+        out.append((mu, pbar, e.residual_jvp(du)))
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
+    assert np.array_equal(out[0][2], out[1][2])
