@@ -28,7 +28,7 @@ CASES = {
     "weno3_ns_hex9": (lambda: Mesh.box_hex(9, 9, 9), SCHEME_WENO, 2, 0, NAVIER_STOKES, 1),
     "weno3_tet": (lambda: Mesh.box_tet(10, 10, 10, jitter=0.0), SCHEME_WENO, 2, 0, EULER, 1),
     "cweno4_ns_mixed10": (lambda: Mesh.mixed_box(10, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES, 1),
-    "cweno4_mixed16": (lambda: Mesh.mixed_box(16, seed=4), SCHEME_WENO, 3, 5, EULER, 1),
+    "cweno4_mixed16": (lambda: Mesh.mixed_box(16, seed=1234), SCHEME_WENO, 3, 5, EULER, 1),
     "muscl_p2_hex8": (lambda: Mesh.box_hex(8, 8, 8), SCHEME_MUSCL, 2, 0, EULER, 1),
 }
 
