@@ -79,7 +79,7 @@ struct Problem {
   void* gbuf;               // stencil polynomials G[ll][d][v], interleaved like the stencils
   double* qbuf;             // characteristic WENO: G_l^T S G_l per stencil, 15 values, interleaved
   double* isb;              // conserved WENO: smoothness indicators [A][NV] per cell, interleaved (k_wis)
-  bool wface;               // IORDER 4 conserved WENO through k_wis + k_wface
+  bool wface;               // conserved WENO through k_wface (IORDER 4: after k_wis)
   int8_t* wflag;            // cells whose reconstruction was reduced (CHECKSOL or not FULL) [n];
                             // k_wface writes it for k_wpost's fall-back pass, k_wpost under MOOD
   // MOOD (RUNGE_KUTTA3_MOOD): all nullptr without it

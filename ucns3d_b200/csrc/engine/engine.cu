@@ -577,12 +577,14 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
   const int64_t ngrp = (n + 31) / 32;
   if (!(c.scheme == 2 && c.iorder == 1))
     rc = rc ? rc : alloc(e, e->gbuf, (size_t)ngrp * 32 * c.admis_max * c.ideg * NV * T);
-  if (c.scheme == 3 && c.wenwrt == 1 && c.iorder == 4) {  // smoothness indicators of every stencil (k_wis)
+  if (c.scheme == 3 && c.wenwrt == 1) {
+    // IORDER 4: smoothness indicators of every stencil in their own kernel
     const char* wis = std::getenv("UCG_WENO_IS");
-    if (!(wis && wis[0] == '0')) rc = rc ? rc : alloc(e, e->isb, (size_t)ngrp * 32 * c.admis_max * NV * 8);
+    const bool own = c.iorder == 4 && !(wis && wis[0] == '0');
+    if (own) rc = rc ? rc : alloc(e, e->isb, (size_t)ngrp * 32 * c.admis_max * NV * 8);
     // face values one warp per variable (k_wface), unless UCG_WENO_FACE=0
     const char* wf = std::getenv("UCG_WENO_FACE");
-    e->wface = !(wis && wis[0] == '0') && !(wf && wf[0] == '0');
+    e->wface = (own || c.iorder < 4) && !(wf && wf[0] == '0');
     if (e->wface) rc = rc ? rc : alloc(e, e->wflag, (size_t)n);
   }
   if (c.mood) {  // RECALC (zero at the start, memory.f90:1002-1005), flags, MOOD_O, candidate

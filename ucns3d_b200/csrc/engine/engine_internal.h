@@ -74,7 +74,7 @@ struct ucg_engine {
   cudaEvent_t mark = nullptr;  // recorded after the least squares while ucg_time_kernels runs
   bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: no shared sets, every cell through k_lsq_ring
   int nsm = 148;
-  bool wface = false;          // IORDER 4 conserved WENO: face values one warp per variable (k_wface)
+  bool wface = false;          // conserved WENO: face values one warp per variable (k_wface)
   long lsq_wait = -1;          // polls of a k_lsq_ring stage wait (ucg_set_wait_limit; < 0 the default)
   std::vector<uint8_t> recon_done;  // per cell, for ucg_upload_recon chunks
   std::vector<int8_t> admis_h;      // ADMIS per cell, for the stencil checks of ucg_upload_recon

@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
   }
 }
 
-// k_wface (conserved-variable WENO, IORDER 4, indicators from k_wis): the
+// k_wface (conserved-variable WENO; IORDER 4: indicators from k_wis): the
 // nonlinear weights, the combined polynomial and its face values, one block
 // per 32-cell group with one warp per conserved variable (lane i: cell i of
 // the group).  A thread holds one variable's combined polynomial (ID
@@ -786,7 +786,17 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
 // Weights, combination and face values take k_wpost's operations in
 // k_wpost's order.  Under MOOD the cells that are not FULL are reconstructed
 // too (over their admissible stencils) and marked.
-template <int P, typename T>
+// OWN (IORDER 1-3): each warp forms its variable's indicators itself, g^T S g
+// of one polynomial at a time from the cells' triangles, which the five warps
+// read from L1.  One lane per cell with all five variables (k_wpost) is bound
+// by load latency at 12 warps per SM: WENO3, 82,944 tetrahedra FP64 0.190 ->
+// 0.131 ms, mixed 0.103 -> 0.099, 64,000 hexahedra mixed 0.118 -> 0.094, 3,072
+// tetrahedra FP64 0.044 -> 0.028.  At IORDER 3 it wins only where k_wpost's
+// blocks leave SMs idle, below a block of 128 per SM (CWENO4, 9,728 cells FP64
+// 0.156 -> 0.089 ms, mixed 0.075 -> 0.044); above, reading the triangles in
+// five warps costs more than it hides (271,872 cells mixed 0.564 -> 0.626,
+// 24,576 FP64 0.133 -> 0.139).
+template <int P, typename T, bool OWN = false>
 __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int L2 = ID < 9 ? ID : 9;
@@ -814,23 +824,70 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
   const double lc1 = 1.0 - 1.0 / p.lwci;
   const double lk = adm > 1 ? (1.0 - lc1) / (adm - 1) : 0.0;
   if (tid < 32) s_flag[tid] = full ? 0 : 1;
+  const T* Gc = (const T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + v * 32 + lane;
+  auto G = [&](int l, int d) -> T { return Gc[(int64_t)((l * ID + d) * NV) * 32]; };
+  // the central polynomial (CWENO: the central stencil with the lower-order
+  // ones removed, reconstruct_p.f90:956-965)
+  auto central = [&](T (&g)[ID]) {
+#pragma unroll
+    for (int d = 0; d < ID; ++d) g[d] = live ? G(0, d) : T(0);
+    if (live && cw) {
+      T g3[L2];
+#pragma unroll
+      for (int d = 0; d < L2; ++d) g3[d] = T(0);
+      for (int l2 = 1; l2 < adm; ++l2)
+#pragma unroll
+        for (int d = 0; d < L2; ++d)
+          if (d < ID2) g3[d] = g3[d] + T(lk) * G(l2, d);
+#pragma unroll
+      for (int d = 0; d < ID; ++d) g[d] = T(1.0 / lc1) * (g[d] - (d < L2 ? g3[d] : T(0)));
+    }
+  };
   // ---- weights of variable v (WENOWEIGHTS, FP64)
   double w[MA];
   {
-    const double* is = p.isb + grp * (int64_t)A * NV * 32 + lane + v * 32;
+    const double* isg = OWN ? nullptr : p.isb + grp * (int64_t)A * NV * 32 + lane + v * 32;
+    double is[MA];
+    if constexpr (OWN) {
+      constexpr int VEC = Vec<T>::N;
+      const T* Pc = (const T*)p.ind + grp * p.istride * 32 + lane * VEC;
+#pragma unroll
+      for (int l = 0; l < MA; ++l) {
+        is[l] = 0.0;
+        if (l < adm) {
+          T q[1] = {T(0)};
+          if (cw && l > 0) {
+            T g[L2][1];
+#pragma unroll
+            for (int d = 0; d < L2; ++d) g[d][0] = d < ID2 ? G(l, d) : T(0);
+            quad_form<L2, 1>(Pc + (int64_t)(p.i2off / VEC) * 32 * VEC, g, ID2, q);
+          } else {
+            T c0[ID], g[ID][1];
+            if (l == 0) central(c0);
+#pragma unroll
+            for (int d = 0; d < ID; ++d) g[d][0] = l == 0 ? c0[d] : G(l, d);
+            quad_form<ID, 1>(Pc, g, ID, q);
+          }
+          is[l] = (double)q[0];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int l = 0; l < MA; ++l) is[l] = l < adm ? isg[(int64_t)l * NV * 32] : 0.0;
+    }
     const double lam0 = cw ? lc1 : p.lwci, lamk = cw ? lk : 1.0;
     double tau = 0.0, sum = 0.0;
     if (cw && p.wenoz) {
 #pragma unroll
       for (int l = 0; l < MA; ++l)
-        if (l < adm) tau += fabs(is[0] - is[(int64_t)l * NV * 32]);
+        if (l < adm) tau += fabs(is[0] - is[l]);
       tau = tau / (adm - 1);
     }
 #pragma unroll
     for (int l = 0; l < MA; ++l) {
       w[l] = 0.0;
       if (l < adm) {
-        const double e = p.weno_eps + is[(int64_t)l * NV * 32];
+        const double e = p.weno_eps + is[l];
         const double lam = l == 0 ? lam0 : lamk;
         double wt;
         if (cw && p.wenoz) {
@@ -848,24 +905,9 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
 #pragma unroll
     for (int l = 0; l < MA; ++l) w[l] = w[l] / sum;
   }
-  // ---- combined polynomial of variable v (CWENO: the central stencil with
-  // the lower-order ones removed, reconstruct_p.f90:956-965)
-  const T* Gc = (const T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + v * 32 + lane;
-  auto G = [&](int l, int d) -> T { return Gc[(int64_t)((l * ID + d) * NV) * 32]; };
+  // ---- combined polynomial of variable v
   T gh[ID];
-#pragma unroll
-  for (int d = 0; d < ID; ++d) gh[d] = live ? G(0, d) : T(0);
-  if (live && cw) {
-    T g3[L2];
-#pragma unroll
-    for (int d = 0; d < L2; ++d) g3[d] = T(0);
-    for (int l2 = 1; l2 < adm; ++l2)
-#pragma unroll
-      for (int d = 0; d < L2; ++d)
-        if (d < ID2) g3[d] = g3[d] + T(lk) * G(l2, d);
-#pragma unroll
-    for (int d = 0; d < ID; ++d) gh[d] = T(1.0 / lc1) * (gh[d] - (d < L2 ? g3[d] : T(0)));
-  }
+  central(gh);
   if (live) {
     const T w0 = T(w[0]);
 #pragma unroll
@@ -1808,27 +1850,30 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     // at IORDER 2-3 the triangle is small and the extra kernel costs more
     // than it saves (2.1 M-cell CWENO4: 17.3 -> 19.6 ms)
     bool done = false;
+    const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+    const size_t smem = ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
+    const unsigned ng = (unsigned)((p.n + 31) / 32);
     if constexpr (P == 4) {
-      if (p.wface && p.isb && p.scheme == 3) {
-        const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-        const size_t smem = ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
-        cudaFuncSetAttribute(k_wface<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (p.isb && p.scheme == 3) {
         const cudaError_t e = launch_wis<P, T>(p, st);
         if (e != cudaSuccess) return e;
-        k_wface<P, T><<<(unsigned)((p.n + 31) / 32), 32 * NV, smem, st>>>(p, U);
-        k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
-        *launches += 2;
-        done = true;
-      }
-    }
-    if constexpr (P == 4) {
-      if (!done && p.isb && p.scheme == 3) {
-        const cudaError_t e = launch_wis<P, T>(p, st);
-        if (e != cudaSuccess) return e;
-        k_wpost<P, T, true><<<b, 128, 0, st>>>(p, U);
         ++*launches;
+        if (p.wface) {
+          cudaFuncSetAttribute(k_wface<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          k_wface<P, T><<<ng, 32 * NV, smem, st>>>(p, U);
+          k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
+          ++*launches;
+        } else {
+          k_wpost<P, T, true><<<b, 128, 0, st>>>(p, U);
+        }
         done = true;
       }
+    } else if (p.wface && p.scheme == 3 && (P < 3 || p.n < (int64_t)p.nsm * 128)) {
+      cudaFuncSetAttribute(k_wface<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_wface<P, T, true><<<ng, 32 * NV, smem, st>>>(p, U);
+      k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
+      ++*launches;
+      done = true;
     }
     if (!done) k_wpost<P, T><<<b, 128, 0, st>>>(p, U);
   }
