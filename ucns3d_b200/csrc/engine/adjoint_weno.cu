@@ -30,8 +30,9 @@ using namespace ucg;
 namespace {
 
 // gr += 2 S g for the packed triangle P of S (rows padded to vectors; P_dd =
-// S_dd, P_de = 2 S_de), over the first nd <= NMAX rows
-template <int NMAX>
+// S_dd, P_de = 2 S_de), over the first nd <= NMAX rows; STR 32: the cell's
+// own triangle in the interleaved tables, 1: a shared set's, contiguous
+template <int NMAX, int STR = 32>
 __device__ __forceinline__ void tri_grad(const double* __restrict__ P, const double (&g)[NMAX], int nd,
                                          double (&gr)[NMAX]) {
   constexpr int VEC = Vec<double>::N;
@@ -43,7 +44,7 @@ __device__ __forceinline__ void tri_grad(const double* __restrict__ P, const dou
       for (int q = 0; q < (NMAX - d + VEC - 1) / VEC; ++q)
         if (d + q * VEC < nd) {
           double sv[VEC];
-          ldv(P + (int64_t)(rs + q) * 32 * VEC, sv);
+          ldv(P + (int64_t)(rs + q) * STR * VEC, sv);
 #pragma unroll
           for (int i = 0; i < VEC; ++i) {
             const int e = d + q * VEC + i;
@@ -64,12 +65,12 @@ __device__ __forceinline__ void tri_grad(const double* __restrict__ P, const dou
 }
 
 // IS = g^T S g and gr = 2 S g in one pass over the packed triangle
-template <int NMAX>
+template <int NMAX, int STR = 32>
 __device__ __forceinline__ double is_and_grad(const double* __restrict__ P, const double (&g)[NMAX], int nd,
                                               double (&gr)[NMAX]) {
 #pragma unroll
   for (int d = 0; d < NMAX; ++d) gr[d] = 0.0;
-  tri_grad<NMAX>(P, g, nd, gr);
+  tri_grad<NMAX, STR>(P, g, nd, gr);
   double is = 0.0;
 #pragma unroll
   for (int d = 0; d < NMAX; ++d)
@@ -84,7 +85,21 @@ __device__ __forceinline__ double is_and_grad(const double* __restrict__ P, cons
 // at the CHECKSOL test (all five variables of a face value); and the five
 // warps read the same smoothness matrices at about the same time, so those
 // come from DRAM about once per pass instead of once per variable.
+// Where all cells of the group share a matrix set (p.gset) the block keeps the
+// set's triangles in shared memory and the warps read them as broadcasts: the
+// 35 passes over the cells' own copies (152 KB a group at IORDER 4) come from
+// L2.  24^3 WENO5: k_adj_wpost 0.86 -> 0.74 ms, k_jvp_wpost
+// 0.72 -> 0.57.
 constexpr int WP_THREADS = NV * 32;
+extern __shared__ __align__(16) double wp_tri[];
+// the group's shared triangles into wp_tri (all threads; a barrier follows)
+__device__ __forceinline__ bool group_triangles(const Problem& p, int64_t grp) {
+  const int gs = p.ntile ? p.gset[grp] : -1;
+  if (gs < 0) return false;
+  const double2* src = (const double2*)((const double*)p.setind + gs * p.istride);
+  for (int i = threadIdx.x; i < p.istride / 2; i += WP_THREADS) ((double2*)wp_tri)[i] = src[i];
+  return true;
+}
 #ifndef UCG_AWP_MINB
 #define UCG_AWP_MINB 2  // blocks per SM the register budget is sized for
 #endif
@@ -211,6 +226,8 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_adj_wpost(Problem 
   const bool cell = c < p.n;
   const bool full = cell && p.full[c];
   if (v == 0) sFall[lane] = cell && !full ? 1 : 0;
+  const bool shared = group_triangles(p, grp);
+  __syncthreads();
   const int A = p.admis_max, IM = p.imax;
   const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
   const int FQ = MF * QS;
@@ -283,7 +300,7 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_adj_wpost(Problem 
         double g[L2], gr[L2];
 #pragma unroll
         for (int d = 0; d < L2; ++d) g[d] = poly(ll, d);
-        s = is_and_grad<L2>(Pc2, g, ID2, gr);
+        s = shared ? is_and_grad<L2, 1>(wp_tri + p.i2off, g, ID2, gr) : is_and_grad<L2>(Pc2, g, ID2, gr);
 #pragma unroll
         for (int d = 0; d < L2; ++d)
           if (d < ID2) GB(ll, d) = gr[d];
@@ -291,7 +308,7 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_adj_wpost(Problem 
         double g[ID], gr[ID];
 #pragma unroll
         for (int d = 0; d < ID; ++d) g[d] = poly(ll, d);
-        s = is_and_grad<ID>(Pc, g, ID, gr);
+        s = shared ? is_and_grad<ID, 1>(wp_tri, g, ID, gr) : is_and_grad<ID>(Pc, g, ID, gr);
 #pragma unroll
         for (int d = 0; d < ID; ++d) GB(ll, d) = gr[d];
       }
@@ -637,6 +654,8 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_jvp_wpost(Problem 
   const bool cell = c < p.n;
   const bool live = cell && p.full[c];
   if (v == 0) sFall[lane] = cell && !live ? 1 : 0;
+  const bool shared = group_triangles(p, grp);
+  __syncthreads();
   const int A = p.admis_max;
   const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
   const int FQ = MF * QS;
@@ -687,14 +706,14 @@ __global__ void __launch_bounds__(WP_THREADS, UCG_AWP_MINB) k_jvp_wpost(Problem 
         double g[L2], gr[L2];
 #pragma unroll
         for (int d = 0; d < L2; ++d) g[d] = poly(ll, d);
-        a = is_and_grad<L2>(Pc2, g, ID2, gr);
+        a = shared ? is_and_grad<L2, 1>(wp_tri + p.i2off, g, ID2, gr) : is_and_grad<L2>(Pc2, g, ID2, gr);
 #pragma unroll
         for (int d = 0; d < L2; ++d) da += dpoly(ll, d) * gr[d];
       } else {
         double g[ID], gr[ID];
 #pragma unroll
         for (int d = 0; d < ID; ++d) g[d] = poly(ll, d);
-        a = is_and_grad<ID>(Pc, g, ID, gr);
+        a = shared ? is_and_grad<ID, 1>(wp_tri, g, ID, gr) : is_and_grad<ID>(Pc, g, ID, gr);
 #pragma unroll
         for (int d = 0; d < ID; ++d) da += dpoly(ll, d) * gr[d];
       }
@@ -1016,7 +1035,10 @@ template <int P>
 cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, double* gbar, double* scr, double* selfc,
                      double* contrib, cudaStream_t st, int64_t* launches) {
   constexpr int ID = Deg<P>::ideg;
-  k_adj_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, 0, st>>>(p, U, adjF, gbar, scr, selfc, contrib);
+  const size_t tri = p.ntile ? (size_t)p.istride * 8 : 0;
+  const cudaError_t ea = cudaFuncSetAttribute(k_adj_wpost<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri);
+  if (ea != cudaSuccess) return ea;
+  k_adj_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, tri, st>>>(p, U, adjF, gbar, scr, selfc, contrib);
   if (p.ntile) {
     const bool cw = p.ees == 5 && p.admis_max > 1;
     cudaError_t e = launch_adj_set<P, ID, false>(p, cw ? 1 : p.admis_max, gbar, scr, contrib, st);
@@ -1042,7 +1064,9 @@ cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, doub
 template <int P>
 void launch_jvp_t(const Problem& p, const double* U, const double* dU, const double* dG, double* tdul,
                   cudaStream_t st) {
-  k_jvp_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, 0, st>>>(p, U, dU, dG, tdul);
+  const size_t tri = p.ntile ? (size_t)p.istride * 8 : 0;
+  cudaFuncSetAttribute(k_jvp_wpost<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri);
+  k_jvp_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, tri, st>>>(p, U, dU, dG, tdul);
 }
 
 }  // namespace

@@ -73,6 +73,7 @@ struct Problem {
   int64_t sstride;
   int sso[8];
   const void* setind;       // [nset][istride] the sets' packed smoothness triangles (WENO)
+  const int32_t* gset;      // [groups] the set that all cells of a 32-cell group share, -1 = none
   const int32_t* ugrp;      // [nugrp] 32-cell groups with cells that are not tiled (k_lsq_ring)
   int64_t nugrp;
   // scratch
@@ -149,6 +150,14 @@ constexpr int SET_TILE = 128;
 template <typename T>
 __host__ __device__ constexpr int set_stride(int nd) {
   return (nd + Vec<T>::N - 1) / Vec<T>::N * Vec<T>::N;
+}
+
+// elements of a packed triangle of n rows, each padded to whole vectors
+template <typename T>
+__host__ __device__ constexpr int tri_len(int n) {
+  int t = 0;
+  for (int d = 0; d < n; ++d) t += set_stride<T>(n - d);
+  return t;
 }
 
 template <int P>

@@ -135,6 +135,7 @@ Problem make_problem(ucg_engine* e) {
   p.sstride = e->sstride;
   for (int k = 0; k < 8; ++k) p.sso[k] = e->sso[k];
   p.setind = e->setind.p;
+  p.gset = (const int32_t*)e->gset.p;
   p.ugrp = (const int32_t*)e->ugrp.p;
   p.nugrp = e->nugrp;
   p.gbuf = e->gbuf.p;
@@ -637,7 +638,7 @@ void ucg_destroy(ucg_engine* e) {
                    &e->qbuf, &e->d_n2o, &e->permbuf, &e->fgrad, &e->isb, &e->wflag, &e->mprev, &e->mflag,
                    &e->msel, &e->mmus, &e->mord, &e->Um, &e->imp_dtl, &e->imp_dinv, &e->imp_off, &e->imp_du,
                    &e->tcell, &e->tset, &e->tiled, &e->setmat, &e->setind,
-                   &e->ugrp,
+                   &e->gset, &e->ugrp,
                    &e->dual_hist, &e->dual_part, &e->halo_send, &e->halo_recv, &e->wl_buf};
   for (DevBuf* b : all) release(*b);
   adjoint_release(e);
@@ -981,6 +982,14 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
   rc = rc ? rc : upload(e, e->tiled, tiled);
   rc = rc ? rc : alloc(e, e->setmat, (size_t)nset * e->sstride * tsize(e));
   if (c.scheme == 3) rc = rc ? rc : alloc(e, e->setind, (size_t)nset * e->layout.istride * tsize(e));
+  std::vector<int32_t> gset((size_t)((n + 31) / 32), -1);
+  for (int64_t g = 0; g < n; g += 32) {
+    int32_t t = set_of[table(g)];
+    for (int64_t i = g; i < n && i < g + 32; ++i)
+      if (set_of[table(i)] != t) t = -1;
+    gset[(size_t)(g >> 5)] = t;
+  }
+  rc = rc ? rc : upload(e, e->gset, gset);
   rc = rc ? rc : upload(e, e->ugrp, ugrp);
   e->nugrp = (int64_t)ugrp.size();
   if (rc) return rc;

@@ -1491,7 +1491,8 @@ __global__ void k_visc_facegrad(Problem p) {
 // variable fit in registers, and the five warps read the same triangles and
 // stencil polynomials at about the same time (from L1).  One lane per cell
 // with all five variables (four 64-thread blocks per SM, 1-1.4 KB of spills)
-// was latency-bound: 27,000 cells, WENO5 FP64: 5.92 ms -> 0.52 + 1.28 ms.
+// was latency-bound: 27,000 cells, WENO5 FP64: 5.92 ms -> 0.16 + 1.06 ms.
+// Three blocks of k_char_forms per SM (0.52 ms with two, 0.66 with four).
 //
 // Rows d < IDEGFREE2 of sum_l2 lk G_l2, what CWENO takes off its central
 // stencil (reconstruct_p.f90:1723-1737), of variable v into s[d][v][lane].
@@ -1510,12 +1511,13 @@ __device__ __forceinline__ void char_lower_sum(const Problem& p, const T* Gc, in
 // G_l^T S G_l (symmetric 5x5, upper triangle row by row) of every stencil:
 // block (group, stencil), warp w forms the column products with variable w.
 template <int P, typename T>
-__global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
+__global__ void __launch_bounds__(32 * NV, 3) k_char_forms(Problem p) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int VEC = Vec<T>::N;
   constexpr int L2 = ID < 9 ? ID : 9;
   __shared__ T s_a[NV * NV][32];
   __shared__ T s_g[L2 * NV * 32];
+  __shared__ __align__(16) T s_tri[tri_len<T>(ID)];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ll = blockIdx.y;
   const int64_t grp = blockIdx.x, c = grp * 32 + lane;
   const bool cell = c < p.n, full = cell && p.full[c];
@@ -1524,10 +1526,16 @@ __global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
   const int A = p.admis_max, ID2 = p.ideg2;
   const bool cw = p.ees == 5, low = cw && ll > 0, rem = cw && ll == 0;
   const T* Gc = (const T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
-  if (rem) {
-    char_lower_sum<P, T>(p, Gc, adm, w, lane, s_g);
-    __syncthreads();
+  // where all cells of the group share a matrix set, its triangle is read as
+  // broadcasts (27,000 cells, WENO5 FP64: 0.41 -> 0.16 ms)
+  const int gs = p.ntile ? p.gset[grp] : -1;
+  if (gs >= 0) {
+    const T* src = (const T*)p.setind + gs * p.istride + (low ? p.i2off : 0);
+    const int nt = low ? (int)p.istride - p.i2off : p.i2off;
+    for (int i = threadIdx.x; i < nt / VEC; i += 32 * NV) ((float4*)s_tri)[i] = ((const float4*)src)[i];
   }
+  if (rem) char_lower_sum<P, T>(p, Gc, adm, w, lane, s_g);
+  __syncthreads();
   const T ilc = T(1.0 / (1.0 - 1.0 / p.lwci));
   auto Gp = [&](int d, int u) -> T {
     const T g = Gc[(int64_t)((ll * ID + d) * NV + u) * 32];
@@ -1538,8 +1546,8 @@ __global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
 #pragma unroll
   for (int u = 0; u < NV; ++u) a[u] = T(0);
   // a[u] += g[d][u] * sum_{e>=d} P_de g[e][w], the packed triangle as in quad_form
-  auto form = [&](auto& g, const T* Pl, int nd) {
-    constexpr int ND = sizeof(g) / sizeof(T);
+  auto form = [&](auto& g, const T* Pl, int nd, auto strc) {
+    constexpr int ND = sizeof(g) / sizeof(T), STR = decltype(strc)::value;
 #pragma unroll
     for (int d = 0; d < ND; ++d) g[d] = d < nd ? Gp(d, w) : T(0);
     int rs = 0;
@@ -1551,7 +1559,7 @@ __global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
         for (int q = 0; q < (ND - d + VEC - 1) / VEC; ++q)
           if (d + q * VEC < nd) {
             T x[VEC];
-            ldv(Pl + (int64_t)(rs + q) * 32 * VEC, x);
+            ldv(Pl + (int64_t)(rs + q) * STR * VEC, x);
 #pragma unroll
             for (int i = 0; i < VEC; ++i)
               if (d + q * VEC + i < ND) t += x[i] * g[d + q * VEC + i];
@@ -1565,10 +1573,12 @@ __global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
   if (ll < adm) {
     if (low) {
       T g[L2];
-      form(g, Pc + (int64_t)(p.i2off / VEC) * 32 * VEC, ID2);
+      if (gs >= 0) form(g, s_tri, ID2, IntC<1>());
+      else form(g, Pc + (int64_t)(p.i2off / VEC) * 32 * VEC, ID2, IntC<32>());
     } else {
       T g[ID];
-      form(g, Pc, ID);
+      if (gs >= 0) form(g, s_tri, ID, IntC<1>());
+      else form(g, Pc, ID, IntC<32>());
     }
   }
 #pragma unroll
@@ -1587,10 +1597,13 @@ __global__ void __launch_bounds__(32 * NV) k_char_forms(Problem p) {
 }
 
 // Faces of a block, whose polynomials of one variable stay in registers
-// together, so that each stencil polynomial is read once for all of them.
+// together, so that each stencil polynomial is read once for all of them.  In
+// FP64 at IORDER 4 one face: two leave no registers for loads in flight
+// (27,000 cells: 1.28 ms with two, 1.06 with one and two blocks per SM, 1.38
+// with three).
 template <int P, typename T>
 struct CharFaces {
-  static constexpr int value = P < 4 || sizeof(T) == 4 ? 3 : 2;
+  static constexpr int value = P < 4 || sizeof(T) == 4 ? 3 : 1;
 };
 template <int P, typename T>
 __host__ __device__ constexpr size_t char_face_smem(int QS) {
@@ -1598,7 +1611,7 @@ __host__ __device__ constexpr size_t char_face_smem(int QS) {
   return (size_t)NF * (50 + 7 * NV) * 32 * 8 + ((size_t)((QS * NV) | 1) + L2 * NV) * 32 * sizeof(T);
 }
 template <int P, typename T>
-__global__ void __launch_bounds__(32 * NV) k_char_face(Problem p, const double* __restrict__ U) {
+__global__ void __launch_bounds__(32 * NV, 2) k_char_face(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int L2 = ID < 9 ? ID : 9;
   constexpr int NF = CharFaces<P, T>::value;
