@@ -76,9 +76,37 @@ __global__ void k_over_vol(Problem p, double s, const double* __restrict__ x, do
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < p.n * NV) lam[i] = s * x[i] / p.vol[i / NV];
 }
-// acc[k] += s * part[k], k < 5
-__global__ void k_pacc(double s, const double* __restrict__ part, double* __restrict__ acc) {
-  if (threadIdx.x < NV) acc[threadIdx.x] += s * part[threadIdx.x];
+// The algebra of one reversed RK3 stage after its residual's VJP mu (and the
+// free-stream part), in one pass instead of two copies, two or three sums, a
+// division by the volumes and the five-value sum, each a launch of its own
+// (28,810 cells: 17 launches and copies of 3.3 us a step -> 3 of 2.6).  STAGE 3:
+// x = ub, STAGE 2: x = u2b, STAGE 1: x = u1b, the adjoint of the stage's
+// output; y receives that of its input, lam = y / V the cotangent of the next
+// VJP, u0b collects the step's input:
+//   U3 = 1/3 U0 + 2/3 U2 - 2/3 dt R(U2)/V
+//   U2 = 3/4 U0 + 1/4 U1 - 1/4 dt R(U1)/V
+//   U1 = U0 - dt R(U0)/V              (y = u0b, the next step's ub)
+template <int STAGE>
+__global__ void k_rk_rev(Problem p, double dt, const double* __restrict__ mu, const double* __restrict__ x,
+                         double* __restrict__ y, double* __restrict__ u0b, double* __restrict__ lam,
+                         const double* __restrict__ part, double* __restrict__ pacc) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr double c = STAGE == 3 ? 2.0 / 3.0 : STAGE == 2 ? 0.25 : 1.0;
+  if (i < NV) pacc[i] += -c * dt * part[i];
+  if (i >= p.n * NV) return;
+  const double xi = x[i];
+  double yi;
+  if (STAGE == 3) {
+    yi = -c * dt * mu[i] + c * xi;
+    u0b[i] = (1.0 / 3.0) * xi;
+  } else if (STAGE == 2) {
+    yi = -c * dt * mu[i] + c * xi;
+    u0b[i] = 0.75 * xi + u0b[i];
+  } else {
+    yi = -dt * mu[i] + (xi + u0b[i]);
+  }
+  y[i] = yi;
+  lam[i] = yi / p.vol[i / NV];
 }
 
 // deterministic column sums of a [m][5] array: block k sums column k
@@ -156,11 +184,13 @@ __device__ __forceinline__ void adj_face_inputs(const Problem& p, const double* 
 }
 
 // Interior and mirror faces, owned faces [0, nplain): reverse sweep of HLLC
-// (ad::hllc_adj) in the face frame at every face point.  The rotations are
+// (ad::hllc_adj) in the face frame at every face point.  Eight blocks per SM:
+// latency-bound (340,000 faces 51.7 -> 44.0 us, 16 points a face 121 -> 88 us;
+// ten blocks 51).  The rotations are
 // orthogonal (rot_b = rot_f^T), and a mirror ghost is b = S a in the face
 // frame (S flips the normal momentum; a Navier-Stokes wall, no slip, flips
 // the whole momentum).
-__global__ void __launch_bounds__(64) k_adj_face(Problem p, int64_t nplain, const double* __restrict__ U,
+__global__ void __launch_bounds__(64, 8) k_adj_face(Problem p, int64_t nplain, const double* __restrict__ U,
                                                   const double* __restrict__ lam, double* __restrict__ adjF) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nplain) return;
@@ -1898,19 +1928,40 @@ int ucg_adjoint_run_obj(ucg_engine* e, int32_t objective, int32_t nsteps, double
   const size_t m = (size_t)n * NV, mb = m * 8;
   const int nseg = (nsteps + every - 1) / every;
   const int K = std::min<int>(every, std::max(nsteps, 1));
-  // checkpoints [nseg][n][5], stage states of one segment [K][3][n][5], final state
-  if ((rc = alloc(e, e->adj_traj, ((size_t)std::max(nseg, 1) + (size_t)3 * K + 1) * mb))) return rc;
+  // checkpoints [nseg][n][5], stage states of one segment [K][3][n][5] (the
+  // first step's input is the checkpoint)
+  if ((rc = alloc(e, e->adj_traj, ((size_t)std::max(nseg, 1) + (size_t)3 * K) * mb))) return rc;
   double* ckpt = (double*)e->adj_traj.p;
   double* traj = ckpt + (size_t)std::max(nseg, 1) * m;
-  double* fin = traj + (size_t)3 * K * m;
   double* Un = (double*)e->Un.p;
   Problem p = make_problem(e);
-  // forward with checkpoints
+  // states of step s of segment seg: its input (k = 0) and first two stages
+  auto at = [&](int seg, int s, int k) -> double* {
+    const int j = s - seg * every;
+    return j == 0 && k == 0 ? ckpt + (size_t)seg * m : traj + ((size_t)3 * j + k) * m;
+  };
+  // step s of segment seg with its stages kept; the result into out (nullptr:
+  // the last stage is not needed)
+  auto step_into = [&](int seg, int s, double* out) -> int {
+    double *U0 = at(seg, s, 0), *U1 = at(seg, s, 1), *U2 = at(seg, s, 2);
+    int r;
+    if ((r = launch_recon(e, p, U0))) return r;
+    if ((r = launch_flux(e, p, 1, U0, U0, U1, dt))) return r;
+    if ((r = launch_recon(e, p, U1))) return r;
+    if ((r = launch_flux(e, p, 2, U1, U0, U2, dt))) return r;
+    if (!out) return UCG_OK;
+    if ((r = launch_recon(e, p, U2))) return r;
+    return launch_flux(e, p, 3, U2, U0, out, dt);
+  };
+  // forward with checkpoints; the last segment keeps its states, so it need
+  // not be computed again
   for (int s = 0; s < nsteps; ++s) {
-    if (s % every == 0) CK(cudaMemcpyAsync(ckpt + (size_t)(s / every) * m, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
-    if ((rc = rk3(e, dt))) return rc;
+    const int seg = s / every;
+    if (s % every == 0) CK(cudaMemcpyAsync(ckpt + (size_t)seg * m, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
+    if (seg < nseg - 1) rc = rk3(e, dt);
+    else rc = step_into(seg, s, s + 1 < nsteps ? at(seg, s + 1, 0) : Un);
+    if (rc) return rc;
   }
-  CK(cudaMemcpyAsync(fin, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
   double* sc = bar_scal(e);  // sc[0] J, sc[8..12] pbar accumulator, sc[16..20] partial
   double* pacc = sc + 8;
   double* part = sc + 16;
@@ -1924,49 +1975,27 @@ int ucg_adjoint_run_obj(ucg_engine* e, int32_t objective, int32_t nsteps, double
   double* lam = o.lam;
   if ((rc = run_obj_vjp(e, o, p, Un, ub))) return rc;
   CK(cudaMemsetAsync(pacc, 0, NV * 8, e->stream));
-  const unsigned bm = blocks_for((int64_t)m, 256), bv = blocks_for((int64_t)m, 256);
+  const unsigned bm = blocks_for((int64_t)m, 256);
+  if (nsteps) {
+    k_over_vol<<<bm, 256, 0, e->stream>>>(p, 1.0, ub, lam);
+    e->launches++;
+  }
   for (int seg = nseg - 1; seg >= 0; --seg) {
     const int s0 = seg * every, s1 = std::min(nsteps, s0 + every);
-    CK(cudaMemcpyAsync(Un, ckpt + (size_t)seg * m, mb, cudaMemcpyDeviceToDevice, e->stream));
-    for (int s = s0; s < s1; ++s) {
-      double* t = traj + (size_t)3 * (s - s0) * m;
-      CK(cudaMemcpyAsync(t, Un, mb, cudaMemcpyDeviceToDevice, e->stream));
-      if ((rc = rk3(e, dt))) return rc;
-      CK(cudaMemcpyAsync(t + m, e->Ua.p, mb, cudaMemcpyDeviceToDevice, e->stream));
-      CK(cudaMemcpyAsync(t + 2 * m, e->Ub.p, mb, cudaMemcpyDeviceToDevice, e->stream));
-    }
+    if (seg < nseg - 1)
+      for (int s = s0; s < s1; ++s)
+        if ((rc = step_into(seg, s, s + 1 < s1 ? at(seg, s + 1, 0) : nullptr))) return rc;
     for (int s = s1 - 1; s >= s0; --s) {
-      const double* U0 = traj + (size_t)3 * (s - s0) * m;
-      const double* U1 = U0 + m;
-      const double* U2 = U0 + 2 * m;
-      // U3 = 1/3 U0 + 2/3 U2 - 2/3 dt R(U2)/V
-      k_over_vol<<<bv, 256, 0, e->stream>>>(p, 1.0, ub, lam);
-      if ((rc = run_vjp(e, o, p, U2, lam, mu, part))) return rc;
-      k_pacc<<<1, 32, 0, e->stream>>>(-(2.0 / 3.0) * dt, part, pacc);
-      CK(cudaMemcpyAsync(u2b, ub, mb, cudaMemcpyDeviceToDevice, e->stream));
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, -(2.0 / 3.0) * dt, mu, 2.0 / 3.0, u2b);
-      CK(cudaMemcpyAsync(u0b, ub, mb, cudaMemcpyDeviceToDevice, e->stream));
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, 0.0, ub, 1.0 / 3.0, u0b);
-      // U2 = 3/4 U0 + 1/4 U1 - 1/4 dt R(U1)/V
-      k_over_vol<<<bv, 256, 0, e->stream>>>(p, 1.0, u2b, lam);
-      if ((rc = run_vjp(e, o, p, U1, lam, mu, part))) return rc;
-      k_pacc<<<1, 32, 0, e->stream>>>(-0.25 * dt, part, pacc);
-      CK(cudaMemcpyAsync(u1b, u2b, mb, cudaMemcpyDeviceToDevice, e->stream));
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, -0.25 * dt, mu, 0.25, u1b);
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, 0.75, u2b, 1.0, u0b);
-      // U1 = U0 - dt R(U0)/V
-      k_over_vol<<<bv, 256, 0, e->stream>>>(p, 1.0, u1b, lam);
-      if ((rc = run_vjp(e, o, p, U0, lam, mu, part))) return rc;
-      k_pacc<<<1, 32, 0, e->stream>>>(-dt, part, pacc);
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, 1.0, u1b, 1.0, u0b);
-      k_axpby<<<bm, 256, 0, e->stream>>>((int64_t)m, -dt, mu, 1.0, u0b);
-      CK(cudaMemcpyAsync(ub, u0b, mb, cudaMemcpyDeviceToDevice, e->stream));
-      e->launches += 12;
+      if ((rc = run_vjp(e, o, p, at(seg, s, 2), lam, mu, part))) return rc;
+      k_rk_rev<3><<<bm, 256, 0, e->stream>>>(p, dt, mu, ub, u2b, u0b, lam, part, pacc);
+      if ((rc = run_vjp(e, o, p, at(seg, s, 1), lam, mu, part))) return rc;
+      k_rk_rev<2><<<bm, 256, 0, e->stream>>>(p, dt, mu, u2b, u1b, u0b, lam, part, pacc);
+      if ((rc = run_vjp(e, o, p, at(seg, s, 0), lam, mu, part))) return rc;
+      k_rk_rev<1><<<bm, 256, 0, e->stream>>>(p, dt, mu, u1b, ub, u0b, lam, part, pacc);
+      e->launches += 3;
     }
   }
   CK(cudaGetLastError());
-  // the handle's state is the final state
-  CK(cudaMemcpyAsync(Un, fin, mb, cudaMemcpyDeviceToDevice, e->stream));
   if (J && (rc = copy_out(e, J, sc, 1))) return rc;
   if (dJdU0 && (rc = copy_out(e, dJdU0, ub, m))) return rc;
   if (dJdp && (rc = copy_out(e, dJdp, pacc, NV))) return rc;
