@@ -144,6 +144,17 @@ __device__ __forceinline__ void ldv(const double* p, double (&o)[2]) {
   o[1] = x.y;
 }
 
+// First statement of a kernel launched by launch_pdl: wait for the kernel
+// before it in the stream (its writes are then visible), then let the next one
+// be scheduled as soon as every block of this one has started, so that launch
+// latencies overlap the kernel before.  Such kernels read what earlier kernels
+// wrote only through pointers without __restrict__: a load known to be
+// invariant could be moved above the wait.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // cells of a tile of k_lsq_set, and the row stride of a shared matrix (whole
 // 16-byte vectors)
 constexpr int SET_TILE = 128;

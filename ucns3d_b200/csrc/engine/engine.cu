@@ -181,17 +181,18 @@ int launch_recon_t(ucg_engine* e, const Problem& p, const double* U) {
   if (c.scheme == 2 && c.iorder == 1) {
     const unsigned blocks = (unsigned)((p.n + 31) / 32);
     const bool vk = c.limiter == 7;
+    cudaError_t err;
     if (c.governing == 1) {
       constexpr int TH = 32 * muscl_warps<true>();
-      if (vk) k_muscl<T, true, true><<<blocks, TH, 0, e->stream>>>(p, U);
-      else k_muscl<T, true, false><<<blocks, TH, 0, e->stream>>>(p, U);
+      if (vk) err = launch_pdl(k_muscl<T, true, true>, blocks, TH, e->stream, p, U);
+      else err = launch_pdl(k_muscl<T, true, false>, blocks, TH, e->stream, p, U);
     } else {
       constexpr int TH = 32 * muscl_warps<false>();
-      if (vk) k_muscl<T, false, true><<<blocks, TH, 0, e->stream>>>(p, U);
-      else k_muscl<T, false, false><<<blocks, TH, 0, e->stream>>>(p, U);
+      if (vk) err = launch_pdl(k_muscl<T, false, true>, blocks, TH, e->stream, p, U);
+      else err = launch_pdl(k_muscl<T, false, false>, blocks, TH, e->stream, p, U);
     }
     e->launches++;
-    CK(cudaGetLastError());
+    CK(err);
     return UCG_OK;
   }
   if (c.iorder < 1 || c.iorder > 4) return fail(e, UCG_EINVAL, "iorder out of range");
@@ -211,44 +212,48 @@ int launch_recon(ucg_engine* e, const Problem& p, const double* U) {
 }
 
 template <typename T, bool NS>
-void launch_faces_t(ucg_engine* e, const Problem& p, const double* Uc) {
+cudaError_t launch_faces_t(ucg_engine* e, const Problem& p, const double* Uc) {
+  cudaError_t err;
   constexpr int FB = UCG_FACE_BLOCK;
   const unsigned fb = (unsigned)((e->nown + FB - 1) / FB);
   switch (e->cfg.riemann) {  // the Riemann solver is a template argument of the face kernel
-    case 2: k_face<T, NS, 2><<<fb, FB, 0, e->stream>>>(p, Uc); break;
-    case 3: k_face<T, NS, 3><<<fb, FB, 0, e->stream>>>(p, Uc); break;
-    case 4: k_face<T, NS, 4><<<fb, FB, 0, e->stream>>>(p, Uc); break;
-    case 5: k_face<T, NS, 5><<<fb, FB, 0, e->stream>>>(p, Uc); break;
-    case 9: k_face<T, NS, 9><<<fb, FB, 0, e->stream>>>(p, Uc); break;
-    default: k_face<T, NS, 1><<<fb, FB, 0, e->stream>>>(p, Uc); break;
+    case 2: err = launch_pdl(k_face<T, NS, 2>, fb, FB, e->stream, p, Uc); break;
+    case 3: err = launch_pdl(k_face<T, NS, 3>, fb, FB, e->stream, p, Uc); break;
+    case 4: err = launch_pdl(k_face<T, NS, 4>, fb, FB, e->stream, p, Uc); break;
+    case 5: err = launch_pdl(k_face<T, NS, 5>, fb, FB, e->stream, p, Uc); break;
+    case 9: err = launch_pdl(k_face<T, NS, 9>, fb, FB, e->stream, p, Uc); break;
+    default: err = launch_pdl(k_face<T, NS, 1>, fb, FB, e->stream, p, Uc); break;
   }
   e->launches += 1;
+  return err;
 }
 
 int launch_faces(ucg_engine* e, const Problem& p, const double* Uc) {
   const bool ns = e->cfg.governing == 1;
-  if (e->mixed) ns ? launch_faces_t<float, true>(e, p, Uc) : launch_faces_t<float, false>(e, p, Uc);
-  else ns ? launch_faces_t<double, true>(e, p, Uc) : launch_faces_t<double, false>(e, p, Uc);
-  CK(cudaGetLastError());
+  const cudaError_t err = e->mixed ? ns ? launch_faces_t<float, true>(e, p, Uc) : launch_faces_t<float, false>(e, p, Uc)
+                                   : ns ? launch_faces_t<double, true>(e, p, Uc) : launch_faces_t<double, false>(e, p, Uc);
+  CK(err);
   return UCG_OK;
 }
 
 // the residual and the update cover cells [0, n_update) (all of them unless
 // a partition's roles step only its owned cells)
 template <bool NS, bool CHK>
-void launch_update_t(ucg_engine* e, const Problem& p0, int mode, const double* Uc, const double* Un, double* Uo,
+cudaError_t launch_update_t(ucg_engine* e, const Problem& p0, int mode, const double* Uc, const double* Un, double* Uo,
                      double dt) {
   Problem p = p0;
   p.n = e->n_update;
   const unsigned blocks = (unsigned)((p.n + UPD_CELLS - 1) / UPD_CELLS);
   constexpr int TH = UPD_CELLS * NV;
+  cudaError_t err;
   switch (mode) {
-    case 0: k_update<NS, 0, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    case 1: k_update<NS, 1, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    case 2: k_update<NS, 2, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
-    default: k_update<NS, 3, CHK><<<blocks, TH, 0, e->stream>>>(p, Uc, Un, Uo, dt); break;
+    case 0: err = launch_pdl(k_update<NS, 0, CHK>, blocks, TH, e->stream, p, Uc, Un, Uo, dt); break;
+    case 1: err = launch_pdl(k_update<NS, 1, CHK>, blocks, TH, e->stream, p, Uc, Un, Uo, dt); break;
+    case 2: err = launch_pdl(k_update<NS, 2, CHK>, blocks, TH, e->stream, p, Uc, Un, Uo, dt); break;
+    default: err = launch_pdl(k_update<NS, 3, CHK>, blocks, TH, e->stream, p, Uc, Un, Uo, dt); break;
   }
   e->launches += 1;
+  return err;
 }
 
 // face fluxes, then the residual (mode 0) or RK stage `mode`; check = false
@@ -258,9 +263,11 @@ int launch_flux(ucg_engine* e, const Problem& p, int mode, const double* Uc, con
   int rc = launch_faces(e, p, Uc);
   if (rc) return rc;
   const bool ns = e->cfg.governing == 1;
-  if (ns) check ? launch_update_t<true, true>(e, p, mode, Uc, Un, Uo, dt) : launch_update_t<true, false>(e, p, mode, Uc, Un, Uo, dt);
-  else check ? launch_update_t<false, true>(e, p, mode, Uc, Un, Uo, dt) : launch_update_t<false, false>(e, p, mode, Uc, Un, Uo, dt);
-  CK(cudaGetLastError());
+  const cudaError_t err = ns ? check ? launch_update_t<true, true>(e, p, mode, Uc, Un, Uo, dt)
+                                     : launch_update_t<true, false>(e, p, mode, Uc, Un, Uo, dt)
+                             : check ? launch_update_t<false, true>(e, p, mode, Uc, Un, Uo, dt)
+                                     : launch_update_t<false, false>(e, p, mode, Uc, Un, Uo, dt);
+  CK(err);
   return UCG_OK;
 }
 

@@ -78,7 +78,8 @@ __device__ __forceinline__ void flux_jacobian(const double* q, double gamma, dou
 }
 
 // CALCULATE_CFLL: the local time step of every cell
-__global__ void k_imp_dtl(Problem p, const double* __restrict__ U, double ccfl, double* __restrict__ dtl) {
+__global__ void k_imp_dtl(Problem p, const double* U, double ccfl, double* dtl) {
+  pdl_begin();
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p.n) return;
   double pr[NV];
@@ -109,9 +110,9 @@ __device__ __forceinline__ int64_t off_at(int64_t c, int f, int ij) {
 // divide and square-root sequences of a face and the 1.2 KB of blocks a cell
 // writes, which one thread per cell did face after face in rows of 1,200-byte
 // stride.  28,810 cells: 29.8 -> 11.9 us.
-__global__ void __launch_bounds__(32 * MF) k_imp_jac(Problem p, const double* __restrict__ U,
-                                                     const double* __restrict__ dtl, double dt,
-                                                     double* __restrict__ dinv, double* __restrict__ off) {
+__global__ void __launch_bounds__(32 * MF) k_imp_jac(Problem p, const double* U, const double* dtl, double dt,
+                                                     double* dinv, double* off) {
+  pdl_begin();
   __shared__ double s_v[MF][32];
   const int lane = threadIdx.x & 31, f = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + lane;
@@ -177,11 +178,10 @@ __global__ void __launch_bounds__(32 * MF) k_imp_jac(Problem p, const double* __
 // thread per cell and 1,200-byte rows every load touched 32 sectors.  28,810
 // cells: 15.3 -> 8.2 us.
 template <bool FIRST>
-__global__ void __launch_bounds__(32 * NV) k_imp_sweep(Problem p, const double* __restrict__ dinv,
-                                                       const double* __restrict__ off, const double* __restrict__ du,
-                                                       double* __restrict__ dn, const double* __restrict__ U1,
-                                                       const double* __restrict__ U2, const double* __restrict__ U3,
-                                                       double dt) {
+__global__ void __launch_bounds__(32 * NV) k_imp_sweep(Problem p, const double* dinv, const double* off,
+                                                       const double* du, double* dn, const double* U1,
+                                                       const double* U2, const double* U3, double dt) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + lane;
   if (c >= p.n) return;
@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(32 * NV) k_imp_sweep(Problem p, const double* 
   dn[ci] = dinv[c] * b;
 }
 
-__global__ void k_imp_add(Problem p, double* __restrict__ U, const double* __restrict__ du) {
+__global__ void k_imp_add(Problem p, double* U, const double* du) {
+  pdl_begin();
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p.n) return;
   bool bad = false;
@@ -285,14 +286,14 @@ int implicit_correction(ucg_engine* e, const Problem& p, double* U, double ccfl,
   int rc;
   if ((rc = launch_recon(e, p, U))) return rc;
   if ((rc = launch_flux(e, p, 0, U, U, nullptr, 0.0))) return rc;
-  if (local_steps) k_imp_dtl<<<blocks, 128, 0, e->stream>>>(p, U, ccfl, dtl);
+  if (local_steps) CK(launch_pdl(k_imp_dtl, blocks, 128, e->stream, p, U, ccfl, dtl));
   const unsigned groups = (unsigned)((n + 31) / 32);
-  k_imp_jac<<<groups, 32 * MF, 0, e->stream>>>(p, U, dtl, dt, dinv, off);
+  CK(launch_pdl(k_imp_jac, groups, 32 * MF, e->stream, p, U, dtl, dt, dinv, off));
   const double* U1 = U2 ? U : nullptr;
   int k = 0;  // the first sweep starts from du = 0
-  k_imp_sweep<true><<<groups, 32 * NV, 0, e->stream>>>(p, dinv, off, du[1], du[0], U1, U2, U3, dt);
+  CK(launch_pdl(k_imp_sweep<true>, groups, 32 * NV, e->stream, p, dinv, off, du[1], du[0], U1, U2, U3, dt));
   for (int32_t sw = 1; sw < nsweeps; ++sw) {
-    k_imp_sweep<false><<<groups, 32 * NV, 0, e->stream>>>(p, dinv, off, du[k], du[k ^ 1], U1, U2, U3, dt);
+    CK(launch_pdl(k_imp_sweep<false>, groups, 32 * NV, e->stream, p, dinv, off, du[k], du[k ^ 1], U1, U2, U3, dt));
     k ^= 1;
   }
   e->launches += 2 + nsweeps;
@@ -328,7 +329,7 @@ extern "C" int ucg_implicit_step(ucg_engine* e, double cfl, int32_t nsteps, int3
   for (int32_t s = 0; s < nsteps; ++s) {
     int cur;
     if ((rc = implicit_correction(e, p, U, cfl / 3.0, nsweeps, 0.0, nullptr, nullptr, &cur))) return rc;
-    k_imp_add<<<blocks, 128, 0, e->stream>>>(p, U, (double*)e->imp_du.p + cur * e->n * NV);
+    CK(launch_pdl(k_imp_add, blocks, 128, e->stream, p, U, (double*)e->imp_du.p + cur * e->n * NV));
     e->launches++;
     CK(cudaGetLastError());
   }
@@ -371,7 +372,7 @@ extern "C" int ucg_dual_time_step(ucg_engine* e, double dt, double cfl, int32_t 
     e->dual_ready = true;
   }
   const unsigned blocks = (unsigned)((n + 127) / 128);
-  k_imp_dtl<<<blocks, 128, 0, e->stream>>>(p, U, cfl / 3.0, (double*)e->imp_dtl.p);
+  CK(launch_pdl(k_imp_dtl, blocks, 128, e->stream, p, U, cfl / 3.0, (double*)e->imp_dtl.p));
   e->launches++;
   double firsti = 0.0;
   int32_t jj = 0;
@@ -382,7 +383,7 @@ extern "C" int ucg_dual_time_step(ucg_engine* e, double dt, double cfl, int32_t 
     const double* du = (const double*)e->imp_du.p + cur * n * NV;
     k_imp_norm_part<<<(unsigned)nblk, 256, 0, e->stream>>>(p, du, part);
     k_imp_norm_sum<<<1, 1, 0, e->stream>>>(part, nblk, part + nblk);
-    k_imp_add<<<blocks, 128, 0, e->stream>>>(p, U, du);
+    CK(launch_pdl(k_imp_add, blocks, 128, e->stream, p, U, du));
     e->launches += 3;
     double res = 0.0;
     CK(cudaMemcpyAsync(&res, part + nblk, 8, cudaMemcpyDeviceToHost, e->stream));
@@ -468,7 +469,7 @@ extern "C" int ucg_dual_time_step_explicit(ucg_engine* e, double dt, double cfl,
     e->dual_ready = true;
   }
   const unsigned blocks = (unsigned)((n + 127) / 128);
-  k_imp_dtl<<<blocks, 128, 0, e->stream>>>(p, U, cfl / 3.0, dtl);
+  CK(launch_pdl(k_imp_dtl, blocks, 128, e->stream, p, U, cfl / 3.0, dtl));
   e->launches++;
   double firsti = 0.0;
   int32_t jj = 0;
@@ -478,7 +479,7 @@ extern "C" int ucg_dual_time_step_explicit(ucg_engine* e, double dt, double cfl,
     k_dtex_du<<<blocks, 128, 0, e->stream>>>(p, U, U2, U3, dtl, dt, du);
     k_imp_norm_part<<<(unsigned)nblk, 256, 0, e->stream>>>(p, du, part);
     k_imp_norm_sum<<<1, 1, 0, e->stream>>>(part, nblk, part + nblk);
-    k_imp_add<<<blocks, 128, 0, e->stream>>>(p, U, du);
+    CK(launch_pdl(k_imp_add, blocks, 128, e->stream, p, U, du));
     e->launches += 4;
     double res = 0.0;
     CK(cudaMemcpyAsync(&res, part + nblk, 8, cudaMemcpyDeviceToHost, e->stream));

@@ -37,7 +37,8 @@ __host__ __device__ constexpr int muscl_warps() {
   return NS ? NV + 4 : NV;
 }
 template <typename T, bool NS, bool VK>
-__global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Problem p, const double* __restrict__ U) {
+__global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Problem p, const double* U) {
+  pdl_begin();
   constexpr int NW = muscl_warps<NS>();
   constexpr int MC = 8;  // members per pass of the primitive records
   __shared__ double s_d[MF * NV][33];
@@ -187,7 +188,8 @@ __global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Pr
 // CWENO4 57.3 -> 56.2 ms; eight (128 registers) gained less.  Euler keeps
 // the compiler's choice (eight blocks changed the 64^3 WENO5 step by 0.5 %).
 template <typename T, bool NS, int RK>
-__global__ void __launch_bounds__(UCG_FACE_BLOCK, NS ? 6 : 1) k_face(Problem p, const double* __restrict__ Uc) {
+__global__ void __launch_bounds__(UCG_FACE_BLOCK, NS ? 6 : 1) k_face(Problem p, const double* Uc) {
+  pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.nown) return;
   const int32_t code = p.own[i];
@@ -322,8 +324,9 @@ __device__ __forceinline__ double cfl_dt(const Problem& p, const double* pr, dou
 // k_dt_init and a k_cfl launch; the first stage resets that slot.
 constexpr int UPD_CELLS = 32;
 template <bool NS, int MODE, bool CHK = true>
-__global__ void __launch_bounds__(UPD_CELLS * NV) k_update(Problem p, const double* __restrict__ Uc, const double* Un,
+__global__ void __launch_bounds__(UPD_CELLS * NV) k_update(Problem p, const double* Uc, const double* Un,
                                                            double* Uout, double dt_host) {
+  pdl_begin();
   __shared__ double s_u[UPD_CELLS * NV];
   const int tid = threadIdx.x, cl = tid / NV, v = tid - cl * NV;
   const int64_t c0 = (int64_t)blockIdx.x * UPD_CELLS, c = c0 + cl, i = c0 * NV + tid;
