@@ -178,8 +178,8 @@ def load_peaks():
 # Only measured entries are listed; other workloads report traffic null.  The
 # traffic grows in proportion to the cells, so a launch on a larger mesh of the
 # same workload moves this times its cells.
-#   vortex_hex_weno5, mixed: 32^3 capture of k_lsq_set (97.6 + 113.9 MB)
-LSQ_DRAM_BYTES_PER_CELL = {("vortex_hex_weno5", 1): 6_456}
+#   vortex_hex_weno5, mixed: 32^3 capture of k_lsq_set (97.2 + 105.4 MB)
+LSQ_DRAM_BYTES_PER_CELL = {("vortex_hex_weno5", 1): 6_182}
 
 
 def lsq_bytes_per_cell(cfg, sets_per_cell=1.0):
@@ -244,9 +244,13 @@ def recon_kernels(cfg, wenwrt):
     """The kernels of one reconstruction (the launch sequence of launch_weno)."""
     if cfg.scheme == 2 and cfg.iorder == 1:
         return "k_muscl"
-    if cfg.scheme == 3 and cfg.iorder == 4 and wenwrt == 1:
+    if cfg.scheme == 3 and wenwrt == 2:
+        return "least squares + k_char_forms + k_char_face + k_wpost fall-back"
+    if cfg.scheme == 3 and cfg.iorder == 4:
         return "least squares + indicators + k_wface + k_wpost fall-back"
-    return "least squares + k_wpost"
+    if cfg.scheme == 3 and cfg.iorder < 3:
+        return "least squares + k_wface + k_wpost fall-back"
+    return "least squares + k_wpost (small meshes at IORDER 3: k_wface)"
 
 
 L2_BYTES = 126 * 2 ** 20
