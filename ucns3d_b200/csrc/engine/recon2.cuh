@@ -1339,13 +1339,40 @@ __global__ void k_visc_prim(Problem p, const double* __restrict__ U) {
 // form FP32 on the differences of (T, u, v, w) from the cell's own, like
 // the stencil least squares of the conserved variables (all four variables
 // in one pass there).
-template <int P, typename T>
-__global__ void __launch_bounds__(128) k_visc_lsq(Problem p, const double* __restrict__ U) {
+// SET: a block takes a tile of cells that share a matrix set (plan_sets) and
+// reads stencil 1's rows from shared memory as 16-byte broadcasts instead of
+// streaming every cell's copy from DRAM, with the records of VG members in
+// flight; the same sums in the same order.  The first blocks take the groups
+// that the tiles leave (p.ugrp), whose few lanes' chain of loads runs beside
+// the tiles.  271,872 cells, CWENO4 mixed form: 0.270 -> 0.149 ms (0.167 at three
+// blocks per SM, 0.229 at five with two members in flight; the groups left in
+// a launch of their own 0.056 more).
+template <int P, typename T, bool SET = false>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 && P <= 3 ? 4 : 1) k_visc_lsq(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int VP = sizeof(T) == 4 || ID * 4 <= 80 ? 4 : 2;  // variables per pass
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.n) return;
+  constexpr int RS = set_stride<T>(ID), VEC = Vec<T>::N, VG = 4;
+  extern __shared__ __align__(16) unsigned char vl_smem[];
+  const T* s = (const T*)vl_smem;
   const int IM = p.imax, W = IM + 1;
+  const unsigned nown = SET ? (unsigned)((p.nugrp + 3) / 4) : 0;
+  const bool tiled = SET && blockIdx.x >= nown;
+  int64_t c;
+  if (tiled) {
+    const int64_t tile = blockIdx.x - nown;
+    const float4* src = (const float4*)((const T*)p.setmat + p.tset[tile] * p.sstride + p.sso[0]);
+    for (int i = threadIdx.x; i < IM * RS / VEC; i += SET_TILE) ((float4*)vl_smem)[i] = src[i];
+    __syncthreads();
+    c = p.tcell[tile * SET_TILE + threadIdx.x];
+    if (c < 0) return;
+  } else {
+    c = (int64_t)blockIdx.x * 128 + threadIdx.x;
+    if (SET) {
+      if ((c >> 5) >= p.nugrp) return;
+      c = (int64_t)p.ugrp[c >> 5] * 32 + (c & 31);
+    }
+    if (c >= p.n) return;
+  }
   double pm[NV];
   cons2prim(p.gamma, U + c * NV, pm);
   const double s0[4] = {pm[4] / (pm[0] * p.r_gas), pm[1], pm[2], pm[3]};
@@ -1361,18 +1388,48 @@ __global__ void __launch_bounds__(128) k_visc_lsq(Problem p, const double* __res
     for (int d = 0; d < ID; ++d)
 #pragma unroll
       for (int j = 0; j < VP; ++j) acc[d][j] = T(0);
-    for (int k = 0; k < IM; ++k) {
-      const double2* q = (const double2*)(p.prim + (int64_t)st[(k + 1) * 32] * 4);
-      const double2 qa = q[0], qb = q[1];
-      const double sy[4] = {qa.x, qa.y, qb.x, qb.y};
-      T ds[VP];
+    if (tiled) {
+      for (int k0 = 0; k0 < IM; k0 += VG) {
+        double2 qa[VG], qb[VG];
 #pragma unroll
-      for (int j = 0; j < VP; ++j) ds[j] = T(sy[v0 + j] - s0[v0 + j]);
+        for (int i = 0; i < VG; ++i) {
+          const int k = k0 + i < IM ? k0 + i : IM - 1;
+          const double2* q = (const double2*)(p.prim + (int64_t)st[(k + 1) * 32] * 4);
+          qa[i] = q[0], qb[i] = q[1];
+        }
 #pragma unroll
-      for (int d = 0; d < ID; ++d) {
-        const T m = M[(k * ID + d) * 32];
+        for (int i = 0; i < VG; ++i)
+          if (k0 + i < IM) {
+            const double sy[4] = {qa[i].x, qa[i].y, qb[i].x, qb[i].y};
+            T ds[VP];
 #pragma unroll
-        for (int j = 0; j < VP; ++j) acc[d][j] += m * ds[j];
+            for (int j = 0; j < VP; ++j) ds[j] = T(sy[v0 + j] - s0[v0 + j]);
+#pragma unroll
+            for (int q = 0; q < RS / VEC; ++q) {
+              T m[VEC];
+              ldv(s + (k0 + i) * RS + q * VEC, m);
+#pragma unroll
+              for (int r = 0; r < VEC; ++r)
+                if (q * VEC + r < ID)
+#pragma unroll
+                  for (int j = 0; j < VP; ++j) acc[q * VEC + r][j] += m[r] * ds[j];
+            }
+          }
+      }
+    } else {
+      for (int k = 0; k < IM; ++k) {
+        const double2* q = (const double2*)(p.prim + (int64_t)st[(k + 1) * 32] * 4);
+        const double2 qa = q[0], qb = q[1];
+        const double sy[4] = {qa.x, qa.y, qb.x, qb.y};
+        T ds[VP];
+#pragma unroll
+        for (int j = 0; j < VP; ++j) ds[j] = T(sy[v0 + j] - s0[v0 + j]);
+#pragma unroll
+        for (int d = 0; d < ID; ++d) {
+          const T m = M[(k * ID + d) * 32];
+#pragma unroll
+          for (int j = 0; j < VP; ++j) acc[d][j] += m * ds[j];
+        }
       }
     }
     // 16-byte stores: a row's four FP32 values, or FP64 pairs (VP even;
@@ -1448,8 +1505,15 @@ __device__ __forceinline__ void visc_point_grad(const Problem& p, int64_t c, int
   }
 }
 
+// Without bounds the compiler keeps to the 64 registers of a 1,024-thread
+// block: WENO5 FP64 (8,000 cells) spilled, reconstruction after the least
+// squares 3.13 -> 0.25 ms, WENO5 mixed (13,824) 0.57 -> 0.21, CWENO4 FP64
+// (271,872) 2.30 -> 2.07.  Blocks per SM: FP32 8 (CWENO4, 271,872 cells: 0.388 ms
+// at one, 0.330 at six, 0.314 at eight, 0.360 at ten), FP64 5 (WENO5 0.244 to
+// 0.247 ms at three to five, 0.270 at eight; CWENO4 2.14, 2.09, 2.07, 2.06 at
+// three, four, five and eight).
 template <int P, typename T>
-__global__ void k_visc_facegrad(Problem p) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 5) k_visc_facegrad(Problem p) {
   const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = t / QS;
@@ -1893,7 +1957,13 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
   ++*launches;
   if (ns) {
     k_visc_prim<P, T><<<(unsigned)((pa.n + 255) / 256), 256, 0, st>>>(pa, U);
-    k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
+    if (p.ntile) {
+      const size_t rows = (size_t)p.imax * set_stride<T>(Deg<P>::ideg) * sizeof(T);
+      cudaFuncSetAttribute(k_visc_lsq<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
+      k_visc_lsq<P, T, true><<<(unsigned)((p.nugrp + 3) / 4 + p.ntile), 128, rows, st>>>(p, U);
+    } else {
+      k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
+    }
     *launches += 2;
     const int64_t nfp = p.nown * QS;
     k_visc_facegrad<P, T><<<(unsigned)((nfp + 127) / 128), 128, 0, st>>>(p);
