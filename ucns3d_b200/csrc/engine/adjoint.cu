@@ -522,30 +522,23 @@ struct FwdStore {
   double* d;
   int8_t* b;
   int64_t n;
-  __device__ void put(int64_t c, const MusclFwd& m) const {
-    int j = 0;
+  // variable v's fields (k_adj_fwd; the other fields have one writer each)
+  __device__ void put(int64_t c, int v, double u0, const double (&g)[3], double lo, double hi, double slope, int amin,
+                      int amax, int fstar) const {
+    d[v * n + c] = u0;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) d[(j++) * n + c] = m.u0[v];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) d[(j++) * n + c] = m.g[k][v];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      d[(j++) * n + c] = m.lo[v];
-      d[(j++) * n + c] = m.hi[v];
-      d[(j++) * n + c] = m.slope[v];
-    }
-    d[j * n + c] = m.epsi2;
-    j = 0;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      b[(j++) * n + c] = (int8_t)m.amin[v];
-      b[(j++) * n + c] = (int8_t)m.amax[v];
-      b[(j++) * n + c] = (int8_t)m.fstar[v];
-    }
-    b[(j++) * n + c] = (int8_t)m.first;
-    b[j * n + c] = (int8_t)m.fmask;
+    for (int k = 0; k < 3; ++k) d[(NV + k * NV + v) * n + c] = g[k];
+    d[(4 * NV + 3 * v) * n + c] = lo;
+    d[(4 * NV + 3 * v + 1) * n + c] = hi;
+    d[(4 * NV + 3 * v + 2) * n + c] = slope;
+    b[3 * v * n + c] = (int8_t)amin;
+    b[(3 * v + 1) * n + c] = (int8_t)amax;
+    b[(3 * v + 2) * n + c] = (int8_t)fstar;
+  }
+  __device__ void put_epsi2(int64_t c, double e) const { d[(int64_t)(FWD_D - 1) * n + c] = e; }
+  __device__ void put_cell(int64_t c, bool first, int fmask) const {
+    b[3 * NV * n + c] = (int8_t)first;
+    b[(3 * NV + 1) * n + c] = (int8_t)fmask;
   }
   __device__ void get(int64_t c, MusclFwd& m) const {
     int j = 0;
@@ -588,175 +581,151 @@ __device__ __forceinline__ double muscl_dd(const MusclFwd& m, const double* b, i
   return (m.u0[v] + res) - m.u0[v];
 }
 
-__device__ void muscl_forward(const Problem& p, const double* __restrict__ U, int64_t c, MusclFwd& m) {
-  const int IM = p.imax, W = IM + 1, nf = p.nfaces[c];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) m.u0[v] = U[c * NV + v];
-  const int64_t grp = c >> 5;
-  const int lane = (int)(c & 31);
-  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + lane;
-  const double* M = (const double*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + lane;
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-#pragma unroll
-    for (int v = 0; v < NV; ++v) m.g[d][v] = 0.0;
-  for (int k = 0; k < IM; ++k) {
-    const int64_t y = st[(k + 1) * 32];
-    const double m0 = M[(k * 3 + 0) * 32], m1 = M[(k * 3 + 1) * 32], m2 = M[(k * 3 + 2) * 32];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double du = U[y * NV + v] - m.u0[v];
-      m.g[0][v] += m0 * du;
-      m.g[1][v] += m1 * du;
-      m.g[2][v] += m2 * du;
-    }
-  }
-  double mn[NV], mx[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    mn[v] = mx[v] = m.u0[v];
-    m.amin[v] = m.amax[v] = 0;
-  }
-  for (int f = 0; f < nf; ++f) {
-    const int64_t nb = p.neigh[c * MF + f];
-    if (nb < 0) continue;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double un = U[nb * NV + v];
-      if (un < mn[v]) {
-        mn[v] = un;
-        m.amin[v] = 1 + IM + f;
-      }
-      if (un > mx[v]) {
-        mx[v] = un;
-        m.amax[v] = 1 + IM + f;
-      }
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    m.lo[v] = mn[v] - m.u0[v];
-    m.hi[v] = mx[v] - m.u0[v];
-  }
-  const double e3 = p.kappa_ven * p.minedge[c];
-  m.epsi2 = e3 * e3 * e3;
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    m.slope[v] = TOLBIG;
-    m.fstar[v] = -1;
-  }
-  for (int f = 0; f < nf; ++f) {
-    double b[3];
-    muscl_basis(p, c, f, b);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double ps = venkat(muscl_dd(m, b, v), m.lo[v], m.hi[v], m.epsi2);
-      if (ps < m.slope[v]) {
-        m.slope[v] = ps;
-        m.fstar[v] = f;
-      }
-    }
-  }
-  double pm[NV];
-  cons2prim(p.gamma, m.u0, pm);
-  m.first = false;
-  for (int f = 0; f < nf; ++f) {
-    double b[3], uf[NV];
-    muscl_basis(p, c, f, b);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) uf[v] = m.u0[v] + muscl_dd(m, b, v) * m.slope[v];
-    m.first = m.first || jump_bad(p.gamma, pm, uf, 0.95);
-  }
-}
-
-// Navier-Stokes: the cell's gradient of (T, u, v, w) ([T, u, v, w][x, y,
-// z]) from the viscous least squares on stencil 1 and the frame (AINVJT),
-// in the operations and order of k_muscl's viscous part (gradients.f90:
-// 502-706, SOLUTIONTRIAV2): the cell's record of ulv.
-__device__ __forceinline__ void visc_cell_gradient(const Problem& p, const double* __restrict__ U, int64_t c,
-                                                   double* gr) {
-  const int IM = p.imax, W = IM + 1;
-  double u0[NV], pm[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) u0[v] = U[c * NV + v];
-  cons2prim(p.gamma, u0, pm);
-  const double t0 = pm[4] / (pm[0] * p.r_gas);
-  const int64_t grp = c >> 5;
-  const int lane = (int)(c & 31);
-  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + lane;
-  const double* M = (const double*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + lane;
-  double gvv[3][4] = {};
-  for (int k = 0; k < IM; ++k) {
-    const int64_t y = st[(k + 1) * 32];
-    double uy[NV], py[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) uy[v] = U[y * NV + v];
-    const double m0 = M[(k * 3 + 0) * 32], m1 = M[(k * 3 + 1) * 32], m2 = M[(k * 3 + 2) * 32];
-    cons2prim(p.gamma, uy, py);
-    const double ds[4] = {py[4] / (py[0] * p.r_gas) - t0, py[1] - pm[1], py[2] - pm[2], py[3] - pm[3]};
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      gvv[0][v] += m0 * ds[v];
-      gvv[1][v] += m1 * ds[v];
-      gvv[2][v] += m2 * ds[v];
-    }
-  }
-  const double* J = p.jinv + c * 9;
-#pragma unroll
-  for (int v = 0; v < 4; ++v)
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      gr[v * 3 + k] = J[0 * 3 + k] * gvv[0][v] + J[1 * 3 + k] * gvv[1][v] + J[2 * 3 + k] * gvv[2][v];
-}
-
 // The reconstruction of every cell with its intermediates kept for the
 // reverse sweep: face values (minus the mean) to dul exactly as k_muscl
 // writes them, the MusclFwd record to fwd[c]; for Navier-Stokes the cell's
-// viscous gradient to ulv (read by k_adj_visc).
+// gradient of (T, u, v, w) ([T, u, v, w][x, y, z]) to ulv (read by
+// k_adj_visc).
 // A face neighbour that is also a cell of the stencil shares the stencil
 // cell's slot: the bound slots amin/amax are remapped to it, and fmask keeps
 // the faces whose neighbour has a slot of its own (the reverse map in
 // adj_setup makes the same choice).
-__global__ void __launch_bounds__(128) k_adj_fwd(Problem p, const double* __restrict__ U, FwdStore fwd) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.n) return;
-  MusclFwd m;
-  muscl_forward(p, U, c, m);
-  const int IM = p.imax, nf = p.nfaces[c];
-  double* out = (double*)p.dul + c * (int64_t)MF * NV;
-  for (int f = 0; f < nf; ++f) {
-    double b[3];
-    muscl_basis(p, c, f, b);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) out[f * NV + v] = m.first ? 0.0 : muscl_dd(m, b, v) * m.slope[v];
+// Latency-bound, so laid out as k_muscl: a 32-cell group per block, one warp
+// per variable (and per variable of the viscous gradient), the faces' slots
+// and CHECKSOLX shared out over the warps; the same operations in the same
+// order per value.  One lane per cell with all variables took 92 us
+// (115,260 cells, Navier-Stokes) and 23.2 us (28,810, Euler); this 85 and 14.4 us
+// (at the compiler's 64 registers 96 and 18.3).
+template <bool NS>
+__global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_adj_fwd(Problem p, const double* __restrict__ U,
+                                                                                FwdStore fwd) {
+  constexpr int NW = muscl_warps<NS>();
+  constexpr int MC = 8;  // members per pass of the primitive records
+  __shared__ double s_d[MF * NV][33];
+  __shared__ double s_p[NS ? MC + 1 : 1][4][32];
+  __shared__ int s_first[32], s_nf[32], s_slot[MF][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t grp = blockIdx.x, g0 = grp * 32;
+  const int ncl = p.n - g0 < 32 ? (int)(p.n - g0) : 32;  // cells of this group
+  const int ln = lane < ncl ? lane : ncl - 1;            // spare lanes repeat the last cell
+  const int64_t c = g0 + ln;
+  const bool live = lane < ncl;
+  const int IM = p.imax, W = IM + 1, QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + ln;
+  const double* M = (const double*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + ln;
+  const int nf = p.nfaces[c];
+  if (w == 0) {
+    s_first[lane] = 0;
+    s_nf[lane] = nf;
   }
-  const int32_t* st = p.sten + (c >> 5) * (int64_t)p.admis_max * (IM + 1) * 32 + (c & 31);
-  int slot_of[MF];
-  m.fmask = 0;
-  for (int f = 0; f < MF; ++f) {
-    const int64_t nb = f < nf ? p.neigh[c * MF + f] : -1;
-    slot_of[f] = 1 + IM + f;
-    if (nb < 0) continue;
-    for (int k = 0; k < IM; ++k)
-      if (st[(k + 1) * 32] == nb) {
-        slot_of[f] = 1 + k;
-        break;
+  if (NS) {
+    double gv[3] = {0.0, 0.0, 0.0};
+    for (int k0 = 0; k0 < IM; k0 += MC) {
+      if (k0) __syncthreads();  // the last pass's records have been read
+      const int j = k0 + w - 1;
+      if (w == 0 ? k0 == 0 : w <= MC && j < IM) {  // warp 0: the cell itself
+        const double* uy = U + (w == 0 ? c : (int64_t)st[(j + 1) * 32]) * NV;
+        double u[NV], py[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) u[v] = uy[v];
+        cons2prim(p.gamma, u, py);
+        s_p[w][0][lane] = py[4] / (py[0] * p.r_gas);
+#pragma unroll
+        for (int v = 1; v < 4; ++v) s_p[w][v][lane] = py[v];
       }
-    if (slot_of[f] == 1 + IM + f) m.fmask |= 1 << f;
-  }
+      __syncthreads();
+      if (w >= NV) {
+        const double t0 = s_p[0][w - NV][lane];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (m.amin[v] > IM) m.amin[v] = slot_of[m.amin[v] - 1 - IM];
-    if (m.amax[v] > IM) m.amax[v] = slot_of[m.amax[v] - 1 - IM];
-  }
-  fwd.put(c, m);
-  if (p.governing == 1) {
-    double gr[12];
-    visc_cell_gradient(p, U, c, gr);
-    const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-    double* o = p.ulv + c * (int64_t)QS * 12;
+        for (int i = 0; i < MC; ++i)
+          if (k0 + i < IM) {
+            const double ds = s_p[i + 1][w - NV][lane] - t0;
 #pragma unroll
-    for (int j = 0; j < 12; ++j) o[j] = gr[j];
+            for (int d = 0; d < 3; ++d) gv[d] += M[((k0 + i) * 3 + d) * 32] * ds;
+          }
+      }
+    }
+    if (w >= NV && live) {
+      const double* J = p.jinv + c * 9;
+      double* o = p.ulv + c * (int64_t)QS * 12 + (w - NV) * 3;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) o[k] = J[0 * 3 + k] * gv[0] + J[1 * 3 + k] * gv[1] + J[2 * 3 + k] * gv[2];
+    }
+  }
+  // the slot of each face's neighbour (-1: a physical face)
+  for (int f = NW - 1 - w; f < MF; f += NW) {
+    const int nb = f < nf ? p.neigh[c * MF + f] : -1;
+    int s = nb < 0 ? -1 : 1 + IM + f;
+    for (int k = IM; k-- > 0;)
+      if (nb >= 0 && st[(k + 1) * 32] == nb) s = 1 + k;
+    s_slot[f][lane] = s;
+  }
+  double u0 = 0.0, g[3] = {0.0, 0.0, 0.0}, lo = 0.0, hi = 0.0, slope = TOLBIG;
+  int amin = -1, amax = -1, fstar = -1;  // faces of the bounds (-1: the cell) and of the least slope
+  if (w < NV) {
+    u0 = U[c * NV + w];
+#pragma unroll 8
+    for (int k = 0; k < IM; ++k) {
+      const double du = U[(int64_t)st[(k + 1) * 32] * NV + w] - u0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) g[d] += M[(k * 3 + d) * 32] * du;
+    }
+    lo = hi = u0;
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      const int nb = f < nf ? p.neigh[c * MF + f] : -1;
+      const double un = nb >= 0 ? U[(int64_t)nb * NV + w] : u0;
+      if (un < lo) lo = un, amin = f;
+      if (un > hi) hi = un, amax = f;
+    }
+    lo -= u0;
+    hi -= u0;
+    const double ke = p.kappa_ven * p.minedge[c];
+    const double epsi2 = ke * ke * ke;
+    if (w == 0 && live) fwd.put_epsi2(c, epsi2);
+    double dd[MF];
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      dd[f] = 0.0;
+      if (f < nf) {
+        double b[3];
+        muscl_basis(p, c, f, b);
+        const double res = b[0] * g[0] + b[1] * g[1] + b[2] * g[2];
+        dd[f] = (u0 + res) - u0;
+        const double ps = venkat(dd[f], lo, hi, epsi2);
+        if (ps < slope) slope = ps, fstar = f;
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < MF; ++f) s_d[f * NV + w][lane] = dd[f] * slope;
+  }
+  __syncthreads();
+  if (w < NV && live)
+    fwd.put(c, w, u0, g, lo, hi, slope, amin < 0 ? 0 : s_slot[amin][lane], amax < 0 ? 0 : s_slot[amax][lane], fstar);
+  {  // CHECKSOLX on the limited face values
+    double um[NV], pm[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) um[v] = U[c * NV + v];
+    cons2prim(p.gamma, um, pm);
+    for (int f = w; f < nf; f += NW) {
+      double uf[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) uf[v] = um[v] + s_d[f * NV + v][lane];
+      if (jump_bad(p.gamma, pm, uf, 0.95)) s_first[lane] = 1;
+    }
+  }
+  __syncthreads();
+  if (w == NW - 1 && live) {
+    int fmask = 0;
+    for (int f = 0; f < MF; ++f)
+      if (s_slot[f][lane] == 1 + IM + f) fmask |= 1 << f;
+    fwd.put_cell(c, s_first[lane] != 0, fmask);
+  }
+  const int r = lane, f = r / NV;
+  if (r < MF * NV) {
+    double* out = (double*)p.dul + g0 * MF * NV + r;
+    for (int cl = w; cl < ncl; cl += NW)
+      if (f < s_nf[cl]) out[cl * MF * NV] = s_first[cl] ? 0.0 : s_d[r][cl];
   }
 }
 
@@ -939,129 +908,144 @@ struct Dp5 {
 // which are the reconstruction itself, go out as k_muscl writes it (in place
 // of a k_muscl launch): the face values to dul and, with tgr, the cell's
 // viscous gradient to ulv (read by k_jvp_face).
-__global__ void __launch_bounds__(128) k_jvp_muscl(Problem p, const double* __restrict__ U,
-                                                   const double* __restrict__ dU, double* __restrict__ tdul,
-                                                   double* __restrict__ tgr, bool base) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.n) return;
+// One warp per variable of a 32-cell group, as k_muscl and k_adj_fwd
+// (NS: with tgr).  One lane per cell with all variables (204 registers, eight
+// warps per SM) took 160 us (115,260 cells, Navier-Stokes); this 134 us (at the
+// compiler's 92 registers 162).
+template <bool NS>
+__global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 3 : 5)
+    k_jvp_muscl(Problem p, const double* __restrict__ U, const double* __restrict__ dU, double* __restrict__ tdul,
+                double* __restrict__ tgr, bool base) {
   using D = Dual<1>;
-  const int IM = p.imax, W = IM + 1, nf = p.nfaces[c];
-  const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-  D u0[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    u0[v] = D(U[c * NV + v]);
-    u0[v].d[0] = dU[c * NV + v];
-  }
-  const int64_t grp = c >> 5;
-  const int lane = (int)(c & 31);
-  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + lane;
-  const double* M = (const double*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + lane;
-  D g[3][NV], gvv[3][4];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) g[d][v] = D(0.0);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) gvv[d][a] = D(0.0);
-  }
-  D s0[4];
-  if (tgr) {
-    D pm0[NV];
-    cons2prim(p.gamma, u0, pm0);
-    s0[0] = pm0[4] / (pm0[0] * p.r_gas);
-    s0[1] = pm0[1];
-    s0[2] = pm0[2];
-    s0[3] = pm0[3];
-  }
-  for (int k = 0; k < IM; ++k) {
-    const int64_t y = st[(k + 1) * 32];
-    const double m0 = M[(k * 3 + 0) * 32], m1 = M[(k * 3 + 1) * 32], m2 = M[(k * 3 + 2) * 32];
-    D uy[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      uy[v] = D(U[y * NV + v]);
-      uy[v].d[0] = dU[y * NV + v];
-      const D du = uy[v] - u0[v];
-      g[0][v] = g[0][v] + m0 * du;
-      g[1][v] = g[1][v] + m1 * du;
-      g[2][v] = g[2][v] + m2 * du;
-    }
-    if (tgr) {
-      D py[NV];
-      cons2prim(p.gamma, uy, py);
-      const D ds[4] = {py[4] / (py[0] * p.r_gas) - s0[0], py[1] - s0[1], py[2] - s0[2], py[3] - s0[3]};
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        gvv[0][a] = gvv[0][a] + m0 * ds[a];
-        gvv[1][a] = gvv[1][a] + m1 * ds[a];
-        gvv[2][a] = gvv[2][a] + m2 * ds[a];
-      }
-    }
-  }
-  if (tgr) {
-    const double* Jc = p.jinv + c * 9;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int kk = 0; kk < 3; ++kk) {
-        const D t = Jc[0 * 3 + kk] * gvv[0][a] + Jc[1 * 3 + kk] * gvv[1][a] + Jc[2 * 3 + kk] * gvv[2][a];
-        tgr[c * 12 + a * 3 + kk] = t.d[0];
-        if (base) p.ulv[c * (int64_t)QS * 12 + a * 3 + kk] = t.v;
-      }
-  }
-  D mn[NV], mx[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) mn[v] = mx[v] = u0[v];
-  for (int f = 0; f < nf; ++f) {
-    const int64_t nb = p.neigh[c * MF + f];
-    if (nb < 0) continue;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      D un(U[nb * NV + v]);
-      un.d[0] = dU[nb * NV + v];
-      if (un.v < mn[v].v) mn[v] = un;
-      if (un.v > mx[v].v) mx[v] = un;
-    }
-  }
-  const double e3 = p.kappa_ven * p.minedge[c];
-  const double epsi2 = e3 * e3 * e3;
-  const double* qp = (const double*)p.qpts + grp * (int64_t)MF * QS * 3 * 32 + lane;
-  const double* bm = (const double*)p.bmean + grp * 3 * 32 + lane;
-  auto face_d = [&](int f, int v) -> D {
-    const double b0 = qp[(f * QS * 3 + 0) * 32] - bm[0], b1 = qp[(f * QS * 3 + 1) * 32] - bm[32],
-                 b2 = qp[(f * QS * 3 + 2) * 32] - bm[64];
-    const D res = b0 * g[0][v] + b1 * g[1][v] + b2 * g[2][v];
-    return (u0[v] + res) - u0[v];
+  constexpr int NW = muscl_warps<NS>();
+  constexpr int MC = 8;  // members per pass of the primitive records
+  __shared__ double s_d[MF * NV][33], s_t[MF * NV][33];                  // limited face values, their tangents
+  __shared__ double s_p[NS ? MC + 1 : 1][4][32], s_q[NS ? MC + 1 : 1][4][32];  // T, u, v, w and their tangents
+  __shared__ int s_first[32], s_nf[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t grp = blockIdx.x, g0 = grp * 32;
+  const int ncl = p.n - g0 < 32 ? (int)(p.n - g0) : 32;  // cells of this group
+  const int ln = lane < ncl ? lane : ncl - 1;            // spare lanes repeat the last cell
+  const int64_t c = g0 + ln;
+  const int IM = p.imax, W = IM + 1, QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  const int32_t* st = p.sten + grp * (int64_t)p.admis_max * W * 32 + ln;
+  const double* M = (const double*)p.invmat + (grp * p.tstride + p.soff[0]) * 32 + ln;
+  const int nf = p.nfaces[c];
+  auto state = [&](int64_t y, int v) -> D {
+    D u(U[y * NV + v]);
+    u.d[0] = dU[y * NV + v];
+    return u;
   };
-  D slope[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) slope[v] = D(TOLBIG);
-  for (int f = 0; f < nf; ++f)
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const D ps = venkat(face_d(f, v), mn[v] - u0[v], mx[v] - u0[v], epsi2);
-      if (ps.v < slope[v].v) slope[v] = ps;
-    }
-  double pm[NV], u0v[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) u0v[v] = u0[v].v;
-  cons2prim(p.gamma, u0v, pm);
-  bool first = false;
-  for (int f = 0; f < nf; ++f) {
-    double uf[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) uf[v] = u0v[v] + face_d(f, v).v * slope[v].v;
-    first = first || jump_bad(p.gamma, pm, uf, 0.95);
+  if (w == 0) {
+    s_first[lane] = 0;
+    s_nf[lane] = nf;
   }
-  double* dul = (double*)p.dul;
-  for (int f = 0; f < nf; ++f)
+  if (NS) {
+    D gv[3] = {D(0.0), D(0.0), D(0.0)};
+    for (int k0 = 0; k0 < IM; k0 += MC) {
+      if (k0) __syncthreads();  // the last pass's records have been read
+      const int j = k0 + w - 1;
+      if (w == 0 ? k0 == 0 : w <= MC && j < IM) {  // warp 0: the cell itself
+        const int64_t y = w == 0 ? c : (int64_t)st[(j + 1) * 32];
+        D u[NV], py[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const D x = face_d(f, v) * slope[v];
-      tdul[(c * MF + f) * NV + v] = first ? 0.0 : x.d[0];
-      if (base) dul[(c * MF + f) * NV + v] = first ? 0.0 : x.v;
+        for (int v = 0; v < NV; ++v) u[v] = state(y, v);
+        cons2prim(p.gamma, u, py);
+        const D t = py[4] / (py[0] * p.r_gas);
+        s_p[w][0][lane] = t.v;
+        s_q[w][0][lane] = t.d[0];
+#pragma unroll
+        for (int v = 1; v < 4; ++v) {
+          s_p[w][v][lane] = py[v].v;
+          s_q[w][v][lane] = py[v].d[0];
+        }
+      }
+      __syncthreads();
+      if (w >= NV) {
+        D t0(s_p[0][w - NV][lane]);
+        t0.d[0] = s_q[0][w - NV][lane];
+#pragma unroll
+        for (int i = 0; i < MC; ++i)
+          if (k0 + i < IM) {
+            D y(s_p[i + 1][w - NV][lane]);
+            y.d[0] = s_q[i + 1][w - NV][lane];
+            const D ds = y - t0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) gv[d] = gv[d] + M[((k0 + i) * 3 + d) * 32] * ds;
+          }
+      }
     }
+    if (w >= NV && lane < ncl) {
+      const double* J = p.jinv + c * 9;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const D t = J[0 * 3 + k] * gv[0] + J[1 * 3 + k] * gv[1] + J[2 * 3 + k] * gv[2];
+        tgr[c * 12 + (w - NV) * 3 + k] = t.d[0];
+        if (base) p.ulv[c * (int64_t)QS * 12 + (w - NV) * 3 + k] = t.v;
+      }
+    }
+  }
+  if (w < NV) {
+    const D u0 = state(c, w);
+    D g[3] = {D(0.0), D(0.0), D(0.0)};
+#pragma unroll 4
+    for (int k = 0; k < IM; ++k) {
+      const D du = state(st[(k + 1) * 32], w) - u0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) g[d] = g[d] + M[(k * 3 + d) * 32] * du;
+    }
+    D mn = u0, mx = u0;
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      const int nb = f < nf ? p.neigh[c * MF + f] : -1;
+      const D un = nb >= 0 ? state(nb, w) : u0;
+      if (un.v < mn.v) mn = un;
+      if (un.v > mx.v) mx = un;
+    }
+    const double ke = p.kappa_ven * p.minedge[c];
+    const double epsi2 = ke * ke * ke;
+    D dd[MF], slope(TOLBIG);
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      dd[f] = D(0.0);
+      if (f < nf) {
+        double b[3];
+        muscl_basis(p, c, f, b);
+        const D res = b[0] * g[0] + b[1] * g[1] + b[2] * g[2];
+        dd[f] = (u0 + res) - u0;
+        const D ps = venkat(dd[f], mn - u0, mx - u0, epsi2);
+        if (ps.v < slope.v) slope = ps;
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      const D x = dd[f] * slope;
+      s_d[f * NV + w][lane] = x.v;
+      s_t[f * NV + w][lane] = x.d[0];
+    }
+  }
+  __syncthreads();
+  {  // CHECKSOLX on the limited face values
+    double um[NV], pm[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) um[v] = U[c * NV + v];
+    cons2prim(p.gamma, um, pm);
+    for (int f = w; f < nf; f += NW) {
+      double uf[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) uf[v] = um[v] + s_d[f * NV + v][lane];
+      if (jump_bad(p.gamma, pm, uf, 0.95)) s_first[lane] = 1;
+    }
+  }
+  __syncthreads();
+  const int r = lane, f = r / NV;
+  if (r < MF * NV)
+    for (int cl = w; cl < ncl; cl += NW)
+      if (f < s_nf[cl]) {
+        const int64_t o = (g0 + cl) * MF * NV + r;
+        tdul[o] = s_first[cl] ? 0.0 : s_t[r][cl];
+        if (base) ((double*)p.dul)[o] = s_first[cl] ? 0.0 : s_d[r][cl];
+      }
 }
 
 // tangent of the face fluxes (owner and negated neighbour copy); with tgr
@@ -1318,7 +1302,10 @@ FwdStore fwd_store(ucg_engine* e) {
 
 // the reconstruction of U with its intermediates (face values to dul)
 int adj_forward(ucg_engine* e, const Problem& p, const double* U) {
-  k_adj_fwd<<<blocks_for(e->n, 128), 128, 0, e->stream>>>(p, U, fwd_store(e));
+  if (e->cfg.governing == 1)
+    k_adj_fwd<true><<<blocks_for(e->n, 32), 32 * muscl_warps<true>(), 0, e->stream>>>(p, U, fwd_store(e));
+  else
+    k_adj_fwd<false><<<blocks_for(e->n, 32), 32 * muscl_warps<false>(), 0, e->stream>>>(p, U, fwd_store(e));
   e->launches++;
   CK(cudaGetLastError());
   return UCG_OK;
@@ -1374,7 +1361,12 @@ int jvp_device(ucg_engine* e, const Problem& p, const double* U, const double* d
   }
   const int64_t n = e->n;
   double* tgr = e->cfg.governing == 1 ? (double*)e->adj_tgr.p : nullptr;
-  k_jvp_muscl<<<blocks_for(n, 128), 128, 0, e->stream>>>(p, U, dU, (double*)e->adj_tdul.p, tgr, !recon);
+  if (tgr)
+    k_jvp_muscl<true><<<blocks_for(n, 32), 32 * muscl_warps<true>(), 0, e->stream>>>(
+        p, U, dU, (double*)e->adj_tdul.p, tgr, !recon);
+  else
+    k_jvp_muscl<false><<<blocks_for(n, 32), 32 * muscl_warps<false>(), 0, e->stream>>>(
+        p, U, dU, (double*)e->adj_tdul.p, nullptr, !recon);
   k_jvp_face<<<blocks_for(e->nown, 128), 128, 0, e->stream>>>(p, U, dU, (const double*)e->adj_tdul.p, dp,
                                                               (double*)e->adj_tflux.p, tgr, nullptr);
   k_jvp_sum<<<blocks_for(n, 256), 256, 0, e->stream>>>(p, (const double*)e->adj_tflux.p, dR);
@@ -1458,7 +1450,8 @@ int force_device(ucg_engine* e, const Problem& p, const double* U, const double*
     CK(launch_lsq_f64(e->cfg.iorder, pt, dU, e->stream, &e->launches));
     if ((rc = launch_weno_tangent(e, p, U, dU, (const double*)e->adjw_gbar.p, tdul))) return rc;
   } else if (dU) {
-    k_jvp_muscl<<<blocks_for(e->n, 128), 128, 0, e->stream>>>(p, U, dU, tdul, nullptr, false);
+    k_jvp_muscl<false><<<blocks_for(e->n, 32), 32 * muscl_warps<false>(), 0, e->stream>>>(p, U, dU, tdul, nullptr,
+                                                                                        false);
     e->launches++;
   }
   k_force_cell<<<blocks_for(e->n, 128), 128, 0, e->stream>>>(p, U, dU, tdul, (double*)e->adj_fcell.p, nullptr, 0.0);

@@ -155,6 +155,14 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// warps of a 32-cell group in the MUSCL kernels (k_muscl, k_adj_fwd,
+// k_jvp_muscl): one per conserved variable, Navier-Stokes one more for each
+// of T, u, v, w
+template <bool NS>
+__host__ __device__ constexpr int muscl_warps() {
+  return NS ? NV + 4 : NV;
+}
+
 // cells of a tile of k_lsq_set, and the row stride of a shared matrix (whole
 // 16-byte vectors)
 constexpr int SET_TILE = 128;

@@ -32,10 +32,6 @@ namespace ucg {
 // 41.2 us.  56 registers (four blocks of nine warps, seven of five per SM): with
 // the compiler's choice the same kernel took 40.5 us at 32,768 cells.
 // ======================================================================
-template <bool NS>
-__host__ __device__ constexpr int muscl_warps() {
-  return NS ? NV + 4 : NV;
-}
 template <typename T, bool NS, bool VK>
 __global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Problem p, const double* U) {
   pdl_begin();
