@@ -92,6 +92,11 @@ __device__ __forceinline__ double is_and_grad(const double* __restrict__ P, cons
 // 0.72 -> 0.57.
 constexpr int WP_THREADS = NV * 32;
 extern __shared__ __align__(16) double wp_tri[];
+// of S and, with CWENO, of S2 (at most nine rows)
+template <int P>
+constexpr size_t group_tri_smem() {
+  return (size_t)(tri_len<double>(Deg<P>::ideg) + tri_len<double>(9)) * 8;
+}
 // the group's shared triangles into wp_tri (all threads; a barrier follows)
 __device__ __forceinline__ bool group_triangles(const Problem& p, int64_t grp) {
   const int gs = p.ntile ? p.gset[grp] : -1;
@@ -1022,7 +1027,7 @@ template <int P, int ND, bool LOW>
 cudaError_t launch_adj_set(const Problem& p, int nst, const double* gbar, double* selfs, double* contrib,
                            cudaStream_t st) {
   const size_t smem = (size_t)(LOW ? p.imax2 : p.imax) * set_stride<double>(ND) * 8;
-  const cudaError_t e = cudaFuncSetAttribute(k_adj_lsq_set<P, ND, LOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_adj_lsq_set<P, ND, LOW>, SET_SMEM);
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)p.ntile, (unsigned)(nst * AdjPass<ND>::count));
   k_adj_lsq_set<P, ND, LOW><<<grid, SET_TILE, smem, st>>>(p, gbar, selfs, contrib);
@@ -1036,7 +1041,7 @@ cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, doub
                      double* contrib, cudaStream_t st, int64_t* launches) {
   constexpr int ID = Deg<P>::ideg;
   const size_t tri = p.ntile ? (size_t)p.istride * 8 : 0;
-  const cudaError_t ea = cudaFuncSetAttribute(k_adj_wpost<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri);
+  const cudaError_t ea = smem_limit(k_adj_wpost<P>, group_tri_smem<P>());
   if (ea != cudaSuccess) return ea;
   k_adj_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, tri, st>>>(p, U, adjF, gbar, scr, selfc, contrib);
   if (p.ntile) {
@@ -1062,11 +1067,13 @@ cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, doub
 }
 
 template <int P>
-void launch_jvp_t(const Problem& p, const double* U, const double* dU, const double* dG, double* tdul,
-                  cudaStream_t st) {
+cudaError_t launch_jvp_t(const Problem& p, const double* U, const double* dU, const double* dG, double* tdul,
+                         cudaStream_t st) {
   const size_t tri = p.ntile ? (size_t)p.istride * 8 : 0;
-  cudaFuncSetAttribute(k_jvp_wpost<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri);
+  const cudaError_t e = smem_limit(k_jvp_wpost<P>, group_tri_smem<P>());
+  if (e != cudaSuccess) return e;
   k_jvp_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, tri, st>>>(p, U, dU, dG, tdul);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -1076,14 +1083,13 @@ namespace ucg_host {
 int launch_weno_tangent(ucg_engine* e, const Problem& p, const double* U, const double* dU, const double* dG,
                         double* tdul) {
   switch (e->cfg.iorder) {
-    case 1: launch_jvp_t<1>(p, U, dU, dG, tdul, e->stream); break;
-    case 2: launch_jvp_t<2>(p, U, dU, dG, tdul, e->stream); break;
-    case 3: launch_jvp_t<3>(p, U, dU, dG, tdul, e->stream); break;
-    case 4: launch_jvp_t<4>(p, U, dU, dG, tdul, e->stream); break;
+    case 1: CK(launch_jvp_t<1>(p, U, dU, dG, tdul, e->stream)); break;
+    case 2: CK(launch_jvp_t<2>(p, U, dU, dG, tdul, e->stream)); break;
+    case 3: CK(launch_jvp_t<3>(p, U, dU, dG, tdul, e->stream)); break;
+    case 4: CK(launch_jvp_t<4>(p, U, dU, dG, tdul, e->stream)); break;
     default: return fail(e, UCG_EINVAL, "iorder out of range");
   }
   e->launches++;
-  CK(cudaGetLastError());
   return UCG_OK;
 }
 

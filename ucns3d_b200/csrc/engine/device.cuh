@@ -171,6 +171,19 @@ __host__ __device__ constexpr int set_stride(int nd) {
   return (nd + Vec<T>::N - 1) / Vec<T>::N * Vec<T>::N;
 }
 
+// The dynamic shared memory that a kernel may be launched with is a property of
+// the device's context: engines on other threads launch the same kernel.  So
+// the limit is always set to the same value, a constant of the kernel that
+// covers every engine, and never to what one engine's launch needs (a thread
+// that lowered it between another's limit and launch had that launch refused).
+constexpr size_t SMEM_BLOCK = 227 * 1024;  // of a block, static and dynamic together
+constexpr size_t SET_SMEM = 226 * 1024;    // of the kernels that keep a set's rows (k_lsq_set: 0.2 KB static)
+constexpr size_t LOW_SMEM = 206 * 1024;    // of k_lsq_low (up to 20 KB static)
+template <typename... KA>
+cudaError_t smem_limit(void (*k)(KA...), size_t most) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // elements of a packed triangle of n rows, each padded to whole vectors
 template <typename T>
 __host__ __device__ constexpr int tri_len(int n) {

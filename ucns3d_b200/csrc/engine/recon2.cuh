@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(256, Ring<P, T>::BPS) k_lsq_ring(Problem p, co
 template <int P, typename T>
 cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) {
   using R = Ring<P, T>;
-  const cudaError_t e = cudaFuncSetAttribute(k_lsq_ring<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem);
+  const cudaError_t e = smem_limit(k_lsq_ring<P, T>, R::smem);
   if (e != cudaSuccess) return e;
   const int64_t items = (p.ntile ? p.nugrp : (p.n + 31) / 32) * p.admis_max, nb = (items + 3) / 4;
   const long wait = p.lsq_bulk && p.lsq_wait >= 0 ? p.lsq_wait : LSQ_WAIT;
@@ -578,7 +578,7 @@ template <int P, typename T, int ND>
 cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cudaStream_t st) {
   using R = SetRing<T, ND>;
   const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + 2 * R::NSTG * R::elems) * sizeof(T);
-  const cudaError_t e = cudaFuncSetAttribute(k_lsq_set<P, T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_lsq_set<P, T, ND>, SET_SMEM);
   if (e != cudaSuccess) return e;
   k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U);
   return cudaGetLastError();
@@ -586,7 +586,7 @@ cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cu
 template <int P, typename T, int ND>
 cudaError_t launch_lsq_low(const Problem& p, const double* U, cudaStream_t st) {
   const size_t smem = (size_t)p.imax2 * set_stride<T>(ND) * sizeof(T);
-  const cudaError_t e = cudaFuncSetAttribute(k_lsq_low<P, T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_lsq_low<P, T, ND>, LOW_SMEM);
   if (e != cudaSuccess) return e;
   k_lsq_low<P, T, ND><<<dim3((unsigned)p.ntile, (unsigned)p.admis_max - 1), SET_TILE, smem, st>>>(p, U);
   return cudaGetLastError();
@@ -796,6 +796,10 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
 // 0.156 -> 0.089 ms, mixed 0.075 -> 0.044); above, reading the triangles in
 // five warps costs more than it hides (271,872 cells mixed 0.564 -> 0.626,
 // 24,576 FP64 0.133 -> 0.139).
+template <typename T>
+__host__ __device__ constexpr size_t wface_smem(int QS) {
+  return ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
+}
 template <int P, typename T, bool OWN = false>
 __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
@@ -1864,7 +1868,7 @@ cudaError_t launch_wpost_char(const Problem& p, const double* U, cudaStream_t st
   constexpr int NF = CharFaces<P, T>::value;
   const unsigned ng = (unsigned)((p.n + 31) / 32);
   const size_t smem = char_face_smem<P, T>(QS);
-  const cudaError_t e = cudaFuncSetAttribute(k_char_face<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_char_face<P, T>, char_face_smem<P, T>(MQ));
   if (e != cudaSuccess) return e;
   k_char_forms<P, T><<<dim3(ng, (unsigned)p.admis_max), 32 * NV, 0, st>>>(p);
   k_char_face<P, T><<<dim3(ng, (MF + NF - 1) / NF), 32 * NV, smem, st>>>(p, U);
@@ -1928,7 +1932,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     // than it saves (2.1 M-cell CWENO4: 17.3 -> 19.6 ms)
     bool done = false;
     const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-    const size_t smem = ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
+    const size_t smem = wface_smem<T>(QS);
     const unsigned ng = (unsigned)((p.n + 31) / 32);
     if constexpr (P == 4) {
       if (p.isb && p.scheme == 3) {
@@ -1936,7 +1940,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
         if (e != cudaSuccess) return e;
         ++*launches;
         if (p.wface) {
-          cudaFuncSetAttribute(k_wface<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          const cudaError_t ef = smem_limit(k_wface<P, T>, wface_smem<T>(MQ));
+          if (ef != cudaSuccess) return ef;
           k_wface<P, T><<<ng, 32 * NV, smem, st>>>(p, U);
           k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
           ++*launches;
@@ -1946,7 +1951,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
         done = true;
       }
     } else if (p.wface && p.scheme == 3 && (P < 3 || p.n < (int64_t)p.nsm * 128)) {
-      cudaFuncSetAttribute(k_wface<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      const cudaError_t e = smem_limit(k_wface<P, T, true>, wface_smem<T>(MQ));
+      if (e != cudaSuccess) return e;
       k_wface<P, T, true><<<ng, 32 * NV, smem, st>>>(p, U);
       k_wpost<P, T, false, true><<<b, 128, 0, st>>>(p, U);
       ++*launches;
@@ -1959,7 +1965,8 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     k_visc_prim<P, T><<<(unsigned)((pa.n + 255) / 256), 256, 0, st>>>(pa, U);
     if (p.ntile) {
       const size_t rows = (size_t)p.imax * set_stride<T>(Deg<P>::ideg) * sizeof(T);
-      cudaFuncSetAttribute(k_visc_lsq<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
+      const cudaError_t e = smem_limit(k_visc_lsq<P, T, true>, SET_SMEM);
+      if (e != cudaSuccess) return e;
       k_visc_lsq<P, T, true><<<(unsigned)((p.nugrp + 3) / 4 + p.ntile), 128, rows, st>>>(p, U);
     } else {
       k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);

@@ -459,8 +459,9 @@ int ucg_build_recon(ucg_engine* e, const ucg_shapes* s, const ucg_recon* r) {
   if (cudaGetLastError() != cudaSuccess) return bail(cuda_fail(e, cudaErrorLaunchFailure, "k_setup_mean"));
   // ---- matrix sets, staged and expanded like uploaded ones
   const size_t lsq_smem = lsq_smem_doubles(c.imax, c.ideg) * 8;
-  if (cudaFuncSetAttribute(k_setup_lsq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsq_smem) != cudaSuccess)
-    return bail(cuda_fail(e, cudaGetLastError(), "cudaFuncSetAttribute"));
+  if (lsq_smem > SMEM_BLOCK)
+    return bail(cuda_fail(e, cudaErrorInvalidValue, "k_setup_lsq: a stencil's matrices do not fit in shared memory"));
+  if (const cudaError_t es = smem_limit(k_setup_lsq, SMEM_BLOCK)) return bail(cuda_fail(e, es, "k_setup_lsq"));
   DevBuf tidbuf;
   if (r->table_id) {
     if ((rc = upload_vec(e, tidbuf, r->table_id, n))) return bail(rc);
