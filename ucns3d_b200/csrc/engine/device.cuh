@@ -170,6 +170,8 @@ template <typename T>
 __host__ __device__ constexpr int set_stride(int nd) {
   return (nd + Vec<T>::N - 1) / Vec<T>::N * Vec<T>::N;
 }
+// gathered differences of the two rings of a k_lsq_set block (SetRing)
+constexpr int SET_RING = 2 * 4 * 4 * 32 * NV;
 
 // The dynamic shared memory that a kernel may be launched with is a property of
 // the device's context: engines on other threads launch the same kernel.  So

@@ -926,18 +926,25 @@ namespace {
 // SET_MIN cells share (a quarter of a tile: below that a tile costs more than
 // the group of 32 that k_lsq_ring would read), cut into tiles of SET_TILE in
 // device order.  set_of gets each table's set, -1 where its cells read their
-// own tables.  Kept only where it pays: a tile is taken to cost three fifths of
-// what its 128 cells cost k_lsq_ring, which costs the same for a group of 32
-// cells whether one or all of them are left to it.  Measured, all cells tiled
-// against all through the ring: WENO5 64^3 mixed 2.13 / 4.81 ms, 40^3 FP64
-// 1.21 / 2.11, 12^3 FP64 0.058 / 0.090; WENO3 48^3 0.193 / 0.298 (mixed), 0.290
-// / 0.340 (FP64); CWENO4 271,872 cells mixed 0.438 / 0.482, 75,776 FP64 0.236 /
-// 0.234.
+// own tables.  None where the rows of a stencil do not fit in shared memory
+// (k_lsq_set with its rings takes the most of it; IORDER 4 from 701 members in
+// FP64, 1,465 in FP32): k_lsq_ring takes any number.  Kept only where it pays:
+// a tile is taken to cost three fifths of what its 128 cells cost k_lsq_ring,
+// which costs the same for a group of 32 cells whether one or all of them are
+// left to it.  Measured, all cells tiled against all through the ring: WENO5
+// 64^3 mixed 2.13 / 4.81 ms, 40^3 FP64 1.21 / 2.11, 12^3 FP64 0.058 / 0.090;
+// WENO3 48^3 0.193 / 0.298 (mixed), 0.290 / 0.340 (FP64); CWENO4 271,872 cells
+// mixed 0.438 / 0.482, 75,776 FP64 0.236 / 0.234.
 constexpr int64_t SET_MIN = 32;
 int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<int32_t>& set_of, int64_t* tiles) {
   const ucg_config& c = e->cfg;
   const int64_t n = e->n_recon;
   const bool perm = !e->n2o.empty();
+  const int64_t vec = e->mixed ? 4 : 2, ts = (int64_t)tsize(e);
+  auto row = [&](int nd) { return (nd + vec - 1) / vec * vec; };
+  if ((c.imax * row(c.ideg) + SET_RING) * ts > (int64_t)SET_SMEM ||
+      (c.ees == 5 && c.admis_max > 1 && c.imax2 * row(c.ideg2) * ts > (int64_t)LOW_SMEM))
+    return UCG_OK;
   auto table = [&](int64_t cell) { return table_id[perm ? e->n2o[cell] : cell]; };
   std::vector<int64_t> cells(ntab, 0);
   for (int64_t i = 0; i < n; ++i) cells[table(i)]++;
@@ -974,12 +981,11 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
     tcell[(size_t)at[s]++] = (int32_t)i;
     tiled[(size_t)i] = 1;
   }
-  const int64_t vec = e->mixed ? 4 : 2;
   int64_t off = 0;
   for (int ll = 0; ll < c.admis_max; ++ll) {
     const bool low = c.ees == 5 && ll > 0;
     e->sso[ll] = (int)off;
-    off += (int64_t)(low ? c.imax2 : c.imax) * (((low ? c.ideg2 : c.ideg) + vec - 1) / vec * vec);
+    off += (int64_t)(low ? c.imax2 : c.imax) * row(low ? c.ideg2 : c.ideg);
   }
   e->sstride = off;
   e->nset = nset;

@@ -142,6 +142,7 @@ struct SetRing {
   static constexpr int WARPS = 2 * (NSL + NPR);
   static constexpr int MS = 4, NSTG = 4;  // members of a stage, stages (a multiple of NPR)
   static constexpr int elems = MS * 32 * NV;  // of a stage
+  static_assert(2 * NSTG * elems == SET_RING, "plan_sets asks whether the rings fit");
 };
 template <int P, typename T, int ND>
 __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS) k_lsq_set(Problem p, const double* __restrict__ U) {
@@ -577,7 +578,7 @@ cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) 
 template <int P, typename T, int ND>
 cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cudaStream_t st) {
   using R = SetRing<T, ND>;
-  const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + 2 * R::NSTG * R::elems) * sizeof(T);
+  const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + SET_RING) * sizeof(T);
   const cudaError_t e = smem_limit(k_lsq_set<P, T, ND>, SET_SMEM);
   if (e != cudaSuccess) return e;
   k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U);
