@@ -1352,6 +1352,21 @@ __global__ void k_visc_prim(Problem p, const double* __restrict__ U) {
 // the tiles.  271,872 cells, CWENO4 mixed form: 0.270 -> 0.149 ms (0.167 at three
 // blocks per SM, 0.229 at five with two members in flight; the groups left in
 // a launch of their own 0.056 more).
+// Blocks of that launch with left-over groups (four each), and the cell of a
+// thread of a block, -1 for none: a tiled cell of a left-over group has its
+// block among the tiles', so that every cell has one writer.
+__host__ __device__ inline int64_t visc_lsq_own(const Problem& p) { return (p.nugrp + 3) / 4; }
+template <bool SET>
+__host__ __device__ inline int64_t visc_lsq_cell(const Problem& p, int64_t block, int thread) {
+  const int64_t own = SET ? visc_lsq_own(p) : 0;
+  if (SET && block >= own) return p.tcell[(block - own) * SET_TILE + thread];
+  int64_t c = block * 128 + thread;
+  if (SET) {
+    if ((c >> 5) >= p.nugrp) return -1;
+    c = (int64_t)p.ugrp[c >> 5] * 32 + (c & 31);
+  }
+  return c < p.n && !(SET && p.tiled[c]) ? c : -1;
+}
 template <int P, typename T, bool SET = false>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 && P <= 3 ? 4 : 1) k_visc_lsq(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
@@ -1360,24 +1375,15 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 && P <= 3 ? 4 : 1) k_visc_
   extern __shared__ __align__(16) unsigned char vl_smem[];
   const T* s = (const T*)vl_smem;
   const int IM = p.imax, W = IM + 1;
-  const unsigned nown = SET ? (unsigned)((p.nugrp + 3) / 4) : 0;
-  const bool tiled = SET && blockIdx.x >= nown;
-  int64_t c;
+  const bool tiled = SET && blockIdx.x >= visc_lsq_own(p);
   if (tiled) {
-    const int64_t tile = blockIdx.x - nown;
+    const int64_t tile = blockIdx.x - visc_lsq_own(p);
     const float4* src = (const float4*)((const T*)p.setmat + p.tset[tile] * p.sstride + p.sso[0]);
     for (int i = threadIdx.x; i < IM * RS / VEC; i += SET_TILE) ((float4*)vl_smem)[i] = src[i];
     __syncthreads();
-    c = p.tcell[tile * SET_TILE + threadIdx.x];
-    if (c < 0) return;
-  } else {
-    c = (int64_t)blockIdx.x * 128 + threadIdx.x;
-    if (SET) {
-      if ((c >> 5) >= p.nugrp) return;
-      c = (int64_t)p.ugrp[c >> 5] * 32 + (c & 31);
-    }
-    if (c >= p.n) return;
   }
+  const int64_t c = visc_lsq_cell<SET>(p, blockIdx.x, threadIdx.x);
+  if (c < 0) return;
   double pm[NV];
   cons2prim(p.gamma, U + c * NV, pm);
   const double s0[4] = {pm[4] / (pm[0] * p.r_gas), pm[1], pm[2], pm[3]};
@@ -1968,7 +1974,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
       const size_t rows = (size_t)p.imax * set_stride<T>(Deg<P>::ideg) * sizeof(T);
       const cudaError_t e = smem_limit(k_visc_lsq<P, T, true>, SET_SMEM);
       if (e != cudaSuccess) return e;
-      k_visc_lsq<P, T, true><<<(unsigned)((p.nugrp + 3) / 4 + p.ntile), 128, rows, st>>>(p, U);
+      k_visc_lsq<P, T, true><<<(unsigned)(visc_lsq_own(p) + p.ntile), 128, rows, st>>>(p, U);
     } else {
       k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
     }
