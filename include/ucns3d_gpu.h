@@ -277,11 +277,12 @@ int ucg_time_kernels(ucg_engine* e, int32_t reps, double* ms);
 /* Bounded device waits.  The stencil least squares passes its tables and
  * gathered states through rings in shared memory, whose waits give up after
  * 65,536 polls (about 300 ns each, about 20 ms in all).  An engine created
- * with UCG_LSQ_BULK=1 in the environment reads every cell's own tables (no
- * shared matrix sets) and takes `polls` as its bound instead (the default is
- * restored by polls < 0).  A wait that gives up makes its block finish the
- * copies it has in flight (each with the default bound) and return, and the
- * next ucg_check_health reports UCG_ETIMEOUT; the handle stays usable.
+ * with UCG_LSQ_WAIT=1 in the environment takes `polls` as its bound instead
+ * (the default is restored by polls < 0), and so does one created with
+ * UCG_LSQ_BULK=1, which reads every cell's own tables (no shared matrix sets).
+ * A wait that gives up makes its block finish the copies it has in flight (each
+ * with the default bound) and return without its results, and the next
+ * ucg_check_health reports UCG_ETIMEOUT; the handle stays usable.
  * polls = 0 makes every such wait give up at once, which exercises that path
  * without a fault.  No counterpart in the reference. */
 int ucg_set_wait_limit(ucg_engine* e, int64_t polls);

@@ -15,7 +15,7 @@ import pytest
 
 from ucns3d_b200 import _native as N
 from ucns3d_b200.config import EULER, NAVIER_STOKES, make_config
-from ucns3d_b200.engine import Engine
+from ucns3d_b200.engine import Engine, EngineError
 from ucns3d_b200.mesh import IC_TGV, SCHEME_MUSCL, SCHEME_WENO, Mesh, RenumberedMesh
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +91,26 @@ def test_shared_sets_reverse(name):
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
     assert np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("precision", [N.UCG_FP64, N.UCG_MIXED])
+@pytest.mark.parametrize("name", ["weno5_hex12", "weno5_hex_open", "cweno4_ns_mixed10"])
+def test_wait_timeout_is_reported_and_recoverable(name, precision, monkeypatch):
+    """The bounded waits between the warps of k_lsq_set (and of k_lsq_ring for
+    the cells left over): with a limit of 0 polls every wait gives up and the
+    kernels return, ucg_check_health reports UCG_ETIMEOUT, and with the default
+    limit restored the handle gives its residual again, bit for bit."""
+    monkeypatch.setenv("UCG_LSQ_WAIT", "1")
+    m, e, own, U = _engines(name, precision)
+    own.close()
+    e.set_state(U)
+    ref = e.residual()
+    e.check_health()
+    assert e.lib.ucg_set_wait_limit(e._h, 0) == N.UCG_OK
+    e.residual()
+    with pytest.raises(EngineError) as ei:
+        e.check_health()
+    assert ei.value.code == N.UCG_ETIMEOUT
+    assert e.lib.ucg_set_wait_limit(e._h, -1) == N.UCG_OK
+    assert np.array_equal(e.residual(), ref)
+    e.check_health()

@@ -162,9 +162,8 @@ Problem make_problem(ucg_engine* e) {
   p.dt_dev = nullptr;
   p.dt_next = nullptr;
   p.ccfl = 0.0;
-  p.lsq_bulk = e->lsq_bulk;
   p.nsm = e->nsm;
-  p.lsq_wait = e->lsq_wait;
+  p.lsq_wait = e->lsq_bulk || e->lsq_limit ? e->lsq_wait : -1;
   p.wenwrt = c.wenwrt;
   p.riemann = c.riemann;
   p.limiter = c.limiter;
@@ -540,6 +539,8 @@ int ucg_create(const ucg_config* cfg, int64_t ncells, int device, ucg_engine** o
   {
     const char* bulk = std::getenv("UCG_LSQ_BULK");
     e->lsq_bulk = bulk && bulk[0] == '1';
+    const char* limit = std::getenv("UCG_LSQ_WAIT");
+    e->lsq_limit = limit && limit[0] == '1';
     e->nsm = prop.multiProcessorCount;
   }
   {

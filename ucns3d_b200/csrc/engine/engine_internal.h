@@ -75,7 +75,8 @@ struct ucg_engine {
   bool lsq_bulk = false;       // UCG_LSQ_BULK=1 at ucg_create: no shared sets, every cell through k_lsq_ring
   int nsm = 148;
   bool wface = false;          // conserved WENO: face values one warp per variable (k_wface)
-  long lsq_wait = -1;          // polls of a k_lsq_ring stage wait (ucg_set_wait_limit; < 0 the default)
+  bool lsq_limit = false;      // UCG_LSQ_WAIT=1 at ucg_create: lsq_wait holds with shared sets too
+  long lsq_wait = -1;          // polls of a stage wait of the least squares (ucg_set_wait_limit; < 0 the default)
   std::vector<uint8_t> recon_done;  // per cell, for ucg_upload_recon chunks
   std::vector<int8_t> admis_h;      // ADMIS per cell, for the stencil checks of ucg_upload_recon
   std::vector<int32_t> neigh_h;     // [n][6] face neighbours (host copy, adjoint set-up)

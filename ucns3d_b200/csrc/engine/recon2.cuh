@@ -50,6 +50,7 @@ struct GatherShare {
 
 // polls of one stage wait (about 20 ms; a stage normally lands in microseconds)
 constexpr long LSQ_WAIT = 1L << 16;
+inline long lsq_wait(const Problem& p) { return p.lsq_wait < 0 ? LSQ_WAIT : p.lsq_wait; }
 
 // mbar_wait of a warp that also gives up when another warp of the block has
 __device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity, long limit, const volatile int* stop) {
@@ -129,6 +130,8 @@ struct RowAcc<double> {
 // kernel 2.13, 0.51 and, with k_lsq_low and the 48 groups left to k_lsq_ring,
 // 0.43.  Its shared-memory loads (34 words a row of five multiply-adds, 70
 // cycles a member and 32 cells in FP32) stand before the multiply-adds (43).
+// A wait that gives up (`wait` polls) sets HEALTH_TIMEOUT and s_stop, the other
+// warps see it in their own waits, and the block's polynomials are not stored.
 template <typename T, int ND>
 struct SetRing {
   static constexpr int VEC = Vec<T>::N, NVEC = (ND + VEC - 1) / VEC;  // vectors of rows
@@ -145,7 +148,8 @@ struct SetRing {
   static_assert(2 * NSTG * elems == SET_RING, "plan_sets asks whether the rings fit");
 };
 template <int P, typename T, int ND>
-__global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS) k_lsq_set(Problem p, const double* __restrict__ U) {
+__global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
+    k_lsq_set(Problem p, const double* __restrict__ U, long wait) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int RS = set_stride<T>(ND);
   using R = SetRing<T, ND>;
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS) k_lsq_set(Problem 
         for (int j = 0; j < MS; ++j) sh.load(U, y[j], u[j]);
 #pragma unroll
         for (int j = 0; j < MS; ++j) y[j] = member(k + R::NPR * MS + j);
-        if (!(ok = ring_wait(&empty[slot], ph ^ 1u, LSQ_WAIT, &s_stop))) break;  // the first round finds them empty
+        if (!(ok = ring_wait(&empty[slot], ph ^ 1u, wait, &s_stop))) break;  // the first round finds them empty
         T* du = ring + slot * R::elems + lane;
 #pragma unroll
         for (int j = 0; j < MS; ++j)
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS) k_lsq_set(Problem 
       };
       if (any)
         for (int k = 0; k < nk; k += MS) {
-          if (!(ok = ring_wait(&full[slot], ph, LSQ_WAIT, &s_stop))) break;
+          if (!(ok = ring_wait(&full[slot], ph, wait, &s_stop))) break;
           const T* d = ring + slot * R::elems + lane * NV;
           const T* m = s + k * RS + q0 * VEC;
           if (k + MS <= nk) {
@@ -569,8 +573,7 @@ cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) 
   const cudaError_t e = smem_limit(k_lsq_ring<P, T>, R::smem);
   if (e != cudaSuccess) return e;
   const int64_t items = (p.ntile ? p.nugrp : (p.n + 31) / 32) * p.admis_max, nb = (items + 3) / 4;
-  const long wait = p.lsq_bulk && p.lsq_wait >= 0 ? p.lsq_wait : LSQ_WAIT;
-  k_lsq_ring<P, T><<<(unsigned)(nb < p.nsm * R::BPS ? nb : p.nsm * R::BPS), 256, R::smem, st>>>(p, U, items, wait);
+  k_lsq_ring<P, T><<<(unsigned)(nb < p.nsm * R::BPS ? nb : p.nsm * R::BPS), 256, R::smem, st>>>(p, U, items, lsq_wait(p));
   return cudaGetLastError();
 }
 
@@ -581,7 +584,7 @@ cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cu
   const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + SET_RING) * sizeof(T);
   const cudaError_t e = smem_limit(k_lsq_set<P, T, ND>, SET_SMEM);
   if (e != cudaSuccess) return e;
-  k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U);
+  k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U, lsq_wait(p));
   return cudaGetLastError();
 }
 template <int P, typename T, int ND>
