@@ -62,6 +62,19 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity, long l
   }
   return __all_sync(0xffffffffu, ok);
 }
+// The same with the bound in shared memory, read only when a poll has failed
+// (k_lsq_set: a limit that the loops carry took 102 registers instead of 96 and
+// with them the second block per SM, 2.13 -> 3.37 ms); a warp that gives up sets
+// it to -1 for the others.
+__device__ __forceinline__ bool set_wait(uint64_t* bar, unsigned parity, const volatile int* limit) {
+  bool ok = false;
+  for (long it = 0; it < LSQ_WAIT; ++it) {
+    ok = mbar_try_wait(bar, parity);
+    if (ok || it >= *limit) break;
+    if (it > 64) __nanosleep(256);
+  }
+  return __all_sync(0xffffffffu, ok);
+}
 
 template <int N>
 struct IntC {
@@ -130,8 +143,8 @@ struct RowAcc<double> {
 // kernel 2.13, 0.51 and, with k_lsq_low and the 48 groups left to k_lsq_ring,
 // 0.43.  Its shared-memory loads (34 words a row of five multiply-adds, 70
 // cycles a member and 32 cells in FP32) stand before the multiply-adds (43).
-// A wait that gives up (`wait` polls) sets HEALTH_TIMEOUT and s_stop, the other
-// warps see it in their own waits, and the block's polynomials are not stored.
+// A wait that gives up (`wait` polls) sets HEALTH_TIMEOUT and ends the waits of
+// the block's other warps, and its polynomials are not stored.
 template <typename T, int ND>
 struct SetRing {
   static constexpr int VEC = Vec<T>::N, NVEC = (ND + VEC - 1) / VEC;  // vectors of rows
@@ -149,7 +162,7 @@ struct SetRing {
 };
 template <int P, typename T, int ND>
 __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
-    k_lsq_set(Problem p, const double* __restrict__ U, long wait) {
+    k_lsq_set(Problem p, const double* __restrict__ U, int wait) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int RS = set_stride<T>(ND);
   using R = SetRing<T, ND>;
@@ -157,7 +170,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
   constexpr int TH = 32 * R::WARPS;
   extern __shared__ __align__(16) unsigned char ls_smem[];
   __shared__ __align__(8) uint64_t s_full[2][NSTG], s_empty[2][NSTG];
-  __shared__ int s_stop;
+  __shared__ int s_limit;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = warp & 1, role = warp >> 1;
   const int64_t tile = blockIdx.x >> 1;
   const int ll = blockIdx.y;
@@ -168,10 +181,10 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
   T* ring = s + nk * RS + half * NSTG * R::elems;
   uint64_t *full = s_full[half], *empty = s_empty[half];
   if (threadIdx.x == 0) {
-    s_stop = 0;
+    s_limit = wait;
     for (int w = 0; w < 2; ++w)
       for (int i = 0; i < NSTG; ++i) {
-        mbar_init(&s_full[w][i], 1);
+        mbar_init(&s_full[w][i], wait ? 1 : 2);  // limit 0: no stage is ever full
         mbar_init(&s_empty[w][i], R::NSL);
       }
     mbar_fence_init();
@@ -206,7 +219,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
         for (int j = 0; j < MS; ++j) sh.load(U, y[j], u[j]);
 #pragma unroll
         for (int j = 0; j < MS; ++j) y[j] = member(k + R::NPR * MS + j);
-        if (!(ok = ring_wait(&empty[slot], ph ^ 1u, wait, &s_stop))) break;  // the first round finds them empty
+        if (!(ok = set_wait(&empty[slot], ph ^ 1u, &s_limit))) break;  // the first round finds them empty
         T* du = ring + slot * R::elems + lane;
 #pragma unroll
         for (int j = 0; j < MS; ++j)
@@ -234,7 +247,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
       };
       if (any)
         for (int k = 0; k < nk; k += MS) {
-          if (!(ok = ring_wait(&full[slot], ph, wait, &s_stop))) break;
+          if (!(ok = set_wait(&full[slot], ph, &s_limit))) break;
           const T* d = ring + slot * R::elems + lane * NV;
           const T* m = s + k * RS + q0 * VEC;
           if (k + MS <= nk) {
@@ -262,7 +275,7 @@ __global__ void __launch_bounds__(32 * SetRing<T, ND>::WARPS)
   }
   if (!ok && lane == 0) {
     atomicOr(p.health, HEALTH_TIMEOUT);
-    *(volatile int*)&s_stop = 1;
+    *(volatile int*)&s_limit = -1;
   }
 }
 
@@ -584,7 +597,7 @@ cudaError_t launch_lsq_set_t(const Problem& p, const double* U, unsigned nst, cu
   const size_t smem = ((size_t)p.imax * set_stride<T>(ND) + SET_RING) * sizeof(T);
   const cudaError_t e = smem_limit(k_lsq_set<P, T, ND>, SET_SMEM);
   if (e != cudaSuccess) return e;
-  k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U, lsq_wait(p));
+  k_lsq_set<P, T, ND><<<dim3((unsigned)p.ntile * 2, nst), 32 * R::WARPS, smem, st>>>(p, U, (int)(lsq_wait(p) < LSQ_WAIT ? lsq_wait(p) : LSQ_WAIT));
   return cudaGetLastError();
 }
 template <int P, typename T, int ND>
