@@ -172,69 +172,92 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-# DRAM traffic of one launch of the stencil least squares per cell,
-# dram__bytes_read.sum + dram__bytes_write.sum of a one-kernel ncu capture
-# divided by the cells of the captured mesh, keyed by (workload, precision).
-# Only measured entries are listed; other workloads report traffic null.  The
-# traffic grows in proportion to the cells, so a launch on a larger mesh of the
-# same workload moves this times its cells.
-#   vortex_hex_weno5, mixed: 32^3 capture of k_lsq_set (97.2 + 105.4 MB)
-LSQ_DRAM_BYTES_PER_CELL = {("vortex_hex_weno5", 1): 6_182}
+# DRAM bytes of one launch of the stencil least squares on a mesh of `cells`
+# cells, dram__bytes_read.sum and dram__bytes_write.sum of a one-kernel ncu
+# capture, keyed by (workload, precision); only measured entries are listed.
+#   vortex_hex_weno5, mixed: 32^3 capture of k_lsq_set
+LSQ_DRAM = {("vortex_hex_weno5", 1): {"cells": 32 ** 3, "read": 97.2e6, "written": 105.4e6}}
 
 
-def lsq_bytes_per_cell(cfg, sets_per_cell=1.0):
+def lsq_rows(cfg):
+    """(members, rows) of each stencil's pseudo-inverse."""
+    return [((cfg.imax2, cfg.ideg2) if cfg.ees == 5 and ll > 0 else (cfg.imax, cfg.ideg))
+            for ll in range(cfg.admis_max)]
+
+
+def table_size(cfg):
+    from ucns3d_b200 import _native as N
+    return 4 if cfg.precision == N.UCG_MIXED else 8
+
+
+def lsq_traffic(workload, cfg, ncells):
+    """DRAM bytes of one launch of the least squares and where the figure is
+    from: the capture itself at its size; on a larger mesh an estimate, in which
+    the reads grow with the cells and the polynomials are written out but for
+    what the capture left in L2 (as many bytes on any mesh)."""
+    m = LSQ_DRAM.get((workload, int(cfg.precision)))
+    if m is None or cfg.wenwrt != 1 or ncells < m["cells"]:
+        return None, None
+    if ncells == m["cells"]:
+        return m["read"] + m["written"], "ncu capture at this size"
+    g = table_size(cfg) * 5 * sum(nd for _, nd in lsq_rows(cfg))
+    left = g * m["cells"] - m["written"]
+    return m["read"] * ncells / m["cells"] + g * ncells - left, f"estimate from an ncu capture of {m['cells']} cells"
+
+
+def sets_per_cell(ncells, shared):
+    """Matrix sets that the least squares reads per cell: the shared sets once
+    (Engine.shared_sets), every other cell's own copy."""
+    return (ncells - shared["cells"] + shared["sets"]) / ncells
+
+
+def lsq_bytes_per_cell(cfg, per_cell):
     """Algorithmic bytes of the stencil least squares per cell: the
-    pseudo-inverse slices (times the distinct matrix sets per cell) and stencil
+    pseudo-inverse slices (times the matrix sets read per cell) and stencil
     indices of every stencil, the cell's own state, and the stencil polynomials
     G written (neighbour states come through L2; they are counted once, in the
     flux kernel)."""
-    from ucns3d_b200 import _native as N
-    s = 4 if cfg.precision == N.UCG_MIXED else 8
-    b = 5 * 8
-    for ll in range(cfg.admis_max):
-        low = cfg.ees == 5 and ll > 0
-        nk, nd = (cfg.imax2, cfg.ideg2) if low else (cfg.imax, cfg.ideg)
-        b += s * nk * nd * sets_per_cell + 4 * nk + s * nd * 5
-    return b
+    s = table_size(cfg)
+    return 5 * 8 + sum(s * nk * nd * per_cell + 4 * nk + s * nd * 5 for nk, nd in lsq_rows(cfg))
 
 
 def lsq_flops_per_cell(cfg):
     """Multiply-adds of the stencil least squares per cell, times two."""
-    return sum(10 * ((cfg.imax2 * cfg.ideg2) if cfg.ees == 5 and ll > 0 else cfg.imax * cfg.ideg)
-               for ll in range(cfg.admis_max))
+    return sum(10 * nk * nd for nk, nd in lsq_rows(cfg))
 
 
-def lsq_roofline(cfg, mesh, ncells, ms, peak, peak_kind, sm_mhz):
-    """The least squares against what bounds it: DRAM where the cells have
-    their own matrices, the FP32 (FP64) multiply-adds where they share sets
-    (nominal peak: 148 SMs x 128 (64) lanes at the SM clock)."""
+def lsq_roofline(cfg, ncells, shared, ms, peak, peak_kind, sm_mhz):
+    """The least squares against what bounds it, the longer of two times: its
+    bytes at the DRAM rate, or its FP32 (FP64) multiply-adds at the nominal peak
+    (148 SMs x 128 (64) lanes at the SM clock)."""
     from ucns3d_b200 import _native as N
-    share = mesh.ntables / ncells
-    bpc = lsq_bytes_per_cell(cfg, share)
+    bpc = lsq_bytes_per_cell(cfg, sets_per_cell(ncells, shared))
     hbm = bpc * ncells / (ms / 1000.0) / 1e9
-    if share > 0.5 or cfg.scheme == 2 and cfg.iorder == 1:
-        return {"bound": "hbm", "achieved": hbm, "peak": peak, "unit": "GB/s", "frac": hbm / peak,
-                "peak_kind": peak_kind, "nominal_peak": NOMINAL_HBM_GBS, "frac_nominal": hbm / NOMINAL_HBM_GBS,
-                "bytes_per_cell": bpc}
     lanes = 128 if cfg.precision == N.UCG_MIXED else 64
     top = 148 * lanes * 2 * sm_mhz * 1e6 / 1e12
     tf = lsq_flops_per_cell(cfg) * ncells / (ms / 1000.0) / 1e12
+    out = {"bytes_per_cell": bpc, "shared_cells": shared["cells"], "shared_sets": shared["sets"]}
+    if hbm / peak >= tf / top:
+        return {"bound": "hbm", "achieved": hbm, "peak": peak, "unit": "GB/s", "frac": hbm / peak,
+                "peak_kind": peak_kind, "nominal_peak": NOMINAL_HBM_GBS, "frac_nominal": hbm / NOMINAL_HBM_GBS, **out}
     return {"bound": "fma", "achieved": tf, "peak": top, "unit": "TFLOP/s", "frac": tf / top, "peak_kind": "nominal",
-            "hbm_gbs": hbm, "bytes_per_cell": bpc, "distinct_matrix_sets": mesh.ntables}
+            "hbm_gbs": hbm, **out}
 
 
-def recon_bytes_per_cell(cfg, sets_per_cell=1.0):
-    """Algorithmic bytes the reconstruction kernel must move per cell: the
-    pseudo-inverses and smoothness matrices (times the distinct matrix sets per
-    cell), stencil indices, face quadrature points and basis means of the cell,
+def recon_bytes_per_cell(cfg, per_cell):
+    """Algorithmic bytes the reconstruction kernels must move per cell: the
+    pseudo-inverses (times the matrix sets read per cell), the smoothness
+    matrix, stencil indices, face quadrature points and basis means of the cell,
     its own state and its face values written (neighbour state counted once,
-    in the flux kernel)."""
-    from ucns3d_b200 import _native as N
-    s = 4 if cfg.precision == N.UCG_MIXED else 8
+    in the flux kernel).  The kernels that read a shared smoothness matrix once
+    are those of IORDER 4 without CWENO and of characteristic variables; the
+    others read every cell's own copy."""
+    s = table_size(cfg)
     nq = max(cfg.nq_quad, cfg.nq_tri)
-    b = s * cfg.ideg * cfg.imax * cfg.admis_max * sets_per_cell + 4 * (cfg.imax + 1) * cfg.admis_max
+    b = sum(s * nk * nd * per_cell + 4 * (nk + 1) for nk, nd in lsq_rows(cfg))
     if cfg.scheme == 3:  # packed upper triangle of the smoothness matrix
-        b += s * cfg.ideg * (cfg.ideg + 1) // 2 * sets_per_cell
+        once = cfg.wenwrt == 2 or (cfg.iorder == 4 and cfg.ees != 5)
+        b += s * cfg.ideg * (cfg.ideg + 1) // 2 * (per_cell if once else 1.0)
     b += s * 6 * nq * 3 + s * cfg.ideg + 5 * 8
     b += s * 6 * nq * 5  # face values written
     return b
@@ -331,11 +354,12 @@ def run_gpu(args, case, ws, local, timed_e2e=True):
         t1 = time.perf_counter()
         e2e = dict(seconds=t1 - t0, bytes_in=nin.nbytes, bytes_out=nout.nbytes)
     nbytes_dev = eng.device_bytes
+    shared = eng.shared_sets()
     co = eng.cell_order()
     order = {"renumbered": co["renumbered"], "gather_cost_caller": co["cost_caller"], "gather_cost_rcm": co["cost_rcm"]}
     eng.close()
     return dict(ms=ms, kern=kern, state=state, clocks=clocks, launches=launches, e2e=e2e, device_bytes=nbytes_dev,
-                order=order)
+                order=order, shared=shared)
 
 
 def run_accuracy(case, local, steps):
@@ -797,14 +821,13 @@ def main():
     e2e_value = ws * ncells * 3 * args.steps / e2e_s
     # roofline of the stencil least squares, achieved from its CUDA-event
     # duration on the engine stream; the whole reconstruction beside it
-    share = c32.mesh.ntables / ncells
+    share = sets_per_cell(ncells, r32["shared"])
     table_bytes = lsq_bytes_per_cell(cfg32, share) * ncells  # tables, indices, polynomials: what a stage touches
     lsq_ms = r32["kern"]["lsq"]
     sm_mhz = (r32["clocks"] or {}).get("sm_mhz") or 1965.0
-    roof = lsq_roofline(cfg32, c32.mesh, ncells, lsq_ms, peak, peak_kind, sm_mhz)
+    roof = lsq_roofline(cfg32, ncells, r32["shared"], lsq_ms, peak, peak_kind, sm_mhz)
     rbpc = recon_bytes_per_cell(cfg32, share)
-    per_cell = LSQ_DRAM_BYTES_PER_CELL.get((args.case, int(cfg32.precision)))
-    traffic = per_cell * ncells if per_cell is not None and args.wenwrt == 1 else None
+    traffic, traffic_kind = lsq_traffic(args.case, cfg32, ncells)
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -815,7 +838,7 @@ def main():
                    "parallelism": f"replicas x{ws}",
                    "l2": ("inputs larger than L2 (stencils, tables, polynomials)" if table_bytes > L2_BYTES
                           else "inputs smaller than L2: not an HBM-roofline case")},
-        "roofline": {**roof, "traffic": traffic, "traffic_unit": "bytes per launch",
+        "roofline": {**roof, "traffic": traffic, "traffic_unit": "bytes per launch", "traffic_kind": traffic_kind,
                      "kernel": "stencil least squares", "kernel_ms": lsq_ms,
                      "reconstruction": {"kernels": recon_kernels(cfg32, args.wenwrt), "bytes_per_cell": rbpc,
                                         "ms": r32["kern"]["recon"],
@@ -838,7 +861,7 @@ def main():
         ra, rb = r64["state"][:, 0], r32["state"][:, 0]
         l2 = float(np.sqrt(np.mean((ra - rb) ** 2)) / np.sqrt(np.mean(ra ** 2)))
         linf = float(np.abs(ra - rb).max() / np.abs(ra).max())
-        roof64 = lsq_roofline(cfg64, c32.mesh, ncells, r64["kern"]["lsq"], peak, peak_kind, sm_mhz)
+        roof64 = lsq_roofline(cfg64, ncells, r64["shared"], r64["kern"]["lsq"], peak, peak_kind, sm_mhz)
         out["fp64"] = {"value": v64, "ms_per_step": ms64 / args.steps, "kernel_ms": r64["kern"],
                        "roofline_frac": roof64["frac"], "roofline_bound": roof64["bound"],
                        "mixed_speedup": value / v64,

@@ -274,11 +274,18 @@ int ucg_synchronize(ucg_engine* e);
  * evaluation.  For profiling; it leaves the state unchanged.               */
 int ucg_time_kernels(ucg_engine* e, int32_t reps, double* ms);
 
+/* Which cells share matrix sets: the cells whose least squares read the copy
+ * of a set that at least 32 cells share (ucg_recon.table_id of one upload),
+ * and the number of such sets; 0 and 0 where every cell reads its own tables.
+ * Either pointer may be NULL.  No counterpart in the reference. */
+int ucg_shared_sets(const ucg_engine* e, int64_t* cells, int64_t* sets);
+
 /* Bounded device waits.  The stencil least squares passes its tables and
  * gathered states through rings in shared memory, whose waits give up after
  * 65,536 polls (about 300 ns each, about 20 ms in all).  An engine created
  * with UCG_LSQ_WAIT=1 in the environment takes `polls` as its bound instead
- * (the default is restored by polls < 0), and so does one created with
+ * (the default, also the most with shared matrix sets, is restored by polls < 0),
+ * and so does one created with
  * UCG_LSQ_BULK=1, which reads every cell's own tables (no shared matrix sets).
  * A wait that gives up makes its block finish the copies it has in flight (each
  * with the default bound) and return without its results, and the next

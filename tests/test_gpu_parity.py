@@ -26,6 +26,7 @@ SMALL = {
     "weno5_hex": (lambda: Mesh.box_hex(12, 12, 12), SCHEME_WENO, 4, 0, EULER),
     "cweno4_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=5), SCHEME_WENO, 3, 5, EULER),
     "cweno4_ns_mixed": (lambda: Mesh.mixed_box(8, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES),
+    "cweno4_ns_mixed10": (lambda: Mesh.mixed_box(10, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES),
     "weno3_ns_hex": (lambda: Mesh.box_hex(8, 8, 8), SCHEME_WENO, 2, 0, NAVIER_STOKES),
     "muscl_bump": (lambda: Mesh.bump_channel(24, 10, 2, seed=2), SCHEME_MUSCL, 1, 0, EULER),
     "muscl_p2_hex": (lambda: Mesh.box_hex(8, 8, 8), SCHEME_MUSCL, 2, 0, EULER),
@@ -212,26 +213,30 @@ def test_device_dt_stepping_matches_host_dt():
     np.testing.assert_array_equal(a.get_state(), b.get_state())
 
 
-@pytest.mark.parametrize("name", ["weno5_hex", "cweno4_tet", "weno3_tet"])
+@pytest.mark.parametrize("name", ["weno5_hex", "cweno4_ns_mixed10", "weno3_ns_hex"])
 @pytest.mark.parametrize("precision", [N.UCG_FP64, N.UCG_MIXED])
 def test_bulk_copy_lsq_is_bitwise_equal(name, precision, monkeypatch):
-    """The opt-in least squares through the shared-memory bulk-copy ring
-    (UCG_LSQ_BULK=1 at engine creation) forms the same products in the same
-    order as the default kernel: residuals equal bit for bit."""
+    """Meshes whose cells share matrix sets, which the default engine reads from
+    shared memory (k_lsq_set, k_lsq_low), against every cell's own tables
+    through the bulk-copy ring (k_lsq_ring, UCG_LSQ_BULK=1 at engine creation):
+    the same products in the same order, residuals equal bit for bit."""
     m, cfg, U = _setup(name, precision)
-    out = []
+    out, shared = [], []
     for bulk in ("0", "1"):
         monkeypatch.setenv("UCG_LSQ_BULK", bulk)
         e = Engine(m, cfg)
         e.set_state(U)
         out.append(e.residual())
+        shared.append(e.shared_sets()["cells"])
         e.check_health()
         e.close()
+    assert shared[0] > m.ncells // 2 and shared[1] == 0  # two different kernels
     assert np.array_equal(out[0], out[1])
 
 
 def test_bulk_copy_wait_timeout_is_reported_and_recoverable(monkeypatch):
-    """The bounded waits of the opt-in bulk-copy least squares: with a wait
+    """The bounded waits of the least squares through the bulk-copy ring
+    (UCG_LSQ_BULK=1: every cell's own tables): with a wait
     limit of 0 polls every stage wait gives up, the warps drain their copies
     in flight and return, ucg_check_health reports UCG_ETIMEOUT, and with the
     default limit restored the same handle gives the normal residual bit for

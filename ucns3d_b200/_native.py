@@ -156,7 +156,7 @@ ENGINE_SYMBOLS = [
     "ucg_tangent_run", "ucg_time_adjoint", "ucg_cell_order", "ucg_adjoint_run_obj", "ucg_tangent_run_obj",
     "ucg_set_wait_limit", "ucg_mood_state", "ucg_build_recon", "ucg_implicit_step",
     "ucg_dual_time_step", "ucg_rk3_stage", "ucg_halo_set", "ucg_halo_pack", "ucg_halo_unpack",
-    "ucg_set_cell_roles", "ucg_dual_time_step_explicit", "ucg_wall_loads",
+    "ucg_set_cell_roles", "ucg_dual_time_step_explicit", "ucg_wall_loads", "ucg_shared_sets",
 ]
 
 
@@ -226,6 +226,8 @@ def engine() -> C.CDLL:
         lib.ucg_tangent_run_obj.argtypes = [vp, C.c_int32, C.c_int32, C.c_double, _f64p, _f64p, _f64p, _f64p]
         lib.ucg_set_wait_limit.restype = C.c_int
         lib.ucg_set_wait_limit.argtypes = [vp, C.c_int64]
+        lib.ucg_shared_sets.restype = C.c_int
+        lib.ucg_shared_sets.argtypes = [vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
         lib.ucg_cell_order.restype = C.c_int
         lib.ucg_cell_order.argtypes = [vp, C.POINTER(C.c_int32), C.POINTER(C.c_int32), _f64p]
         lib.ucg_mood_state.restype = C.c_int

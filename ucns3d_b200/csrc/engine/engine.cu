@@ -972,6 +972,7 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
   std::vector<int32_t> tcell((size_t)ntile * SET_TILE, -1), tset((size_t)ntile);
   std::vector<int8_t> tiled((size_t)e->n, 0);
   e->all_tiled = true;
+  e->ntiled = 0;
   for (int64_t i = 0; i < n; ++i) {
     const int32_t s = set_of[table(i)];
     if (s < 0) {
@@ -981,6 +982,7 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
     tset[(size_t)(at[s] / SET_TILE)] = s;
     tcell[(size_t)at[s]++] = (int32_t)i;
     tiled[(size_t)i] = 1;
+    e->ntiled++;
   }
   int64_t off = 0;
   for (int ll = 0; ll < c.admis_max; ++ll) {
@@ -1399,6 +1401,13 @@ int ucg_mood_state(ucg_engine* e, int32_t* order, int32_t* recalc) {
 int ucg_set_wait_limit(ucg_engine* e, int64_t polls) {
   if (!e) return UCG_EINVAL;
   e->lsq_wait = polls < 0 ? -1 : (long)polls;
+  return UCG_OK;
+}
+
+int ucg_shared_sets(const ucg_engine* e, int64_t* cells, int64_t* sets) {
+  if (!e) return UCG_EINVAL;
+  if (cells) *cells = e->ntile ? e->ntiled : 0;
+  if (sets) *sets = e->ntile ? e->nset : 0;
   return UCG_OK;
 }
 

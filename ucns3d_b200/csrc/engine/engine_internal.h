@@ -56,7 +56,7 @@ struct ucg_engine {
   // matrix sets shared by many cells (plan_sets): tiles of cells, each set's
   // matrices once, the groups with cells that are not tiled
   DevBuf tcell, tset, tiled, setmat, setind, gset, ugrp;
-  int64_t ntile = 0, nset = 0, sstride = 0, nugrp = 0;
+  int64_t ntile = 0, ntiled = 0, nset = 0, sstride = 0, nugrp = 0;
   int sso[8] = {0};
   bool all_tiled = false;
   // scratch and state

@@ -250,6 +250,15 @@ class Engine:
         self._check(self.lib.ucg_cell_order(self._h, C.byref(ren), N.ptr(n2o, C.c_int32), N.ptr(cost, C.c_double)))
         return dict(renumbered=bool(ren.value), n2o=n2o, cost_caller=float(cost[0]), cost_rcm=float(cost[1]))
 
+    def shared_sets(self) -> dict:
+        """The cells whose least squares read a matrix set that many cells
+        share, and the number of such sets (0 where every cell reads its own
+        tables)."""
+        v = (C.c_int64 * 2)()
+        self._check(self.lib.ucg_shared_sets(self._h, C.cast(C.byref(v, 0), C.POINTER(C.c_int64)),
+                                             C.cast(C.byref(v, 8), C.POINTER(C.c_int64))))
+        return dict(cells=int(v[0]), sets=int(v[1]))
+
     def implicit_step(self, cfl: float, nsteps: int = 1, nsweeps: int = 10):
         """`nsteps` implicit pseudo-time steps toward the steady state
         (IMPLICIT_TIMEs with `nsweeps` relaxation sweeps)."""
