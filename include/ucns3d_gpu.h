@@ -284,9 +284,9 @@ int ucg_shared_sets(const ucg_engine* e, int64_t* cells, int64_t* sets);
  * gathered states through rings in shared memory, whose waits give up after
  * 65,536 polls (about 300 ns each, about 20 ms in all).  An engine created
  * with UCG_LSQ_WAIT=1 in the environment takes `polls` as its bound instead
- * (the default, also the most with shared matrix sets, is restored by polls < 0),
- * and so does one created with
- * UCG_LSQ_BULK=1, which reads every cell's own tables (no shared matrix sets).
+ * (at most the default with shared matrix sets; the default is restored by
+ * polls < 0), and so does one created with UCG_LSQ_BULK=1, which reads every
+ * cell's own tables (no shared matrix sets).
  * A wait that gives up makes its block finish the copies it has in flight (each
  * with the default bound) and return without its results, and the next
  * ucg_check_health reports UCG_ETIMEOUT; the handle stays usable.

@@ -160,17 +160,14 @@ __global__ void __launch_bounds__(32 * muscl_warps<NS>(), NS ? 4 : 7) k_muscl(Pr
 }
 
 // ======================================================================
-// Face fluxes fused with the RK stage update.  Eight lanes per cell, lane f
-// integrates face f; the face sums are added in face order
-// (CALCULATE_FLUXESHI_CONVECTIVE flux_p.f90:478, CALCULATE_FLUXESHI_DIFFUSIVE
-// flux_p.f90:1520), then RUNGE_KUTTA3 (time_p.f90:885-1027).
-// MODE 0: write the residual; MODE 1/2/3: RK stage 1/2/3.
+// Face fluxes (CALCULATE_FLUXESHI_CONVECTIVE flux_p.f90:478,
+// CALCULATE_FLUXESHI_DIFFUSIVE flux_p.f90:1520), k_face; their sum per cell in
+// face order with the RK stage, k_update.
 // ======================================================================
 // One thread per owned face (the cell with the smaller index, or the only
 // cell of a boundary face): the Riemann flux RK (iRiemann: 1 HLLC, 2
 // Rusanov, 3 Roe, 4 rotated Roe-HLL, 5 t-Roe, 9 HLL) and viscous fluxes over the
-// face's points,
-// weighted by w_q * area.  The neighbour's face gets the negated sums: HLLC
+// face's points, weighted by w_q * area.  The neighbour's face gets the negated sums: HLLC
 // and the viscous flux are antisymmetric under swapping the two states and
 // flipping the normal, so each interior face is evaluated once instead of
 // twice as in the reference's per-cell loop.

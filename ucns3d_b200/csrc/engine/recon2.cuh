@@ -6,14 +6,17 @@
 //   k_lsq_set   cells that share a matrix set, tiled (and k_lsq_low, the
 //               CWENO directional stencils of those cells)
 // CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL, MUSCL
-// fall-back, CHECKSOLX (3126-3406): k_wpost, one lane per cell, no block
-// barriers, smoothness indicators as packed quadratic forms; at IORDER 4
-// k_wis / k_wis_set and k_wface; characteristic variables k_char_forms and
-// k_char_face.
+// fall-back, CHECKSOLX (3126-3406):
+//   k_wface     conserved variables, one warp per variable: IORDER 4 with the
+//               indicators of k_wis / k_wis_set, IORDER 1-2 and small meshes
+//               at IORDER 3 with its own
+//   k_char_forms, k_char_face  characteristic variables
+//   k_wpost     one lane per cell: the MUSCL fall-back of the cells that the
+//               above flag; alone at IORDER 3 on large meshes and for
+//               high-order MUSCL
 #pragma once
 
 #include "device.cuh"
-
 
 namespace ucg {
 
@@ -609,8 +612,8 @@ cudaError_t launch_lsq_low(const Problem& p, const double* U, cudaStream_t st) {
   return cudaGetLastError();
 }
 // The tiled cells' indicators come from k_wis_set: IORDER 4 (the only order
-// with indicators of their own kernel), WENO (CWENO's central polynomial needs
-// the other stencils first).
+// with indicators of their own kernel) without CWENO, whose central polynomial
+// (the central stencil less the directional ones) only k_wis forms.
 template <int P>
 bool sets_give_is(const Problem& p) {
   return P == 4 && p.ntile && p.isb && p.scheme == 3 && p.ees != 5;
@@ -809,10 +812,11 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
 // by load latency at 12 warps per SM: WENO3, 82,944 tetrahedra FP64 0.190 ->
 // 0.131 ms, mixed 0.103 -> 0.099, 64,000 hexahedra mixed 0.118 -> 0.094, 3,072
 // tetrahedra FP64 0.044 -> 0.028.  At IORDER 3 it wins only where k_wpost's
-// blocks leave SMs idle, below a block of 128 per SM (CWENO4, 9,728 cells FP64
-// 0.156 -> 0.089 ms, mixed 0.075 -> 0.044); above, reading the triangles in
-// five warps costs more than it hides (271,872 cells mixed 0.564 -> 0.626,
-// 24,576 FP64 0.133 -> 0.139).
+// blocks leave SMs idle, below a block of 128 per SM, 18,944 cells (CWENO4, 9,728
+// cells FP64 0.156 -> 0.089 ms, mixed 0.075 -> 0.044; 16,464 tetrahedra 0.114 ->
+// 0.099, 0.061 -> 0.052; WENO4, 17,576 hexahedra 0.189 -> 0.127, 0.093 -> 0.067);
+// above, reading the triangles in five warps costs more than it hides (271,872
+// cells mixed 0.564 -> 0.626, 24,576 FP64 0.133 -> 0.139).
 template <typename T>
 __host__ __device__ constexpr size_t wface_smem(int QS) {
   return ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
@@ -1008,8 +1012,8 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
 // sum_d m_d(x) g_d - sum_d mean(m_d) g_d: the second sum is formed once per
 // polynomial instead of subtracting the basis means at every face point.
 // ISB: the indicators come from k_wis (p.isb) instead of being formed here.
-// FB: only the cells that k_wface marked in p.wflag, straight to the MUSCL
-// fall-back (the others return at once).  MU (with FB): the first MOOD
+// FB: only the cells that k_wface or k_char_face marked in p.wflag, straight to
+// the MUSCL fall-back (the others return at once).  MU (with FB): the first MOOD
 // cascade, MUSCL on the cells of p.mmus without CHECKSOLX (MUSCL of
 // MOOD_OPERATOR_2, mood.f90:353).
 // Under MOOD (p.mprev) every cell is reconstructed; a reduced cell (CHECKSOL,
@@ -1017,11 +1021,12 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
 // recomputed it (RECALC, reconstruct_p.f90:2306-2315), else it keeps its
 // WENO values and only CHECKSOLX; the reduced flags go to p.wflag.
 // Three blocks of 128 per SM where that measured faster than the two that
-// the kernel's registers otherwise allow: IORDER 2 (WENO3 tets, 82,944
-// cells: 1.109 -> 1.083 ms per step mixed, 1.585 -> 1.540 FP64) and IORDER 3
-// in FP32 (2.1 M-cell CWENO4 Navier-Stokes: 52.7 -> 51.2 ms; in FP64 the
-// bound made the 647 k-cell step 31.8 -> 33.8 ms, so FP64 keeps two; four
-// blocks in FP32 made it 56.0 -> 57.6 ms on another box).
+// the kernel's registers otherwise allow: IORDER 3 in FP32 (2.1 M-cell CWENO4
+// Navier-Stokes step 52.7 -> 51.2 ms; in FP64 the bound made the 647 k-cell
+// step 31.8 -> 33.8 ms, so FP64 keeps two; 271,872 cells in FP32: 0.557 ms with
+// three, 0.577 with two, 0.619 with four), and IORDER 2 (high-order MUSCL and
+// the fall-back; measured with the whole reconstruction of 82,944 WENO3 tets,
+// before k_wface took it: 1.109 -> 1.083 ms per step mixed, 1.585 -> 1.540 FP64).
 template <int P, typename T, bool ISB = false, bool FB = false, bool MU = false>
 __global__ void __launch_bounds__(128, P == 2 || (P == 3 && sizeof(T) == 4) ? 3 : 1)
     k_wpost(Problem p, const double* __restrict__ U) {
@@ -1952,7 +1957,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
     // triangle (595 entries) no longer stays in L1 between the stencils of
     // one lane (64^3 WENO5: FP64 stage 17.2 -> 15.5 ms, mixed 7.80 -> 7.67 ms);
     // at IORDER 2-3 the triangle is small and the extra kernel costs more
-    // than it saves (2.1 M-cell CWENO4: 17.3 -> 19.6 ms)
+    // than it saves (2.1 M-cell CWENO4, every cell's own triangle: 17.3 -> 19.6 ms)
     bool done = false;
     const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
     const size_t smem = wface_smem<T>(QS);
