@@ -1018,9 +1018,7 @@ void launch_visc_jvp_t(const Problem& p, const double* U, const double* dU, doub
   Problem pt = p;
   pt.gv = dgv;
   pt.fgrad = tfg;
-  const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
-  const int64_t nfp = p.nown * QS;
-  k_visc_facegrad<P, double><<<(unsigned)((nfp + 127) / 128), 128, 0, st>>>(pt);
+  launch_visc_facegrad<P, double>(pt, st);
 }
 
 template <int P, int ND, bool LOW>

@@ -1537,15 +1537,8 @@ __device__ __forceinline__ void visc_point_grad(const Problem& p, int64_t c, int
   }
 }
 
-// Without bounds the compiler keeps to the 64 registers of a 1,024-thread
-// block: WENO5 FP64 (8,000 cells) spilled, reconstruction after the least
-// squares 3.13 -> 0.25 ms, WENO5 mixed (13,824) 0.57 -> 0.21, CWENO4 FP64
-// (271,872) 2.30 -> 2.07.  Blocks per SM: FP32 8 (CWENO4, 271,872 cells: 0.388 ms
-// at one, 0.330 at six, 0.314 at eight, 0.360 at ten), FP64 5 (WENO5 0.244 to
-// 0.247 ms at three to five, 0.270 at eight; CWENO4 2.14, 2.09, 2.07, 2.06 at
-// three, four, five and eight).
 template <int P, typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 5) k_visc_facegrad(Problem p) {
+__device__ __forceinline__ void visc_facegrad(const Problem& p) {
   const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = t / QS;
@@ -1568,6 +1561,27 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 5) k_visc_facegrad(P
 #pragma unroll
   for (int k = 0; k < 6; ++k)
     o[k] = make_double2((double)((gl[2 * k] + gr[2 * k]) / T(2)), (double)((gl[2 * k + 1] + gr[2 * k + 1]) / T(2)));
+}
+// FP64 with the registers that the compiler takes (80 below IORDER 4, 128 there):
+// bounded to five blocks per SM it took 96 and at IORDER 4 spilled (reconstruction
+// after the least squares, CWENO4, 271,872 cells 2.065 against 2.026 ms; WENO3, 48^3
+// 0.335, 0.326; WENO5, 24^3 0.367, 0.358).  FP32 eight blocks per SM: CWENO4,
+// 271,872 cells 1.037 ms against 1.050 unbounded, WENO4, 32^3 0.221, 0.224, WENO3,
+// 48^3 0.244, 0.241.
+template <int P>
+__global__ void k_visc_facegrad(Problem p) {
+  visc_facegrad<P, double>(p);
+}
+template <int P>
+__global__ void __launch_bounds__(128, 8) k_visc_facegrad_f32(Problem p) {
+  visc_facegrad<P, float>(p);
+}
+template <int P, typename T>
+void launch_visc_facegrad(const Problem& p, cudaStream_t st) {
+  const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
+  const unsigned b = (unsigned)((p.nown * QS + 127) / 128);
+  if constexpr (sizeof(T) == 4) k_visc_facegrad_f32<P><<<b, 128, 0, st>>>(p);
+  else k_visc_facegrad<P><<<b, 128, 0, st>>>(p);
 }
 
 // CHARACTERISTIC_RECONSTRUCTION (src/reconstruct_p.f90:497-758): per face, the
@@ -2000,8 +2014,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
       k_visc_lsq<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
     }
     *launches += 2;
-    const int64_t nfp = p.nown * QS;
-    k_visc_facegrad<P, T><<<(unsigned)((nfp + 127) / 128), 128, 0, st>>>(p);
+    launch_visc_facegrad<P, T>(p, st);
     *launches += 1;
   }
   return cudaGetLastError();
