@@ -119,3 +119,38 @@ def test_wait_timeout_is_reported_and_recoverable(name, precision, monkeypatch):
     assert e.lib.ucg_set_wait_limit(e._h, -1) == N.UCG_OK
     assert np.array_equal(e.residual(), ref)
     e.check_health()
+
+
+@pytest.mark.parametrize("precision", [N.UCG_FP64, N.UCG_MIXED])
+@pytest.mark.parametrize("ees", [0, 5])
+@pytest.mark.parametrize("mesh", ["hex", "hex_large", "tet", "mixed"])
+def test_iorder1_large_meshes(mesh, ees, precision, monkeypatch):
+    """IORDER 1 from 128 cells per SM on: the least squares one lane per cell
+    (k_lsq_lane) against the ring (UCG_LSQ_BULK=1), bit for bit.  Tiles only
+    without CWENO, below 512 cells per SM and where the cells of a set follow
+    one another (a box of hexahedra)."""
+    import torch
+
+    mk = {"hex": lambda: Mesh.box_hex(27, 27, 29), "tet": lambda: Mesh.box_tet(15, 15, 15, seed=2),
+          "hex_large": lambda: Mesh.box_hex(43, 43, 41), "mixed": lambda: Mesh.mixed_box(20, seed=4)}[mesh]
+    m = mk().prepare(SCHEME_WENO, 1, ees)
+    per_sm = m.ncells / torch.cuda.get_device_properties(0).multi_processor_count
+    assert per_sm >= 512 if mesh == "hex_large" else 128 <= per_sm < 512
+    cfg = make_config(m, governing=EULER, precision=precision, pres=5.0)
+    x = m.centres()
+    U = m.initial_condition(IC_TGV, [1.4, 5.0, 1.0])
+    U = U * (1.0 + 0.02 * np.sin(1.3 * x[:, :1] + 0.7 * x[:, 1:2] + 2.1 * x[:, 2:3] + np.arange(5.0)))
+    out = []
+    for bulk in ("0", "1"):
+        monkeypatch.setenv("UCG_LSQ_BULK", bulk)
+        e = Engine(m, cfg)
+        assert e.shared_sets()["cells"] == (m.ncells if mesh == "hex" and not ees and bulk == "0" else 0)
+        e.set_state(U)
+        r = [e.residual()]
+        if precision == N.UCG_FP64:
+            r.append(e.residual_jvp(U * 1e-2))
+        e.check_health()
+        e.close()
+        out.append(r)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -101,6 +101,7 @@ struct Problem {
   double* fflux;            // [n][MF][NV] convective face sums (owner and negated copy)
   double* vflux;            // [n][MF][NV] viscous face sums
   unsigned* health;
+  bool lsq_bulk; // every cell's least squares through k_lsq_ring
   long lsq_wait; // polls of a stage wait of k_lsq_ring and k_lsq_set before it gives up (< 0: the default)
   int nsm;       // SMs of the device
   int wenwrt;    // 1 conserved-variable WENO, 2 characteristic-variable WENO

@@ -163,6 +163,7 @@ Problem make_problem(ucg_engine* e) {
   p.dt_next = nullptr;
   p.ccfl = 0.0;
   p.nsm = e->nsm;
+  p.lsq_bulk = e->lsq_bulk;
   p.lsq_wait = e->lsq_bulk || e->lsq_limit ? e->lsq_wait : -1;
   p.wenwrt = c.wenwrt;
   p.riemann = c.riemann;
@@ -929,7 +930,11 @@ namespace {
 // device order.  set_of gets each table's set, -1 where its cells read their
 // own tables.  None where the rows of a stencil do not fit in shared memory
 // (k_lsq_set with its rings takes the most of it; IORDER 4 from 701 members in
-// FP64, 1,465 in FP32): k_lsq_ring takes any number.  Kept only where it pays:
+// FP64, 1,465 in FP32): k_lsq_ring takes any number.  At IORDER 1, whose sets are
+// smaller than what a block sets up for them, only where a tile's cells follow one
+// another in memory, without CWENO and below 512 cells per SM (14,580 mixed cells,
+// 5.4 groups a warp: 28 us tiled, 20 through the ring; hexahedra 13,824: 17, 19;
+// 32,768: 26, k_lsq_lane 33; 110,592: 77, 71).  Kept only where it pays:
 // a tile is taken to cost three fifths of what its 128 cells cost k_lsq_ring,
 // which costs the same for a group of 32 cells whether one or all of them are
 // left to it.  Measured, all cells tiled against all through the ring: WENO5
@@ -943,7 +948,7 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
   const bool perm = !e->n2o.empty();
   const int64_t vec = e->mixed ? 4 : 2, ts = (int64_t)tsize(e);
   auto row = [&](int nd) { return (nd + vec - 1) / vec * vec; };
-  if ((c.imax * row(c.ideg) + SET_RING) * ts > (int64_t)SET_SMEM ||
+  if ((c.iorder == 1 && (c.ees == 5 || n >= (int64_t)e->nsm * 512)) || (c.imax * row(c.ideg) + SET_RING) * ts > (int64_t)SET_SMEM ||
       (c.ees == 5 && c.admis_max > 1 && c.imax2 * row(c.ideg2) * ts > (int64_t)LOW_SMEM))
     return UCG_OK;
   auto table = [&](int64_t cell) { return table_id[perm ? e->n2o[cell] : cell]; };
@@ -971,6 +976,10 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
   }
   std::vector<int32_t> tcell((size_t)ntile * SET_TILE, -1), tset((size_t)ntile);
   std::vector<int8_t> tiled((size_t)e->n, 0);
+  // 32-cell groups that the tiles' warps touch: one each where the cells of a
+  // set follow one another
+  std::vector<int64_t> grp((size_t)nset, -1);
+  int64_t warps = 0, touched = 0;
   e->all_tiled = true;
   e->ntiled = 0;
   for (int64_t i = 0; i < n; ++i) {
@@ -980,9 +989,16 @@ int plan_sets(ucg_engine* e, const int32_t* table_id, int64_t ntab, std::vector<
       continue;
     }
     tset[(size_t)(at[s] / SET_TILE)] = s;
+    if (at[s] % 32 == 0) ++warps, grp[(size_t)s] = -1;
+    if (grp[(size_t)s] != i >> 5) ++touched, grp[(size_t)s] = i >> 5;
     tcell[(size_t)at[s]++] = (int32_t)i;
     tiled[(size_t)i] = 1;
     e->ntiled++;
+  }
+  e->tiles_together = touched <= 2 * warps;
+  if (c.iorder == 1 && !e->tiles_together) {
+    set_of.clear();
+    return UCG_OK;
   }
   int64_t off = 0;
   for (int ll = 0; ll < c.admis_max; ++ll) {

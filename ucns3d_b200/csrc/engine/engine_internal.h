@@ -59,6 +59,7 @@ struct ucg_engine {
   int64_t ntile = 0, ntiled = 0, nset = 0, sstride = 0, nugrp = 0;
   int sso[8] = {0};
   bool all_tiled = false;
+  bool tiles_together = false;  // the cells of a tile's warps lie in at most two 32-cell groups on average
   // scratch and state
   DevBuf gbuf, isb, wflag, dul, ulv, fgrad, gv, prim, rhs, Un, Ua, Ub, health, dt, partial, red, staging, own, fflux, vflux, qbuf;
   // MOOD (cfg.mood): RECALC, the cascade's flags and selections, MOOD_O, the candidate state

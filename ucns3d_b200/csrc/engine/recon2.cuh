@@ -5,6 +5,7 @@
 //               shared memory (interleaved over groups of 32 cells)
 //   k_lsq_set   cells that share a matrix set, tiled (and k_lsq_low, the
 //               CWENO directional stencils of those cells)
+//   k_lsq_lane  IORDER 1 on large meshes, one lane per cell
 // CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL, MUSCL
 // fall-back, CHECKSOLX (3126-3406):
 //   k_wface     conserved variables, one warp per variable: IORDER 4 with the
@@ -582,6 +583,64 @@ __global__ void __launch_bounds__(256, Ring<P, T>::BPS) k_lsq_ring(Problem p, co
   }
 }
 
+// LEAST_SQUARES at IORDER 1, one lane per cell: three rows a stencil are so
+// little that the accumulators leave room for the loads, and what a block of
+// k_lsq_ring or k_lsq_set sets up before its first product does not pay.  From 128
+// cells per SM on (below, one wave of lanes waits for its own loads: 512 cells 15
+// us, the ring 11; 8,000 17, 15).  In FP64 and FP32: 114,048 mixed cells WENO 64 and
+// 57 us, the ring 96 and 92, tiles 109 and 80, CWENO 66 and 56, 89 and 83, 109 and
+// 91; 33,408 cells 33 and 22, 36 and 31, 41 and 34.
+template <int P, typename T>
+__global__ void __launch_bounds__(128, 1) k_lsq_lane(Problem p, const double* __restrict__ U) {
+  constexpr int ID = Deg<P>::ideg;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int A = p.admis_max, W = p.imax + 1;
+  const int64_t grp = c >> 5;
+  const int lane = (int)(c & 31);
+  const bool live = c < p.n;
+  const int adm = live ? p.admis[c] : 0;
+  double u0[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) u0[v] = live ? U[c * NV + v] : 0.0;
+  const T* Mi = (const T*)p.invmat + grp * p.tstride * 32 + lane;
+  const int32_t* Si = p.sten + grp * (int64_t)(A * W) * 32 + lane;
+  T* Gi = (T*)p.gbuf + grp * (int64_t)(A * ID * NV) * 32 + lane;
+  for (int ll = 0; ll < A; ++ll) {
+    const bool low = p.ees == 5 && ll > 0;
+    const int nk = low ? p.imax2 : p.imax, nd = low ? p.ideg2 : ID;
+    T acc[ID][NV];
+#pragma unroll
+    for (int d = 0; d < ID; ++d)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[d][v] = T(0);
+    if (ll < adm) {
+      const T* M = Mi + (int64_t)p.soff[ll] * 32;
+      const int32_t* S = Si + (ll * W + 1) * 32;
+#pragma unroll 2
+      for (int k = 0; k < nk; ++k) {
+        const double* uy = U + (int64_t)S[k * 32] * NV;
+        T du[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) du[v] = T(uy[v] - u0[v]);
+        const T* Mk = M + (int64_t)k * nd * 32;
+#pragma unroll
+        for (int d = 0; d < ID; ++d)
+          if (d < nd) {
+            const T m = Mk[d * 32];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[d][v] += m * du[v];
+          }
+      }
+    }
+    if (live)
+#pragma unroll
+      for (int d = 0; d < ID; ++d)
+        if (d < nd)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Gi[(int64_t)((ll * ID + d) * NV + v) * 32] = acc[d][v];
+  }
+}
+
 // the cells' own tables: all groups, or those with cells that are not tiled
 template <int P, typename T>
 cudaError_t launch_lsq_ring(const Problem& p, const double* U, cudaStream_t st) {
@@ -641,6 +700,12 @@ cudaError_t launch_lsq_set(const Problem& p, const double* U, cudaStream_t st, i
 template <int P, typename T>
 cudaError_t launch_lsq(const Problem& p, const double* U, cudaStream_t st, int64_t* launches) {
   ++*launches;
+  if constexpr (P == 1) {
+    if (!p.lsq_bulk && !p.ntile && p.n >= (int64_t)p.nsm * 128) {
+      k_lsq_lane<P, T><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, U);
+      return cudaGetLastError();
+    }
+  }
   return p.ntile ? launch_lsq_set<P, T>(p, U, st, launches) : launch_lsq_ring<P, T>(p, U, st);
 }
 
