@@ -271,9 +271,9 @@ def recon_kernels(cfg, wenwrt):
         return "least squares + k_char_forms + k_char_face + k_wpost fall-back"
     if cfg.scheme == 3 and cfg.iorder == 4:
         return "least squares + indicators + k_wface + k_wpost fall-back"
-    if cfg.scheme == 3 and cfg.iorder < 3:
-        return "least squares + k_wface + k_wpost fall-back"
-    return "least squares + k_wpost (small meshes at IORDER 3: k_wface)"
+    if cfg.scheme == 3:
+        return "least squares + k_wpost, or k_wface + k_wpost fall-back (by order, precision and cells per SM)"
+    return "least squares + k_wpost"
 
 
 L2_BYTES = 126 * 2 ** 20

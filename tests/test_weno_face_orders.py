@@ -2,9 +2,9 @@
 k_wpost's MUSCL fall-back of the cells it flags) against one lane per cell
 (k_wpost, UCG_WENO_FACE=0), bit for bit: both take the same operations in the
 same order.  Cell counts leave part of the last group of 32 unused; the cells
-beside a pressure jump take the fall-back; a mesh of more than 128 cells per
-SM lies on the other side of the rule at IORDER 3, where both engines run
-k_wpost."""
+beside a pressure jump take the fall-back; meshes on both sides of the rule
+(wface_own), beyond which both engines run k_wpost: more than 128 cells per SM
+at IORDER 3, 192 at IORDER 1 (FP64; never in the mixed form) and 2 (mixed form)."""
 import numpy as np
 import pytest
 
@@ -23,7 +23,17 @@ CASES = {
     "cweno4_z_tet": (lambda: Mesh.box_tet(7, 7, 7, seed=9), 3, 5, EULER, {"wenoz": 1}),
     "weno4_hex": (lambda: Mesh.box_hex(9, 9, 11), 3, 0, EULER, {}),
     "weno4_hex_large": (lambda: Mesh.box_hex(28, 28, 25), 3, 0, EULER, {}),
+    "weno2_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=3), 1, 0, EULER, {}),
+    "cweno2_hex": (lambda: Mesh.box_hex(9, 9, 11), 1, 5, EULER, {}),
+    "weno2_hex_large": (lambda: Mesh.box_hex(31, 31, 31), 1, 0, EULER, {}),
+    "weno3_hex_large": (lambda: Mesh.box_hex(31, 31, 31), 2, 0, EULER, {}),
 }
+
+
+def _lanes(name, precision):
+    """Both engines take one lane per cell."""
+    return (name in ("weno4_hex_large", "weno2_hex_large") or
+            (precision == N.UCG_MIXED and name in ("weno2_tet", "cweno2_hex", "weno3_hex_large")))
 
 
 @pytest.mark.parametrize("precision", [N.UCG_FP64, N.UCG_MIXED])
@@ -53,4 +63,4 @@ def test_warp_per_variable_equals_lane_per_cell(name, jump, precision, monkeypat
         e.close()
     assert np.array_equal(out[0], out[1])
     # the fall-back is a launch of its own behind k_wface
-    assert launches[0] - launches[1] == (0 if name == "weno4_hex_large" else 1)
+    assert launches[0] - launches[1] == (0 if _lanes(name, precision) else 1)

@@ -9,12 +9,12 @@
 // CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), CHECKSOL, MUSCL
 // fall-back, CHECKSOLX (3126-3406):
 //   k_wface     conserved variables, one warp per variable: IORDER 4 with the
-//               indicators of k_wis / k_wis_set, IORDER 1-2 and small meshes
-//               at IORDER 3 with its own
+//               indicators of k_wis / k_wis_set, below with its own where
+//               that is faster (wface_own)
 //   k_char_forms, k_char_face  characteristic variables
 //   k_wpost     one lane per cell: the MUSCL fall-back of the cells that the
-//               above flag; alone at IORDER 3 on large meshes and for
-//               high-order MUSCL
+//               above flag; alone where k_wface is not taken and for high-order
+//               MUSCL
 #pragma once
 
 #include "device.cuh"
@@ -871,17 +871,9 @@ __global__ void __launch_bounds__(224) k_wis(Problem p) {
 // Weights, combination and face values take k_wpost's operations in
 // k_wpost's order.  Under MOOD the cells that are not FULL are reconstructed
 // too (over their admissible stencils) and marked.
-// OWN (IORDER 1-3): each warp forms its variable's indicators itself, g^T S g
-// of one polynomial at a time from the cells' triangles, which the five warps
-// read from L1.  One lane per cell with all five variables (k_wpost) is bound
-// by load latency at 12 warps per SM: WENO3, 82,944 tetrahedra FP64 0.190 ->
-// 0.131 ms, mixed 0.103 -> 0.099, 64,000 hexahedra mixed 0.118 -> 0.094, 3,072
-// tetrahedra FP64 0.044 -> 0.028.  At IORDER 3 it wins only where k_wpost's
-// blocks leave SMs idle, below a block of 128 per SM, 18,944 cells (CWENO4, 9,728
-// cells FP64 0.156 -> 0.089 ms, mixed 0.075 -> 0.044; 16,464 tetrahedra 0.114 ->
-// 0.099, 0.061 -> 0.052; WENO4, 17,576 hexahedra 0.189 -> 0.127, 0.093 -> 0.067);
-// above, reading the triangles in five warps costs more than it hides (271,872
-// cells mixed 0.564 -> 0.626, 24,576 FP64 0.133 -> 0.139).
+// OWN (IORDER 1-3, where wface_own says so): each warp forms its variable's
+// indicators itself, g^T S g of one polynomial at a time from the cells'
+// triangles, which the five warps read from L1.
 template <typename T>
 __host__ __device__ constexpr size_t wface_smem(int QS) {
   return ((size_t)MF * QS * 3 + ((QS * NV) | 1)) * 32 * sizeof(T);
@@ -1068,6 +1060,32 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
   if (tid < ncl) p.wflag[grp * 32 + tid] = (int8_t)s_flag[tid];
 }
 
+// Whether k_wface takes the face values below IORDER 4, rather than k_wpost's one
+// lane per cell with all five variables.  k_wpost is bound by load latency at 12
+// warps per SM and wins where its work per cell is small and its blocks fill the
+// SMs: then five warps that read the triangles and form the monomials again cost
+// more than they hide.  Times k_wpost -> k_wface in us:
+//   IORDER 2 FP64, always: 8,000 hexahedra 70 -> 32, 262,144 679 -> 398, 48,000
+//     tetrahedra 104 -> 94, 82,944 190 -> 131, 271,872 mixed cells (CWENO) 571 -> 526
+//     (mixed meshes of 20,000 to 80,000 cells, whose cells without full stencils
+//     then wait for the fall-back's launch, lose up to 13 %: 33,408 150 -> 172)
+//   IORDER 2 FP32, below 192 cells per SM (28,416): 8,000 39 -> 30, 24,389 49 -> 44,
+//     tetrahedra 24,576 43 -> 41; but 29,478 43 -> 57, 29,791 hexahedra 51 -> 60, 83,968
+//     mixed cells 152 -> 181, 271,872 302 -> 411; 64,000 hexahedra alone 117 -> 95
+//   IORDER 1 FP64, below 192 cells per SM: hexahedra 8,000 30 -> 24, 24,389 34 -> 30,
+//     29,791 36 -> 42; CWENO 24,389 54 -> 33, 64,000 65 -> 73; tetrahedra 16,464
+//     25 -> 25, 29,478 30 -> 42
+//   IORDER 1 FP32, never: 512 to 20,000 cells 21 -> 24, 262,144 117 -> 200
+//   IORDER 3, below 128 cells per SM (18,944): CWENO, 9,728 cells FP64 156 -> 89,
+//     FP32 75 -> 44; 16,464 tetrahedra 114 -> 99, 61 -> 52; WENO, 17,576 hexahedra
+//     189 -> 127, 93 -> 67; 24,576 cells FP64 133 -> 139, 271,872 FP32 564 -> 626
+template <int P, typename T>
+bool wface_own(const Problem& p) {
+  constexpr bool f32 = sizeof(T) == 4;
+  if (!p.wface || p.scheme != 3 || (P == 1 && f32)) return false;
+  return (P == 2 && !f32) || p.n < (int64_t)p.nsm * (P == 3 ? 128 : 192);
+}
+
 // k_wpost: one lane per cell, no block barriers.  Indicators and weights of
 // CP_RECONSTRUCTION (src/reconstruct_p.f90:920-1250), the combined
 // polynomial, its face values and CHECKSOL; flagged cells (and every cell of
@@ -1089,9 +1107,8 @@ __global__ void __launch_bounds__(32 * NV) k_wface(Problem p, const double* __re
 // the kernel's registers otherwise allow: IORDER 3 in FP32 (2.1 M-cell CWENO4
 // Navier-Stokes step 52.7 -> 51.2 ms; in FP64 the bound made the 647 k-cell
 // step 31.8 -> 33.8 ms, so FP64 keeps two; 271,872 cells in FP32: 0.557 ms with
-// three, 0.577 with two, 0.619 with four), and IORDER 2 (high-order MUSCL and
-// the fall-back; measured with the whole reconstruction of 82,944 WENO3 tets,
-// before k_wface took it: 1.109 -> 1.083 ms per step mixed, 1.585 -> 1.540 FP64).
+// three, 0.577 with two, 0.619 with four), and IORDER 2 (82,944 WENO3 tets: 1.109
+// -> 1.083 ms per step mixed, 1.585 -> 1.540 FP64, which k_wface has taken since).
 template <int P, typename T, bool ISB = false, bool FB = false, bool MU = false>
 __global__ void __launch_bounds__(128, P == 2 || (P == 3 && sizeof(T) == 4) ? 3 : 1)
     k_wpost(Problem p, const double* __restrict__ U) {
@@ -2057,7 +2074,7 @@ cudaError_t launch_weno_t(const Problem& p, const double* U, bool ns, int QS, cu
         }
         done = true;
       }
-    } else if (p.wface && p.scheme == 3 && (P < 3 || p.n < (int64_t)p.nsm * 128)) {
+    } else if (wface_own<P, T>(p)) {
       const cudaError_t e = smem_limit(k_wface<P, T, true>, wface_smem<T>(MQ));
       if (e != cudaSuccess) return e;
       k_wface<P, T, true><<<ng, 32 * NV, smem, st>>>(p, U);
