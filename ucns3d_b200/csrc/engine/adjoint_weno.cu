@@ -1021,6 +1021,19 @@ void launch_visc_jvp_t(const Problem& p, const double* U, const double* dU, doub
   launch_visc_facegrad<P, double>(pt, st);
 }
 
+// Whether the reverse takes the tiles.  Below IORDER 3 only where the cells of a
+// tile follow one another (Problem::together): a member's contribution is 40
+// bytes a cell whatever the order, and with cells apart its stores cost more than
+// the small matrices that the tile saves (VJP less the residual, tiles against own
+// tables: WENO3, 114,048 mixed cells, 6.3 groups a warp, 1.84 and 1.44 ms, 24,576
+// tetrahedra, 10.6, 0.52 and 0.33; 64,000 hexahedra 0.84 and 0.98; CWENO3, 33,408
+// mixed cells 0.41 and 0.32).  At IORDER 3 and 4 the matrices outweigh them
+// (CWENO4, 114,048 mixed cells 2.38 and 3.04 ms).
+template <int P>
+bool adj_tiles(const Problem& p) {
+  return p.ntile && (P > 2 || p.together);
+}
+
 template <int P, int ND, bool LOW>
 cudaError_t launch_adj_set(const Problem& p, int nst, const double* gbar, double* selfs, double* contrib,
                            cudaStream_t st) {
@@ -1042,7 +1055,8 @@ cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, doub
   const cudaError_t ea = smem_limit(k_adj_wpost<P>, group_tri_smem<P>());
   if (ea != cudaSuccess) return ea;
   k_adj_wpost<P><<<(unsigned)((p.n + 31) / 32), WP_THREADS, tri, st>>>(p, U, adjF, gbar, scr, selfc, contrib);
-  if (p.ntile) {
+  const bool tiles = adj_tiles<P>(p);
+  if (tiles) {
     const bool cw = p.ees == 5 && p.admis_max > 1;
     cudaError_t e = launch_adj_set<P, ID, false>(p, cw ? 1 : p.admis_max, gbar, scr, contrib, st);
     if (e == cudaSuccess && cw) {
@@ -1056,8 +1070,10 @@ cudaError_t launch_t(const Problem& p, const double* U, const double* adjF, doub
     k_adj_self<<<(unsigned)((p.n * NV + 255) / 256), 256, 0, st>>>(p, selfc, scr, contrib);
     *launches += 2;
   }
-  if (!p.ntile || p.tiled) {
-    k_adj_lsq<P><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(p, gbar, selfc, contrib);
+  if (!tiles || p.tiled) {
+    Problem q = p;
+    if (!tiles) q.ntile = 0;  // every cell reads its own tables
+    k_adj_lsq<P><<<(unsigned)((p.n + 127) / 128), 128, 0, st>>>(q, gbar, selfc, contrib);
     ++*launches;
   }
   ++*launches;

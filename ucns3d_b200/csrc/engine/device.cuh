@@ -68,6 +68,7 @@ struct Problem {
   const int32_t* tcell;     // [ntile][SET_TILE] cells, -1 = none (never the first of a tile)
   const int32_t* tset;      // [ntile] set
   int64_t ntile;            // 0: every cell reads its own tables
+  bool together;            // the cells of a tile's warps lie in at most two 32-cell groups on average
   const int8_t* tiled;      // [n] the cell is in a tile; nullptr: every cell is (or none)
   const void* setmat;       // [nset][sstride], stencil ll at sso[ll]: rows [nk][set_stride(nd)]
   int64_t sstride;

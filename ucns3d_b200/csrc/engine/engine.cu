@@ -128,6 +128,7 @@ Problem make_problem(ucg_engine* e) {
     p.soff[k] = e->layout.soff[k];
   }
   p.ntile = e->ntile;
+  p.together = e->tiles_together;
   p.tcell = (const int32_t*)e->tcell.p;
   p.tset = (const int32_t*)e->tset.p;
   p.tiled = e->all_tiled ? nullptr : (const int8_t*)e->tiled.p;
