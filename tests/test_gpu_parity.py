@@ -24,6 +24,8 @@ SMALL = {
     "muscl_euler_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=9), SCHEME_MUSCL, 1, 0, EULER),
     "weno3_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=3), SCHEME_WENO, 2, 0, EULER),
     "weno5_hex": (lambda: Mesh.box_hex(12, 12, 12), SCHEME_WENO, 4, 0, EULER),
+    "weno2_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=6), SCHEME_WENO, 1, 0, EULER),
+    "cweno2_ns_hex": (lambda: Mesh.box_hex(9, 8, 8), SCHEME_WENO, 1, 5, NAVIER_STOKES),
     "cweno4_tet": (lambda: Mesh.box_tet(5, 5, 5, seed=5), SCHEME_WENO, 3, 5, EULER),
     "cweno4_ns_mixed": (lambda: Mesh.mixed_box(8, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES),
     "cweno4_ns_mixed10": (lambda: Mesh.mixed_box(10, seed=4), SCHEME_WENO, 3, 5, NAVIER_STOKES),
@@ -54,7 +56,8 @@ BUMPLIKE = ("muscl_bump", "weno3_channel", "muscl_bump_bt0", "weno5_channel", "m
 # channel with inflow/outflow/slip walls (boundary ghosts in the eigenvectors)
 SMALL["weno3_channel"] = (lambda: Mesh.bump_channel(16, 8, 8, seed=2), SCHEME_WENO, 2, 0, EULER)
 SMALL["weno5_channel"] = (lambda: Mesh.bump_channel(24, 12, 12, seed=2), SCHEME_WENO, 4, 0, EULER)
-CHAR = ["weno3_tet", "weno5_hex", "cweno4_tet", "cweno4_ns_mixed", "weno3_channel", "weno3_ns_bump"]
+CHAR = ["weno3_tet", "weno5_hex", "cweno4_tet", "cweno4_ns_mixed", "weno3_channel", "weno3_ns_bump", "weno2_tet",
+        "cweno2_ns_hex"]
 
 
 def _setup(name, precision=N.UCG_FP64, wenwrt=1):

@@ -1793,9 +1793,21 @@ __global__ void __launch_bounds__(32 * NV, 3) k_char_forms(Problem p) {
 // FP64 at IORDER 4 one face: two leave no registers for loads in flight
 // (27,000 cells: 1.28 ms with two, 1.06 with one and two blocks per SM, 1.38
 // with three).
+// At IORDER 1 and 2, whose polynomials are short, two, and more blocks per SM: with
+// three and two the kernel waited for its loads (38 us a block, the 15 values of
+// each stencil's form read by every warp for every face); there and in FP32 at
+// IORDER 3 the forms are read once for the block's faces (lean).  Characteristic
+// reconstruction after the least squares, us, FP64 and FP32: IORDER 1, 85,184
+// hexahedra 672 -> 522, 508 -> 480, 48,000 tetrahedra 254 -> 192, 183 -> 159; IORDER 2
+// 989 -> 871, 889 -> 676, 427 -> 388, 351 -> 262; IORDER 3 FP32 1285 -> 1204, 523 ->
+// 503 (FP64 1275 -> 1309 on 32,768 hexahedra, IORDER 4 FP32 1014 -> 1063: kept out).
+// One lane per cell took 651, 409, 242, 148; 2054, 859, 637, 275 (IORDER 1, 2): in FP32
+// at IORDER 1 on large meshes it was faster.
 template <int P, typename T>
 struct CharFaces {
-  static constexpr int value = P < 4 || sizeof(T) == 4 ? 3 : 1;
+  static constexpr int value = P < 3 ? 2 : P < 4 || sizeof(T) == 4 ? 3 : 1;
+  static constexpr bool lean = P < 3 || (P == 3 && sizeof(T) == 4);
+  static constexpr int blocks = P < 3 ? (sizeof(T) == 4 ? 4 : 3) : 2;  // per SM
 };
 template <int P, typename T>
 __host__ __device__ constexpr size_t char_face_smem(int QS) {
@@ -1803,10 +1815,12 @@ __host__ __device__ constexpr size_t char_face_smem(int QS) {
   return (size_t)NF * (50 + 7 * NV) * 32 * 8 + ((size_t)((QS * NV) | 1) + L2 * NV) * 32 * sizeof(T);
 }
 template <int P, typename T>
-__global__ void __launch_bounds__(32 * NV, 2) k_char_face(Problem p, const double* __restrict__ U) {
+__global__ void __launch_bounds__(32 * NV, CharFaces<P, T>::blocks)
+    k_char_face(Problem p, const double* __restrict__ U) {
   constexpr int ID = Deg<P>::ideg;
   constexpr int L2 = ID < 9 ? ID : 9;
   constexpr int NF = CharFaces<P, T>::value;
+  constexpr bool LEAN = CharFaces<P, T>::lean;
   constexpr int MA = 7;  // stencils per cell at most
   extern __shared__ __align__(16) unsigned char cf_smem[];
   const int QS = p.nq_quad > p.nq_tri ? p.nq_quad : p.nq_tri;
@@ -1850,26 +1864,8 @@ __global__ void __launch_bounds__(32 * NV, 2) k_char_face(Problem p, const doubl
   __syncthreads();
   // indicators and weights (WENOWEIGHTS, FP64) of characteristic variable v
   const double* Qc = p.qbuf + grp * (int64_t)(A * 15) * 32 + lane;
-  for (int f = 0; f < NF; ++f) {
-    if (f0 + f >= nf) break;
-    double l[NV], w[MA];
-#pragma unroll
-    for (int u = 0; u < NV; ++u) l[u] = s_e[(f * 50 + v * NV + u) * 32 + lane];
+  auto weights = [&](int f, double (&w)[MA]) {  // w: the indicators
     double tau = 0.0, sum = 0.0;
-#pragma unroll
-    for (int ll = 0; ll < MA; ++ll) {
-      w[ll] = 0.0;
-      if (ll < adm) {
-        double is = 0.0;
-        int j = 0;
-#pragma unroll
-        for (int u = 0; u < NV; ++u)
-#pragma unroll
-          for (int k = u; k < NV; ++k, ++j)
-            is += (u == k ? 1.0 : 2.0) * l[u] * l[k] * Qc[(int64_t)(ll * 15 + j) * 32];
-        w[ll] = is;
-      }
-    }
     if (cw && p.wenoz) {
 #pragma unroll
       for (int ll = 0; ll < MA; ++ll)
@@ -1894,6 +1890,54 @@ __global__ void __launch_bounds__(32 * NV, 2) k_char_face(Problem p, const doubl
 #pragma unroll
     for (int ll = 0; ll < MA; ++ll)
       if (ll < adm) s_w[((f * MA + ll) * NV + v) * 32 + lane] = w[ll] / sum;
+  };
+  if constexpr (LEAN) {  // a stencil's form read once for the block's faces
+    double l[NF][NV], w[NF][MA];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int u = 0; u < NV; ++u) l[f][u] = f0 + f < nf ? s_e[(f * 50 + v * NV + u) * 32 + lane] : 0.0;
+#pragma unroll
+    for (int ll = 0; ll < MA; ++ll) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) w[f][ll] = 0.0;
+      if (ll < adm) {
+        int j = 0;
+#pragma unroll
+        for (int u = 0; u < NV; ++u)
+#pragma unroll
+          for (int k = u; k < NV; ++k, ++j) {
+            const double q = Qc[(int64_t)(ll * 15 + j) * 32];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) w[f][ll] += (u == k ? 1.0 : 2.0) * l[f][u] * l[f][k] * q;
+          }
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (f0 + f < nf) weights(f, w[f]);
+  } else {
+    for (int f = 0; f < NF; ++f) {
+      if (f0 + f >= nf) break;
+      double l[NV], w[MA];
+#pragma unroll
+      for (int u = 0; u < NV; ++u) l[u] = s_e[(f * 50 + v * NV + u) * 32 + lane];
+#pragma unroll
+      for (int ll = 0; ll < MA; ++ll) {
+        w[ll] = 0.0;
+        if (ll < adm) {
+          double is = 0.0;
+          int j = 0;
+#pragma unroll
+          for (int u = 0; u < NV; ++u)
+#pragma unroll
+            for (int k = u; k < NV; ++k, ++j)
+              is += (u == k ? 1.0 : 2.0) * l[u] * l[k] * Qc[(int64_t)(ll * 15 + j) * 32];
+          w[ll] = is;
+        }
+      }
+      weights(f, w);
+    }
   }
   __syncthreads();
   // the faces' polynomials of variable v
@@ -1978,8 +2022,16 @@ __global__ void __launch_bounds__(32 * NV, 2) k_char_face(Problem p, const doubl
       for (int k = 0; k < NV; ++k) uf[k] = u0[k] + (double)s_o[lane * RS + q * NV + k];
       flag = flag || jump_bad(p.gamma, pm, uf, 0.85);
     }
-    for (int cl = v; cl < ncl; cl += NV)
-      for (int r = lane; r < QS * NV; r += 32) out[(int64_t)cl * FQ * NV + fc * QS * NV + r] = s_o[cl * RS + r];
+    if constexpr (LEAN) {  // a thread per value: a cell's run is short
+      const int run = QS * NV;
+      for (int k = threadIdx.x; k < ncl * run; k += 32 * NV) {
+        const int cl = k / run, r = k - cl * run;
+        out[(int64_t)cl * FQ * NV + fc * run + r] = s_o[cl * RS + r];
+      }
+    } else {
+      for (int cl = v; cl < ncl; cl += NV)
+        for (int r = lane; r < QS * NV; r += 32) out[(int64_t)cl * FQ * NV + fc * QS * NV + r] = s_o[cl * RS + r];
+    }
   }
   if (flag) p.wflag[c] = 1;  // to the MUSCL fall-back (k_wpost<..., FB>)
 }
