@@ -185,6 +185,14 @@ def lsq_rows(cfg):
             for ll in range(cfg.admis_max)]
 
 
+def stencil_shares(mesh, cfg):
+    """The share of the cells in which each stencil is admissible: only there
+    are its tables and members read."""
+    import numpy as np
+    adm = np.ctypeslib.as_array(mesh.geometry_struct().admis, shape=(mesh.ncells,))
+    return [float((adm > ll).mean()) for ll in range(cfg.admis_max)]
+
+
 def table_size(cfg):
     from ucns3d_b200 import _native as N
     return 4 if cfg.precision == N.UCG_MIXED else 8
@@ -211,31 +219,32 @@ def sets_per_cell(ncells, shared):
     return (ncells - shared["cells"] + shared["sets"]) / ncells
 
 
-def lsq_bytes_per_cell(cfg, per_cell):
+def lsq_bytes_per_cell(cfg, shares, per_cell):
     """Algorithmic bytes of the stencil least squares per cell: the
     pseudo-inverse slices (times the matrix sets read per cell) and stencil
-    indices of every stencil, the cell's own state, and the stencil polynomials
-    G written (neighbour states come through L2; they are counted once, in the
-    flux kernel)."""
+    indices of the admissible stencils, the cell's own state, and the stencil
+    polynomials G written (neighbour states come through L2; they are counted
+    once, in the flux kernel)."""
     s = table_size(cfg)
-    return 5 * 8 + sum(s * nk * nd * per_cell + 4 * nk + s * nd * 5 for nk, nd in lsq_rows(cfg))
+    return 5 * 8 + sum(a * (s * nk * nd * per_cell + 4 * nk) + s * nd * 5
+                       for a, (nk, nd) in zip(shares, lsq_rows(cfg)))
 
 
-def lsq_flops_per_cell(cfg):
+def lsq_flops_per_cell(cfg, shares):
     """Multiply-adds of the stencil least squares per cell, times two."""
-    return sum(10 * nk * nd for nk, nd in lsq_rows(cfg))
+    return sum(10 * a * nk * nd for a, (nk, nd) in zip(shares, lsq_rows(cfg)))
 
 
-def lsq_roofline(cfg, ncells, shared, ms, peak, peak_kind, sm_mhz):
+def lsq_roofline(cfg, shares, ncells, shared, ms, peak, peak_kind, sm_mhz):
     """The least squares against what bounds it, the longer of two times: its
     bytes at the DRAM rate, or its FP32 (FP64) multiply-adds at the nominal peak
     (148 SMs x 128 (64) lanes at the SM clock)."""
     from ucns3d_b200 import _native as N
-    bpc = lsq_bytes_per_cell(cfg, sets_per_cell(ncells, shared))
+    bpc = lsq_bytes_per_cell(cfg, shares, sets_per_cell(ncells, shared))
     hbm = bpc * ncells / (ms / 1000.0) / 1e9
     lanes = 128 if cfg.precision == N.UCG_MIXED else 64
     top = 148 * lanes * 2 * sm_mhz * 1e6 / 1e12
-    tf = lsq_flops_per_cell(cfg) * ncells / (ms / 1000.0) / 1e12
+    tf = lsq_flops_per_cell(cfg, shares) * ncells / (ms / 1000.0) / 1e12
     out = {"bytes_per_cell": bpc, "shared_cells": shared["cells"], "shared_sets": shared["sets"]}
     if hbm / peak >= tf / top:
         return {"bound": "hbm", "achieved": hbm, "peak": peak, "unit": "GB/s", "frac": hbm / peak,
@@ -244,7 +253,7 @@ def lsq_roofline(cfg, ncells, shared, ms, peak, peak_kind, sm_mhz):
             "hbm_gbs": hbm, **out}
 
 
-def recon_bytes_per_cell(cfg, per_cell):
+def recon_bytes_per_cell(cfg, shares, per_cell):
     """Algorithmic bytes the reconstruction kernels must move per cell: the
     pseudo-inverses (times the matrix sets read per cell), the smoothness
     matrix, stencil indices, face quadrature points and basis means of the cell,
@@ -254,7 +263,7 @@ def recon_bytes_per_cell(cfg, per_cell):
     others read every cell's own copy."""
     s = table_size(cfg)
     nq = max(cfg.nq_quad, cfg.nq_tri)
-    b = sum(s * nk * nd * per_cell + 4 * (nk + 1) for nk, nd in lsq_rows(cfg))
+    b = sum(a * (s * nk * nd * per_cell + 4 * (nk + 1)) for a, (nk, nd) in zip(shares, lsq_rows(cfg)))
     if cfg.scheme == 3:  # packed upper triangle of the smoothness matrix
         once = cfg.wenwrt == 2 or (cfg.iorder == 4 and cfg.ees != 5)
         b += s * cfg.ideg * (cfg.ideg + 1) // 2 * (per_cell if once else 1.0)
@@ -822,11 +831,12 @@ def main():
     # roofline of the stencil least squares, achieved from its CUDA-event
     # duration on the engine stream; the whole reconstruction beside it
     share = sets_per_cell(ncells, r32["shared"])
-    table_bytes = lsq_bytes_per_cell(cfg32, share) * ncells  # tables, indices, polynomials: what a stage touches
+    adm = stencil_shares(c32.mesh, cfg32)
+    table_bytes = lsq_bytes_per_cell(cfg32, adm, share) * ncells  # tables, indices, polynomials: what a stage touches
     lsq_ms = r32["kern"]["lsq"]
     sm_mhz = (r32["clocks"] or {}).get("sm_mhz") or 1965.0
-    roof = lsq_roofline(cfg32, ncells, r32["shared"], lsq_ms, peak, peak_kind, sm_mhz)
-    rbpc = recon_bytes_per_cell(cfg32, share)
+    roof = lsq_roofline(cfg32, adm, ncells, r32["shared"], lsq_ms, peak, peak_kind, sm_mhz)
+    rbpc = recon_bytes_per_cell(cfg32, adm, share)
     traffic, traffic_kind = lsq_traffic(args.case, cfg32, ncells)
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
@@ -861,7 +871,7 @@ def main():
         ra, rb = r64["state"][:, 0], r32["state"][:, 0]
         l2 = float(np.sqrt(np.mean((ra - rb) ** 2)) / np.sqrt(np.mean(ra ** 2)))
         linf = float(np.abs(ra - rb).max() / np.abs(ra).max())
-        roof64 = lsq_roofline(cfg64, ncells, r64["shared"], r64["kern"]["lsq"], peak, peak_kind, sm_mhz)
+        roof64 = lsq_roofline(cfg64, adm, ncells, r64["shared"], r64["kern"]["lsq"], peak, peak_kind, sm_mhz)
         out["fp64"] = {"value": v64, "ms_per_step": ms64 / args.steps, "kernel_ms": r64["kern"],
                        "roofline_frac": roof64["frac"], "roofline_bound": roof64["bound"],
                        "mixed_speedup": value / v64,
