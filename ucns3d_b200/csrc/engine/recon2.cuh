@@ -1454,7 +1454,8 @@ __global__ void k_visc_prim(Problem p, const double* __restrict__ U) {
 // that the tiles leave (p.ugrp), whose few lanes' chain of loads runs beside
 // the tiles.  271,872 cells, CWENO4 mixed form: 0.270 -> 0.149 ms (0.167 at three
 // blocks per SM, 0.229 at five with two members in flight; the groups left in
-// a launch of their own 0.056 more).
+// a launch of their own 0.056 more); WENO5 FP64, 8,000 cells, whose 63 blocks
+// waited for one chain of loads, all after the least squares 3.23 -> 0.24.
 // Blocks of that launch with left-over groups (four each), and the cell of a
 // thread of a block, -1 for none: a tiled cell of a left-over group has its
 // block among the tiles', so that every cell has one writer.
